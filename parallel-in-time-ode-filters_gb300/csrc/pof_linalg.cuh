@@ -127,6 +127,49 @@ __device__ __forceinline__ void householder(T alpha, T xn2, T& beta, T& tau, T& 
   }
 }
 
+// true when x is +0 or -0, tested on the bits (a floating-point compare of a
+// double would go through the FP64 pipe)
+__device__ __forceinline__ bool is_zero(double x) { return (__double_as_longlong(x) << 1) == 0; }
+__device__ __forceinline__ bool is_zero(float x) { return (__float_as_uint(x) << 1) == 0; }
+
+// The same reflector in the unnormalized form H = I + kap v v^T with
+// v = (u, x), u = alpha - beta, kap = 1 / (u beta): the tail x is used as it
+// is (no pass that scales it), and the squared norm can be formed together
+// with the dot products of the rows below.  For xn2 != 0 only.  Double
+// precision: ||(alpha, x)|| = h and 1 / (u beta) = -1 / (a2 + |alpha| h) from
+// single-precision seeds and one third-order correction each (as rsqrt_nr and
+// rcp_nr): 11 FP64 instructions.
+template <typename T>
+__device__ __forceinline__ void reflector(T alpha, T xn2, T& beta, T& u, T& kap) {
+  if constexpr (std::is_same<T, double>::value) {
+    const double a2 = fma(alpha, alpha, xn2);
+    const long long bits = __double_as_longlong(a2);
+    const int e = (int)((bits >> 52) & 0x7ff) - 1023;
+    double h;
+    if (e < -1000 || e > 1000) {
+      h = sqrt(a2);
+    } else {
+      const int k = e >> 1;
+      const float mf = __int_as_float(((127 + e - 2 * k) << 23) | (int)((bits >> 29) & 0x7fffff));
+      const double y = widen_with_exp(rsqrtf(mf), -k, 0);
+      const double g = a2 * y;
+      const double r = fma(-g, y, 1.0);
+      h = fma(g, r * fma(r, 0.375, 0.5), g);
+    }
+    // sign(0) = +, so alpha = -0 reflects like +0
+    const long long ab = __double_as_longlong(alpha);
+    const bool neg = ab < 0 && (ab << 1) != 0;
+    beta = neg ? h : __longlong_as_double(__double_as_longlong(h) ^ (1LL << 63));
+    u = alpha - beta;
+    kap = -rcp_nr(fma(fabs(alpha), h, a2));
+  } else {
+    const T nrm = sqrt(fma(alpha, alpha, xn2));
+    beta = alpha >= T(0) ? -nrm : nrm;
+    u = alpha - beta;
+    kap = T(1) / (u * beta);
+  }
+}
+
 // C(MxN) = A(MxK) * B(KxN)
 template <typename T, int M, int K, int N, int LDA, int LDB, int LDC>
 __device__ __forceinline__ void mm(const T* __restrict__ A, const T* __restrict__ B, T* __restrict__ C) {

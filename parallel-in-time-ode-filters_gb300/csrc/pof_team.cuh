@@ -175,6 +175,170 @@ __device__ __forceinline__ void t_tria(const Team<TS>& tm, T* X, T* Y, int wlow 
   tm.sync();
 }
 
+// ---------------------------------------------------------------------------
+// LQ with a triangular pivot block.  Rows [P | W] (M rows, pivot entry (j, j)
+// of row j in column j, tail columns [kb(j), ke(j)) given by `tail`) and MB
+// more rows Y in the same columns below: reflector j combines pivot column j
+// with row j's tail, so that afterwards the pivot block is L (lower
+// triangular, L L^T = P P^T + W W^T) and the rows Y have been multiplied by
+// the same orthogonal matrix.  The tails of the M rows are left as they are
+// (zero in exact arithmetic) and must not be read.
+//
+// This is every triangularization of the filter and smoother: tria([X, L])
+// with a lower-triangular L is [P | W] = [L | X] (TailFixed), a general
+// matrix is P = W with the tail right of the diagonal (TailUpper).
+//
+// GB300 issues one FP64 instruction per warp and 64 cycles on each of the
+// SM's sub-partitions, whatever its lanes do and whether it depends on the
+// one before (measured: 64.4 cycles dependent or independent, 1 or 32 lanes,
+// and 76 once all four sub-partitions issue), so the cost of a reflector is
+// its count of FP64 instructions plus what does not overlap with them.  The
+// row's own squared norm is therefore one more of the dot products (entry 0),
+// the scalars are computed by every lane instead of on one and broadcast (the
+// same instructions), the tail is not rescaled, and one team barrier per
+// reflector is left.  An exactly zero tail (LAPACK's tau = 0) skips the
+// reflector.
+//
+// Entries (the reflector's row and the rows below) are spread over RS row
+// slots; a team with more lanes than entries gives each row G = TS / RS
+// lanes, which take every G-th tail column.
+// ---------------------------------------------------------------------------
+template <int R>
+struct Pow2Ceil {
+  static constexpr int v = R <= 1 ? 1 : (R <= 2 ? 2 : (R <= 4 ? 4 : (R <= 8 ? 8 : (R <= 16 ? 16 : 32))));
+};
+
+template <int KB, int KE>
+struct TailFixed {  // the same columns for every reflector
+  static constexpr int count = KE - KB;
+  __device__ __forceinline__ void operator()(int, int& b, int& e) const { b = KB, e = KE; }
+};
+struct TailUpper {  // the columns right of the diagonal, up to `n`
+  static constexpr int count = 0;  // not a constant
+  int n;
+  __device__ __forceinline__ void operator()(int j, int& b, int& e) const { b = j + 1, e = n; }
+};
+
+template <typename T, int TS, int M, int MB, int LD, int LDY, typename Tail>
+__device__ __forceinline__ void t_lq(const Team<TS>& tm, T* X, T* Y, const Tail& tail, int mlim = M) {
+  constexpr int NE = M + MB;
+  constexpr int RS = Pow2Ceil<NE>::v < TS ? Pow2Ceil<NE>::v : TS;
+  constexpr int G = TS / RS;
+  constexpr int NP = (NE + RS - 1) / RS;
+  const int src = (threadIdx.x & 31) / TS * TS;  // lane 0 of this team within the warp
+  const int slot = tm.r % RS, ph = tm.r / RS;
+  T pend = T(0);  // diagonal of the reflector before, written once every lane has read it
+  int pj = -1;
+#pragma unroll 1
+  for (int j = 0; j < mlim; ++j) {
+    int kb, ke;
+    tail(j, kb, ke);
+    if (kb >= ke) continue;
+    tm.sync();
+    if (pj >= 0 && tm.r == 0) X[pj * LD + pj] = pend;
+    const T* xj = X + j * LD;
+    const T alpha = xj[j];
+    const int ne = M - j + MB;  // entries of this reflector; pass p has one if p RS < ne
+    T* row[NP];
+    T dot[NP];
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+      const int e = slot + p * RS;
+      row[p] = e >= ne ? X + j * LD : (e < M - j ? X + (j + e) * LD : Y + (e - (M - j)) * LDY);
+      dot[p] = T(0);
+    }
+    if constexpr (Tail::count > 0 && Tail::count % G == 0) {
+#pragma unroll
+      for (int t = 0; t < Tail::count; t += G) {
+        const T x = xj[kb + ph + t];
+#pragma unroll
+        for (int p = 0; p < NP; ++p)
+          if (p == 0 || p * RS < ne) dot[p] = fma(row[p][kb + ph + t], x, dot[p]);
+      }
+    } else {
+#pragma unroll 2
+      for (int k = kb + ph; k < ke; k += G) {
+        const T x = xj[k];
+#pragma unroll
+        for (int p = 0; p < NP; ++p)
+          if (p == 0 || p * RS < ne) dot[p] = fma(row[p][k], x, dot[p]);
+      }
+    }
+#pragma unroll
+    for (int o = RS; o < TS; o <<= 1)
+#pragma unroll
+      for (int p = 0; p < NP; ++p) dot[p] += __shfl_xor_sync(tm.mask, dot[p], o, TS);
+    const T xn2 = __shfl_sync(tm.mask, dot[0], src);
+    pj = -1;
+    if (is_zero(xn2)) continue;
+    T beta, u, kap;
+    reflector(alpha, xn2, beta, u, kap);
+    pend = beta;
+    pj = j;
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+      const int e = slot + p * RS;
+      if (e == 0 || e >= ne) continue;
+      T* xi = row[p];
+      const T a = xi[j];
+      const T w = kap * fma(u, a, dot[p]);
+      if (ph == 0) xi[j] = fma(w, u, a);
+      if constexpr (Tail::count > 0 && Tail::count % G == 0) {
+#pragma unroll
+        for (int t = 0; t < Tail::count; t += G) xi[kb + ph + t] = fma(w, xj[kb + ph + t], xi[kb + ph + t]);
+      } else {
+#pragma unroll 2
+        for (int k = kb + ph; k < ke; k += G) xi[k] = fma(w, xj[k], xi[k]);
+      }
+    }
+  }
+  tm.sync();
+  if (pj >= 0 && tm.r == 0) X[pj * LD + pj] = pend;
+  tm.sync();
+}
+
+// The value (op(A) x)(i) for row i = lane's row slot (zero for slots beyond
+// M), A given by its row and column strides; G = TS / slots lanes share a
+// row's terms, every lane of a slot gets the sum.
+template <typename T, int TS, int M, int K>
+__device__ __forceinline__ T t_dotrow(const Team<TS>& tm, const T* A, int rs, int cs, const T* x) {
+  constexpr int RS = Pow2Ceil<M>::v < TS ? Pow2Ceil<M>::v : TS;
+  constexpr int G = TS / RS;
+  static_assert(M <= RS, "one row per lane");
+  const int i = tm.r % RS < M ? tm.r % RS : 0;
+  T s = T(0);
+#pragma unroll
+  for (int k0 = 0; k0 < K; k0 += G) {
+    const int k = k0 + tm.r / RS;
+    if (K % G == 0 || k < K) s = fma(A[i * rs + k * cs], x[k], s);
+  }
+#pragma unroll
+  for (int o = RS; o < TS; o <<= 1) s += __shfl_xor_sync(tm.mask, s, o, TS);
+  return s;
+}
+// C(M x N) = A(M x N) B with B (N x N) lower triangular: column group t of
+// the outputs starts its sum at the group's first column (terms above B's
+// diagonal are exact zeros), one row per lane slot.
+template <typename T, int TS, int M, int N, int LDA, int LDB, int LDC>
+__device__ __forceinline__ void t_mm_lowB(const Team<TS>& tm, const T* A, const T* B, T* C) {
+  constexpr int RS = Pow2Ceil<M>::v < TS ? Pow2Ceil<M>::v : TS;
+  constexpr int CG = TS / RS;
+#pragma unroll
+  for (int i0 = 0; i0 < M; i0 += RS) {
+    const int i = i0 + tm.r % RS;
+    if (M % RS != 0 && i >= M) continue;
+#pragma unroll
+    for (int t = 0; t < N; t += CG) {
+      const int j = t + tm.r / RS;
+      if (N % CG != 0 && j >= N) continue;
+      T s = T(0);
+#pragma unroll
+      for (int k = t; k < N; ++k) s = fma(A[i * LDA + k], B[k * LDB + j], s);
+      C[i * LDC + j] = s;
+    }
+  }
+}
+
 // 1 / L_ii for i = 0..M-1, computed in parallel (lane i) and read by every
 // lane through a shuffle: each division is done once per team, not once per
 // right-hand side.
@@ -278,22 +442,25 @@ struct FiltTeamWs {
   T Xt[D * LD2], Xb[D * LD2];  // [U1^T Z2, I] and [Z2, 0] -> Xi
   T M[D * LD1], Mu[D * LD1], W[D * LD1];
   T UX[D * LD2];
-  T v1[D], v2[D], v3[D];
+  T v1[D], v2[D], v3[D], v4[D];
 };
 
-// e1 <- e1 (x) e2 (pof/parallel_filtsmooth/filter.py:117-142)
+// Xi = tria([[U1^T Z2, I], [Z2, 0]]) as [P | W] = [I | U1^T Z2] over
+// [0 | Z2]: Xi11 = Xt[:, :D], Xi21 = Xb[:, :D], and Xb[:, D:] is Xi22 before
+// its own triangularization -- its only use is Z = tria([A1^T Xi22, Z1]),
+// which takes any square root, so that triangularization (a third of the
+// operator's reflectors) is not done.  M = Xi11^{-1} U1^T A2^T and
+// Mu = Xi11^{-1} U1^T follow; both vector chains of the operator use Mu:
+// m^T Xi21^T = Mu^T Xi21^T and e^T U1^T = Xi21 Mu (e = Xi11^{-T} Xi21^T).
 template <typename T, int TS, int D>
-__device__ __forceinline__ void t_filt_combine(const Team<TS>& tm, FiltTeamWs<T, D>& w) {
+__device__ __forceinline__ void t_filt_xi(const Team<TS>& tm, FiltTeamWs<T, D>& w) {
   using W = FiltTeamWs<T, D>;
-  constexpr int L1 = W::LD1, L2 = W::LD2, D2 = W::D2;
-  // Xi = [[U1^T Z2, I], [Z2, 0]]
-  t_mm<T, TS, D, D, D, L1, L1, L2, true, false>(tm, w.U1, w.Z2, w.Xt);
-  t_fill<T, TS, D, D, L2>(tm, w.Xt + D, T(0), T(1));
-  t_copy<T, TS, D, D, L1, L2>(tm, w.Z2, w.Xb);
-  t_fill<T, TS, D, D, L2>(tm, w.Xb + D, T(0), T(0));
-  t_tria<T, TS, D, D, D2, L2, L2>(tm, w.Xt, w.Xb, D);   // Xi11 = Xt[:, :D], Xi21 = Xb[:, :D]
-  t_tria<T, TS, D, 0, D, L2, L2>(tm, w.Xb + D, w.Xb);  // Xi22 = Xb[:, D:]
-  // M = Xi11^{-1} U1^T A2^T ; Mu = Xi11^{-1} U1^T
+  constexpr int L1 = W::LD1, L2 = W::LD2;
+  t_mm<T, TS, D, D, D, L1, L1, L2, true, false>(tm, w.U1, w.Z2, w.Xt + D);
+  t_fill<T, TS, D, D, L2>(tm, w.Xt, T(0), T(1));
+  t_copy<T, TS, D, D, L1, L2>(tm, w.Z2, w.Xb + D);
+  t_fill<T, TS, D, D, L2>(tm, w.Xb, T(0), T(0));
+  t_lq<T, TS, D, D, L2, L2>(tm, w.Xt, w.Xb, TailFixed<D, 2 * D>{});
   t_mm<T, TS, D, D, D, L1, L1, L1, true, true>(tm, w.U1, w.A2, w.M);
   t_copy<T, TS, D, D, L1, L1, true>(tm, w.U1, w.Mu);
   tm.sync();
@@ -302,65 +469,70 @@ __device__ __forceinline__ void t_filt_combine(const Team<TS>& tm, FiltTeamWs<T,
     t_trsm_l<T, TS / 2, D, D, L2, L1>(h, w.Xt, tm.r >= TS / 2 ? w.Mu : w.M);
   }
   tm.sync();
-  // W = M^T Xi21^T  ; A_new = (A2 - W) A1  (into UX scratch, then copied)
-  t_mm<T, TS, D, D, D, L1, L2, L1, true, true>(tm, w.M, w.Xb, w.W);
+}
+
+// e1 <- e1 (x) e2 (pof/parallel_filtsmooth/filter.py:117-142)
+//
+// Latency-bound on the tree's upper levels (FP64 instructions of one warp,
+// 64 cycles each).  Per combine on a 32-lane team at D = 8 about 530 FP64
+// instructions, from about 1060 with Xi22 triangularized, the e solve and
+// the vector chains one after the other.
+template <typename T, int TS, int D>
+__device__ __forceinline__ void t_filt_combine(const Team<TS>& tm, FiltTeamWs<T, D>& w) {
+  using W = FiltTeamWs<T, D>;
+  constexpr int L1 = W::LD1, L2 = W::LD2;
+  const Team<TS / 2> h;
+  const bool hi = tm.r >= TS / 2;  // the half that runs eta's chain (the other: b's)
+  const bool put = h.r < D;
+  static_assert(TS / 2 >= D || TS == 32, "a half-team holds one row per lane");
+  // b: t2 = b1 + U1 U1^T eta2; eta: s2 = eta2 - Z2 Z2^T b1
+  T* const va = hi ? w.v3 : w.v1;
+  T* const vb = hi ? w.v4 : w.v2;
+  const T* const S = hi ? w.Z2 : w.U1;
+  T x = t_dotrow<T, TS / 2, D, D>(h, S, 1, L1, hi ? w.b1 : w.e2);
+  if (put) va[h.r] = x;
   tm.sync();
+  x = t_dotrow<T, TS / 2, D, D>(h, S, L1, 1, va);
+  if (put) vb[h.r] = hi ? w.e2[h.r] - x : w.b1[h.r] + x;  // read again after t_filt_xi's barriers
+  t_filt_xi<T, TS, D>(tm, w);
+  // b: t3 = Xi21^T t2, t2 -= Mu^T t3; eta: s3 = Mu s2, s2 -= Xi21 s3
+  // (one instruction stream: the halves differ in pointers and strides)
+  x = t_dotrow<T, TS / 2, D, D>(h, hi ? w.Mu : w.Xb, hi ? L1 : 1, hi ? 1 : L2, vb);
+  if (put) va[h.r] = x;
+  tm.sync();
+  x = t_dotrow<T, TS / 2, D, D>(h, hi ? w.Xb : w.Mu, hi ? L2 : 1, hi ? 1 : L1, va);
+  if (put) vb[h.r] -= x;
+  tm.sync();
+  // b = A2 t2 + b2; eta = A1^T s2 + eta1
+  x = t_dotrow<T, TS / 2, D, D>(h, hi ? w.A1 : w.A2, hi ? 1 : L1, hi ? L1 : 1, vb);
+  if (put) {
+    if (hi)
+      w.e1[h.r] += x;
+    else
+      w.b1[h.r] = w.b2[h.r] + x;
+  }
+  // W = A2 - M^T Xi21^T
   for (int idx = tm.r; idx < D * D; idx += TS) {
     const int i = idx / D, j = idx % D;
-    T s = T(0);
+    T s = w.A2[i * L1 + j];
 #pragma unroll
-    for (int k = 0; k < D; ++k) s = fma(w.A2[i * L1 + k] - w.W[i * L1 + k], w.A1[k * L1 + j], s);
-    w.UX[i * L2 + j] = s;
+    for (int k = 0; k < D; ++k) s = fma(-w.M[k * L1 + i], w.Xb[j * L2 + k], s);
+    w.W[i * L1 + j] = s;
   }
-  // b: t2 = b1 + U1 U1^T eta2 ; t3 = Xi21^T t2 ; t2 -= Mu^T t3 ; b = A2 t2 + b2
-  t_mv<T, TS, D, D, L1, true>(tm, w.U1, w.e2, w.v1);
+  // Z = tria([Z1 | A1^T Xi22]) (the rows of Xt reused), U = tria([U2 | M^T])
+  t_mm<T, TS, D, D, D, L1, L2, L2, true, false>(tm, w.A1, w.Xb + D, w.Xt + D);
+  t_copy<T, TS, D, D, L1, L2>(tm, w.Z1, w.Xt);
+  t_copy<T, TS, D, D, L1, L2, true>(tm, w.M, w.UX + D);
+  t_copy<T, TS, D, D, L1, L2>(tm, w.U2, w.UX);
   tm.sync();
-  t_mv<T, TS, D, D, L1, false>(tm, w.U1, w.v1, w.v2);
-  tm.sync();
-  for (int i = tm.r; i < D; i += TS) w.v2[i] += w.b1[i];
-  tm.sync();
-  t_mv<T, TS, D, D, L2, true>(tm, w.Xb, w.v2, w.v3);
-  tm.sync();
-  t_mv<T, TS, D, D, L1, true>(tm, w.Mu, w.v3, w.v1);
-  tm.sync();
-  for (int i = tm.r; i < D; i += TS) w.v2[i] -= w.v1[i];
-  tm.sync();
-  t_mv<T, TS, D, D, L1, false>(tm, w.A2, w.v2, w.v3);  // b_new (without b2) in v3
-  tm.sync();
-  // eta: e = Xi11^{-T} Xi21^T (into Mu) ; t = eta2 - Z2 Z2^T b1 ; t -= e^T U1^T t ; eta = A1^T t + eta1
-  t_copy<T, TS, D, D, L2, L1, true>(tm, w.Xb, w.Mu);
-  t_mv<T, TS, D, D, L1, true>(tm, w.Z2, w.b1, w.v1);
-  tm.sync();
-  t_trsm_lt<T, TS, D, D, L2, L1>(tm, w.Xt, w.Mu);
-  t_mv<T, TS, D, D, L1, false>(tm, w.Z2, w.v1, w.v2);
-  tm.sync();
-  for (int i = tm.r; i < D; i += TS) w.v2[i] = w.e2[i] - w.v2[i];
-  for (int i = tm.r; i < D; i += TS) w.b1[i] = w.v3[i] + w.b2[i];  // b1 no longer read
-  tm.sync();
-  t_mv<T, TS, D, D, L1, true>(tm, w.U1, w.v2, w.v1);
-  tm.sync();
-  t_mv<T, TS, D, D, L1, true>(tm, w.Mu, w.v1, w.v3);
-  tm.sync();
-  for (int i = tm.r; i < D; i += TS) w.v2[i] -= w.v3[i];
-  tm.sync();
-  t_mv<T, TS, D, D, L1, true>(tm, w.A1, w.v2, w.v3);
-  tm.sync();
-  for (int i = tm.r; i < D; i += TS) w.e1[i] = w.v3[i] + w.e1[i];
-  // Z = tria([A1^T Xi22, Z1])  (Xt rows reused: A1 is still the old A)
-  t_mm<T, TS, D, D, D, L1, L2, L2, true, false>(tm, w.A1, w.Xb + D, w.Xt);
-  t_copy<T, TS, D, D, L1, L2>(tm, w.Z1, w.Xt + D);
-  tm.sync();
-  // A1 <- new A (from UX scratch) ; U = tria([M^T, U2]) in UX
-  t_copy<T, TS, D, D, L2, L1>(tm, w.UX, w.A1);
-  tm.sync();
-  t_copy<T, TS, D, D, L1, L2, true>(tm, w.M, w.UX);
-  t_copy<T, TS, D, D, L1, L2>(tm, w.U2, w.UX + D);
+  // A = W A1, kept in M until A1 is no longer read
+  t_mm<T, TS, D, D, D, L1, L1, L1>(tm, w.W, w.A1, w.M);
   {  // U and Z side by side on the two halves of the team
-    const Team<TS / 2> h;
-    T* X = tm.r >= TS / 2 ? w.Xt : w.UX;
-    t_tria<T, TS / 2, D, 0, D2, L2, L2>(h, X, X, D);
+    T* X = hi ? w.Xt : w.UX;
+    t_lq<T, TS / 2, D, 0, L2, L2>(h, X, X, TailFixed<D, 2 * D>{});
   }
   tm.sync();
+  t_copy<T, TS, D, D, L1, L1>(tm, w.M, w.A1);
   t_copy<T, TS, D, D, L2, L1>(tm, w.UX, w.U1);
   t_copy<T, TS, D, D, L2, L1>(tm, w.Xt, w.Z1);
   tm.sync();
@@ -371,38 +543,25 @@ __device__ __forceinline__ void t_filt_combine(const Team<TS>& tm, FiltTeamWs<T,
 template <typename T, int TS, int D>
 __device__ __forceinline__ void t_filt_apply(const Team<TS>& tm, FiltTeamWs<T, D>& w) {
   using W = FiltTeamWs<T, D>;
-  constexpr int L1 = W::LD1, L2 = W::LD2, D2 = W::D2;
-  t_mm<T, TS, D, D, D, L1, L1, L2, true, false>(tm, w.U1, w.Z2, w.Xt);
-  t_fill<T, TS, D, D, L2>(tm, w.Xt + D, T(0), T(1));
-  t_copy<T, TS, D, D, L1, L2>(tm, w.Z2, w.Xb);
-  t_fill<T, TS, D, D, L2>(tm, w.Xb + D, T(0), T(0));
-  t_tria<T, TS, D, D, D2, L2, L2>(tm, w.Xt, w.Xb, D);
-  t_mm<T, TS, D, D, D, L1, L1, L1, true, true>(tm, w.U1, w.A2, w.M);
-  t_copy<T, TS, D, D, L1, L1, true>(tm, w.U1, w.Mu);
+  constexpr int L1 = W::LD1, L2 = W::LD2;
+  const bool put = tm.r < D;
+  T x = t_dotrow<T, TS, D, D>(tm, w.U1, 1, L1, w.e2);
+  if (put) w.v1[tm.r] = x;
   tm.sync();
-  {  // M and Mu side by side on the two halves of the team
-    const Team<TS / 2> h;
-    t_trsm_l<T, TS / 2, D, D, L2, L1>(h, w.Xt, tm.r >= TS / 2 ? w.Mu : w.M);
-  }
+  x = t_dotrow<T, TS, D, D>(tm, w.U1, L1, 1, w.v1);
+  if (put) w.v2[tm.r] = w.b1[tm.r] + x;
+  t_filt_xi<T, TS, D>(tm, w);
+  x = t_dotrow<T, TS, D, D>(tm, w.Xb, 1, L2, w.v2);
+  if (put) w.v3[tm.r] = x;
+  t_copy<T, TS, D, D, L1, L2, true>(tm, w.M, w.UX + D);
+  t_copy<T, TS, D, D, L1, L2>(tm, w.U2, w.UX);
   tm.sync();
-  t_mv<T, TS, D, D, L1, true>(tm, w.U1, w.e2, w.v1);
+  x = t_dotrow<T, TS, D, D>(tm, w.Mu, 1, L1, w.v3);
+  if (put) w.v1[tm.r] = w.v2[tm.r] - x;
   tm.sync();
-  t_mv<T, TS, D, D, L1, false>(tm, w.U1, w.v1, w.v2);
-  tm.sync();
-  for (int i = tm.r; i < D; i += TS) w.v2[i] += w.b1[i];
-  tm.sync();
-  t_mv<T, TS, D, D, L2, true>(tm, w.Xb, w.v2, w.v3);
-  tm.sync();
-  t_mv<T, TS, D, D, L1, true>(tm, w.Mu, w.v3, w.v1);
-  tm.sync();
-  for (int i = tm.r; i < D; i += TS) w.v2[i] -= w.v1[i];
-  tm.sync();
-  t_mv<T, TS, D, D, L1, false>(tm, w.A2, w.v2, w.v3);
-  t_copy<T, TS, D, D, L1, L2, true>(tm, w.M, w.UX);
-  t_copy<T, TS, D, D, L1, L2>(tm, w.U2, w.UX + D);
-  tm.sync();
-  for (int i = tm.r; i < D; i += TS) w.b1[i] = w.v3[i] + w.b2[i];
-  t_tria<T, TS, D, 0, D2, L2, L2>(tm, w.UX, w.UX, D);
+  x = t_dotrow<T, TS, D, D>(tm, w.A2, L1, 1, w.v1);
+  if (put) w.b1[tm.r] = w.b2[tm.r] + x;
+  t_lq<T, TS, D, 0, L2, L2>(tm, w.UX, w.UX, TailFixed<D, 2 * D>{});
   t_copy<T, TS, D, D, L2, L1>(tm, w.UX, w.U1);
   tm.sync();
 }
@@ -416,7 +575,6 @@ struct SmoTeamWs {
   T E1[D * LD1], D1[D * LD1], g1[D];  // later element (or the state: D1 = L, g1 = m)
   T E2[D * LD1], D2m[D * LD1], g2[D];  // earlier element / running composite
   T X[D * LD2], En[D * LD1];
-  T v[D];
 };
 
 // composite (g2, E2, D2) <- (g2, E2, D2) o (g1, E1, D1)
@@ -424,14 +582,13 @@ struct SmoTeamWs {
 template <typename T, int TS, int D>
 __device__ __forceinline__ void t_smooth_combine(const Team<TS>& tm, SmoTeamWs<T, D>& w) {
   using W = SmoTeamWs<T, D>;
-  constexpr int L1 = W::LD1, L2 = W::LD2, D2 = W::D2;
-  t_mv<T, TS, D, D, L1, false>(tm, w.E2, w.g1, w.v);
-  t_mm<T, TS, D, D, D, L1, L1, L2>(tm, w.E2, w.D1, w.X);
-  t_copy<T, TS, D, D, L1, L2>(tm, w.D2m, w.X + D);
+  constexpr int L1 = W::LD1, L2 = W::LD2;
+  const T x = t_dotrow<T, TS, D, D>(tm, w.E2, L1, 1, w.g1);
+  t_mm_lowB<T, TS, D, D, L1, L1, L2>(tm, w.E2, w.D1, w.X + D);
+  t_copy<T, TS, D, D, L1, L2>(tm, w.D2m, w.X);
   t_mm<T, TS, D, D, D, L1, L1, L1>(tm, w.E2, w.E1, w.En);
-  tm.sync();
-  t_tria<T, TS, D, 0, D2, L2, L2>(tm, w.X, w.X, D);
-  for (int i = tm.r; i < D; i += TS) w.g2[i] += w.v[i];
+  t_lq<T, TS, D, 0, L2, L2>(tm, w.X, w.X, TailFixed<D, 2 * D>{});
+  if (tm.r < D) w.g2[tm.r] += x;
   t_copy<T, TS, D, D, L1, L1>(tm, w.En, w.E2);
   t_copy<T, TS, D, D, L2, L1>(tm, w.X, w.D2m);
   tm.sync();
@@ -441,13 +598,12 @@ __device__ __forceinline__ void t_smooth_combine(const Team<TS>& tm, SmoTeamWs<T
 template <typename T, int TS, int D>
 __device__ __forceinline__ void t_smooth_apply(const Team<TS>& tm, SmoTeamWs<T, D>& w) {
   using W = SmoTeamWs<T, D>;
-  constexpr int L1 = W::LD1, L2 = W::LD2, D2 = W::D2;
-  t_mv<T, TS, D, D, L1, false>(tm, w.E2, w.g1, w.v);
-  t_mm<T, TS, D, D, D, L1, L1, L2>(tm, w.E2, w.D1, w.X);
-  t_copy<T, TS, D, D, L1, L2>(tm, w.D2m, w.X + D);
-  tm.sync();
-  t_tria<T, TS, D, 0, D2, L2, L2>(tm, w.X, w.X, D);
-  for (int i = tm.r; i < D; i += TS) w.g1[i] = w.v[i] + w.g2[i];
+  constexpr int L1 = W::LD1, L2 = W::LD2;
+  const T x = t_dotrow<T, TS, D, D>(tm, w.E2, L1, 1, w.g1);
+  t_mm_lowB<T, TS, D, D, L1, L1, L2>(tm, w.E2, w.D1, w.X + D);
+  t_copy<T, TS, D, D, L1, L2>(tm, w.D2m, w.X);
+  t_lq<T, TS, D, 0, L2, L2>(tm, w.X, w.X, TailFixed<D, 2 * D>{});
+  if (tm.r < D) w.g1[tm.r] = x + w.g2[tm.r];
   t_copy<T, TS, D, D, L2, L1>(tm, w.X, w.D1);
   tm.sync();
 }
