@@ -102,27 +102,22 @@ template <typename T, int D, int DY, int TS>
 __global__ void kb_filt_l0_reduce(BView v, const T* __restrict__ F, const T* __restrict__ QL,
                                   const T* __restrict__ H, const T* __restrict__ c, T* __restrict__ out) {
   using WS = L0FoldWs<T, D, DY, false>;
-  POF_BL0_PROLOGUE(WS, D / DY)
+  POF_BL0_PROLOGUE(WS, (StepDims<T, D, DY>::Q1))
   if (t >= v.n1) return;
   if (v.frozen[v.cp[t]]) return;
   StepFoldWs<T, D, DY>& w = ws_.s;
-  constexpr int L1 = Ld<D>::v;
   const int64_t s0 = v.cs[t], s1 = v.ce[t];
-  t_fill<T, TS, D, D, L1>(tm, w.A, T(0), T(1));
-  t_fill<T, TS, D, D, L1>(tm, w.L, T(0), T(0));
-  t_fill<T, TS, D, D, L1>(tm, w.Z, T(0), T(0));
-  for (int i = tm.r; i < D; i += TS) {
-    w.b[i] = T(0);
-    w.eta[i] = T(0);
-  }
+  FoldRegs<T, D> fr;
+  t_fold_start<T, TS, D, DY>(tm, w, fr);
+  int nl = 0;
   for (int64_t s = s0; s < s1; ++s) {
     if (!POF_IN(s, v.n)) break;
-    t_load_step<T, TS, D, DY>(tm, w, H + s * DY * D, c + s * DY, nullptr);
+    const StepObs ob = t_load_step<T, TS, D, DY>(tm, w, H + s * DY * D, c + s * DY, (const T*)nullptr);
     tm.sync();
-    t_cond_fold_step<T, TS, D, DY>(tm, w, fq.F, fq.QL, StepStruct{fq.wq, fq.wf, true});
+    nl = t_cond_fold_step<T, TS, D, DY>(tm, w, fr, fq.F, fq.QL, StepStruct{fq.wq != 0, fq.wf}, ob, nl);
   }
   tm.sync();
-  t_store_filt<T, TS, D>(tm, out, v.n1, t, w.A, w.b, w.L, w.eta, w.Z);
+  t_store_fold<T, TS, D, DY>(tm, out, v.n1, t, w, fr);
 }
 
 // Filter levels >= 2: fold each group [goff[j], goff[j+1]) of level l - 1.
@@ -197,13 +192,12 @@ __global__ void kb_filt_l0_down(BView v, const T* __restrict__ F, const T* __res
                                 T* __restrict__ means, T* __restrict__ chols, T* __restrict__ selems,
                                 double* __restrict__ partials) {
   using WS = L0KFWs<T, D, DY, false>;
-  POF_BL0_PROLOGUE(WS, D / DY)
+  POF_BL0_PROLOGUE(WS, (StepDims<T, D, DY>::Q1))
   if (t >= v.n1) return;
   const int b = v.cp[t];
   if (v.frozen[b]) return;
   StepKFWs<T, D, DY>& w = ws_.s;
-  using GL = SmoLayout<D>;
-  constexpr int L1 = Ld<D>::v, L2 = Ld<2 * D>::v;
+  constexpr int L1 = Ld<D>::v;
   const int64_t s0 = v.cs[t], s1 = v.ce[t];
   const int64_t n = v.n;
   t_load_state<T, TS, D>(tm, states1, v.n1, t, w.m, w.L);
@@ -217,26 +211,18 @@ __global__ void kb_filt_l0_down(BView v, const T* __restrict__ F, const T* __res
         chols[g * D * D + f - D] = w.L[((f - D) / D) * L1 + (f - D) % D];
     }
   }
-  double ssq = 0.0, nll = 0.0, fobj = 0.0;
+  bool lower;
+  int nl = t_ncols<T, TS, D, D, L1>(tm, w.L, &lower);
+  double ssq = 0.0, yy = 0.0;
+  LogProd lp;
   for (int64_t s = s0; s < s1; ++s) {
     if (!POF_IN(s + 1, v.n)) break;  // writes grid point s + 1
-    t_load_step<T, TS, D, DY>(tm, w, H + s * DY * D, c + s * DY, nullptr);
-    for (int i = tm.r; i < D; i += TS) ws_.mold[i] = w.m[i];
+    const StepObs ob = t_load_step<T, TS, D, DY>(tm, w, H + s * DY * D, c + s * DY, (const T*)nullptr);
     tm.sync();
-    t_kf_step<T, TS, D, DY, true>(tm, w, fq.F, fq.QL, StepStruct{fq.wq, fq.wf, true});
-    ssq += (double)w.sc[0];
-    nll += (double)w.sc[1];
-    fobj += (double)t_objective<T, TS, D>(tm, fq.F, fq.QLi, ws_.mold, w.m, ws_.r);
-    for (int f = tm.r; f < GL::NG; f += TS) {
-      T val;
-      if (f < GL::E)
-        val = w.g[f];
-      else if (f < GL::DM)
-        val = w.E[((f - GL::E) % D) * L1 + (f - GL::E) / D];
-      else
-        val = w.Y[((f - GL::DM) / D) * L2 + D + (f - GL::DM) % D];
-      selems[f * n + s] = val;
-    }
+    const int nk = nl;
+    nl = t_kf_step<T, TS, D, DY, true>(tm, w, fq.F, fq.QL, StepStruct{fq.wq != 0, fq.wf}, ob, nl, lower, ssq, yy, lp);
+    lower = true;
+    t_store_selem<T, TS, D, DY>(tm, selems, n, s, w, nk);
     const int64_t g = s + 1;
     for (int f = tm.r; f < D + D * D; f += TS) {
       if (f < D)
@@ -246,11 +232,7 @@ __global__ void kb_filt_l0_down(BView v, const T* __restrict__ F, const T* __res
     }
     tm.sync();
   }
-  if (tm.r == 0) {
-    partials[P_SSQ * v.n1 + t] = ssq;
-    partials[P_NLL * v.n1 + t] = nll;
-    partials[P_FOBJ * v.n1 + t] = fobj;
-  }
+  t_store_partials<TS, DY>(tm, partials, v.n1, t, ssq, yy, lp, s1 - s0, 0.0);
 }
 
 // Smoother level 0: composite of each chunk's smoother elements.
@@ -266,9 +248,10 @@ __global__ void kb_smo_l0_reduce(BView v, const T* __restrict__ selems, T* __res
   for (int64_t i = i0 + 1; i < i1; ++i) {
     t_load_smo<T, TS, D>(tm, selems, v.n, i, w.g1, w.E1, w.D1);
     tm.sync();
-    t_smooth_combine<T, TS, D>(tm, w);
+    t_smooth_combine_raw<T, TS, D>(tm, w, i == i0 + 1);
   }
   tm.sync();
+  if (i1 - i0 == 1) t_smooth_tria<T, TS, D>(tm, w);
   t_store_smo<T, TS, D>(tm, out, v.n1, t, w.g2, w.E2, w.D2m);
 }
 
@@ -339,13 +322,13 @@ __global__ void kb_smo_down(const int64_t* __restrict__ goff, const int32_t* __r
 // given (pof/step.py:42-44), with the chunk's smoother-objective and
 // convergence-test sums (convergence_criteria.py:10).
 template <typename T, int D, int TS>
-__global__ void kb_smo_l0_down(BView v, const T* __restrict__ F, const T* __restrict__ QL,
+__global__ void kb_smo_l0_down(BView v, const T* __restrict__ F, const T* __restrict__ QL, int Q,
                                const T* __restrict__ selems, const T* __restrict__ ends1, T* __restrict__ means,
                                T* __restrict__ chols, const double* __restrict__ scale,
                                const T* __restrict__ means_old, double c_mrtol, double c_matol,
                                double* __restrict__ partials) {
   using WS = SmoL0Ws<T, D, false>;
-  POF_BL0_PROLOGUE(WS, 0)
+  POF_BL0_PROLOGUE(WS, Q)
   if (t >= v.n1) return;
   const int b = v.cp[t];
   if (v.frozen[b]) return;
@@ -355,7 +338,10 @@ __global__ void kb_smo_l0_down(BView v, const T* __restrict__ F, const T* __rest
   const T sc = scale ? (T)scale[b] : T(1);
   t_load_state<T, TS, D>(tm, ends1, v.n1, t, w.g1, w.D1);
   tm.sync();
-  double sobj = 0.0, notclose = 0.0;
+  bool lower;
+  t_ncols<T, TS, D, D, L1>(tm, w.D1, &lower);
+  double sobj = 0.0;
+  int notclose = 0;
   auto close_count = [&](int64_t g) {
     if (!means_old) return;
     for (int i = tm.r; i < D; i += TS) {
@@ -365,7 +351,7 @@ __global__ void kb_smo_l0_down(BView v, const T* __restrict__ F, const T* __rest
         ok = fabs(a - bb) <= c_matol + c_mrtol * fabs(bb);
       else
         ok = (a == bb);
-      notclose += ok ? 0.0 : 1.0;
+      notclose += ok ? 0 : 1;
     }
   };
   if (s1 == v.gb[b] + v.ns[b]) {  // last chunk: the terminal grid point
@@ -379,22 +365,24 @@ __global__ void kb_smo_l0_down(BView v, const T* __restrict__ F, const T* __rest
     for (int i = tm.r; i < D; i += TS) ws_.mnext[i] = w.g1[i];
     t_load_smo<T, TS, D>(tm, selems, v.n, k, w.g2, w.E2, w.D2m);
     tm.sync();
-    t_smooth_apply<T, TS, D>(tm, w);
-    sobj += (double)t_objective<T, TS, D>(tm, fq.F, fq.QLi, w.g1, ws_.mnext, ws_.r);
+    t_smooth_apply_raw<T, TS, D>(tm, w, lower);
+    lower = true;
+    sobj += (double)t_objective<T, TS, D>(tm, fq.F, fq.QLi, w.g1, ws_.mnext, ws_.r, fq.wf);
     const int64_t g = k;
     close_count(g);
     for (int f = tm.r; f < D + D * D; f += TS) {
       if (f < D)
         means[g * D + f] = w.g1[f];
       else
-        chols[g * D * D + f - D] = w.D1[((f - D) / D) * L1 + (f - D) % D] * sc;
+        chols[g * D * D + f - D] = scale ? w.D1[((f - D) / D) * L1 + (f - D) % D] * sc
+                                         : w.D1[((f - D) / D) * L1 + (f - D) % D];
     }
     tm.sync();
   }
-  notclose = (double)tm.sum(notclose);
+  notclose = (int)__reduce_add_sync(tm.mask, (unsigned)notclose);
   if (tm.r == 0) {
     partials[P_SOBJ * v.n1 + t] = sobj;
-    partials[P_NOTCLOSE * v.n1 + t] = notclose;
+    partials[P_NOTCLOSE * v.n1 + t] = (double)notclose;
   }
 }
 
@@ -424,14 +412,12 @@ static __global__ void kb_fin_filter(BView v, const double* __restrict__ partial
   const int64_t c0 = v.pc[k], c1 = v.pc[k + 1];
   const double ssq = warp_chunk_sum(partials + P_SSQ * v.n1, c0, c1, lane);
   const double nll = warp_chunk_sum(partials + P_NLL * v.n1, c0, c1, lane);
-  const double fobj = warp_chunk_sum(partials + P_FOBJ * v.n1, c0, c1, lane);
   if (lane == 0) {
     const double nb = (double)v.ns[b];
     const double s = ssq / nb / (double)DY;
     double* sc = pscal + (int64_t)kBatchScalars * b;
     sc[S_SSQ] = s;
     sc[S_NLL] = nll;
-    sc[S_FOBJ] = fobj;
     pscale[b] = sqrt(s);
   }
 }
@@ -842,7 +828,8 @@ struct BatchDriver {
     }
     {
       ProfScope ps(PK_SMO_L0_DOWN, st);
-      launch_l0<TS, SmoL0Ws<T, D, false>>(kb_smo_l0_down<T, D, TS>, n1, st, v, F, QL, (const T*)selem,
+      launch_l0<TS, SmoL0Ws<T, D, false>>(kb_smo_l0_down<T, D, TS>, n1, st, v, F, QL, StepDims<T, D, DY>::Q1,
+                                          (const T*)selem,
                                           (const T*)at<T>(lw, L.gend[1]), mnew, chols,
                                           a.calibrate ? (const double*)a.pscale : nullptr, mold, a.mrtol, a.matol,
                                           at<double>(lw, L.partials));

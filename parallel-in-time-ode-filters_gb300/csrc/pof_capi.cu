@@ -665,6 +665,7 @@ MixedLayout mixed_layout(int64_t n, int D, int d) {
   MixedLayout m;
   m.p64 = plan_for(POF_F64, n, D, d, true);
   m.p32 = plan_for(POF_F32, n, D, d, false);
+  m.p32.fobj = false;
   size_t off = align_up(m.p64.total);
   m.off32 = off;
   off = align_up(off + m.p32.total);

@@ -145,8 +145,8 @@ inline void launch_team(void (*kern)(KArgs...), int64_t nteams, cudaStream_t st,
 
 // Upper-level launches with few combines (at most this many lanes of wide
 // teams) use the wide teams: they are latency-bound, and a wider team
-// shortens each combine's chain of FP64 instructions (t_tria's column
-// phases, more outputs per t_mm step).  POF_WIDE_LANES overrides.
+// shortens each combine's chain of FP64 instructions (t_lq's lanes per
+// row, more outputs per t_mm step).  POF_WIDE_LANES overrides.
 int wide_lane_limit();
 
 template <typename T, int D, int DY>
@@ -165,6 +165,13 @@ struct Driver {
   static void launch_l0(void (*kern)(KArgs...), int64_t nteams, cudaStream_t st, Args... args) {
     using B = TeamBlockH<WS, TS, FQHeader<T, D, PS>::bytes>;
     const unsigned grid = (unsigned)((nteams + B::teams - 1) / B::teams);
+    kern<<<grid, B::threads, B::smem, st>>>(args...);
+  }
+  // the fold: chunk 0 in a block of its own
+  template <int TS, bool PS, typename WS, typename... KArgs, typename... Args>
+  static void launch_l0_fold(void (*kern)(KArgs...), int64_t nteams, cudaStream_t st, Args... args) {
+    using B = TeamBlockH<WS, TS, FQHeader<T, D, PS>::bytes>;
+    const unsigned grid = 1 + (unsigned)((nteams - 1 + B::teams - 1) / B::teams);
     kern<<<grid, B::threads, B::smem, st>>>(args...);
   }
 
@@ -207,10 +214,10 @@ struct Driver {
       ProfScope ps(PK_FILT_L0_REDUCE, st);
       if constexpr (kTeamL0) {
         if (sm.ft_stride)
-          launch_l0<TS, true, L0FoldWs<T, D, DY, true>>(k_filt_l0_reduce_team<T, D, DY, TS, true>, n1, st, n, p.C0,
+          launch_l0_fold<TS, true, L0FoldWs<T, D, DY, true>>(k_filt_l0_reduce_team<T, D, DY, TS, true>, n1, st, n, p.C0,
                                                         sm, x0m, x0L, b.template at<T>(p.felem[1]), n1);
         else
-          launch_l0<TS, false, L0FoldWs<T, D, DY, false>>(k_filt_l0_reduce_team<T, D, DY, TS, false>, n1, st, n,
+          launch_l0_fold<TS, false, L0FoldWs<T, D, DY, false>>(k_filt_l0_reduce_team<T, D, DY, TS, false>, n1, st, n,
                                                           p.C0, sm, x0m, x0L, b.template at<T>(p.felem[1]), n1);
       }
       else
@@ -262,11 +269,13 @@ struct Driver {
         if (sm.ft_stride)
           launch_l0<TS, true, L0KFWs<T, D, DY, true>>(k_filt_l0_down_team<T, D, DY, TS, true>, n1, st, n, p.C0, sm,
                                                       (const T*)b.template at<T>(p.fstate[1]), n1, means, chols,
-                                                      b.template at<T>(p.selem), b.template at<double>(p.partials));
+                                                      b.template at<T>(p.selem), b.template at<double>(p.partials),
+                                                      p.fobj);
         else
           launch_l0<TS, false, L0KFWs<T, D, DY, false>>(k_filt_l0_down_team<T, D, DY, TS, false>, n1, st, n, p.C0,
                                                         sm, (const T*)b.template at<T>(p.fstate[1]), n1, means, chols,
-                                                        b.template at<T>(p.selem), b.template at<double>(p.partials));
+                                                        b.template at<T>(p.selem), b.template at<double>(p.partials),
+                                                        p.fobj);
       }
       else
         k_filt_l0_down<T, D, DY><<<grid_for(n1, kBlock), kBlock, 0, st>>>(
@@ -293,7 +302,7 @@ struct Driver {
     if (n1 > 1 || p.ks) {
       ProfScope ps(PK_SMO_L0_REDUCE, st);
       if constexpr (kTeamL0)
-        launch_team<SWS, TS>(k_smo_reduce_team<T, D, TS>, n1, st, (const T*)b.template at<T>(p.selem), n, p.C0,
+        launch_team<SWS, TS>(k_smo_l0_reduce_team<T, D, TS>, n1, st, (const T*)b.template at<T>(p.selem), n, p.C0,
                              b.template at<T>(p.gelem[1]), n1);
       else
         k_smo_reduce<T, D><<<grid_for(n1, kBlock), kBlock, 0, st>>>(b.template at<T>(p.selem), n, p.C0,
@@ -349,12 +358,14 @@ struct Driver {
       if constexpr (kTeamL0) {
         if (ft_stride)
           launch_l0<TS, true, SmoL0Ws<T, D, true>>(k_smo_l0_down_team<T, D, TS, true>, n1, st, n, p.C0, F, QL,
-                                                   ft_stride, (const T*)b.template at<T>(p.selem),
+                                                   ft_stride, StepDims<T, D, DY>::Q1,
+                                                   (const T*)b.template at<T>(p.selem),
                                                    (const T*)b.template at<T>(p.gend[1]), n1, means, chols, scl,
                                                    means_old, p.mrtol, p.matol, b.template at<double>(p.partials));
         else
           launch_l0<TS, false, SmoL0Ws<T, D, false>>(k_smo_l0_down_team<T, D, TS, false>, n1, st, n, p.C0, F, QL,
-                                                     ft_stride, (const T*)b.template at<T>(p.selem),
+                                                     ft_stride, StepDims<T, D, DY>::Q1,
+                                                     (const T*)b.template at<T>(p.selem),
                                                      (const T*)b.template at<T>(p.gend[1]), n1, means, chols, scl,
                                                      means_old, p.mrtol, p.matol, b.template at<double>(p.partials));
       }

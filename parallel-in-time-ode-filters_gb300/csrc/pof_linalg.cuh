@@ -132,16 +132,24 @@ __device__ __forceinline__ void householder(T alpha, T xn2, T& beta, T& tau, T& 
 __device__ __forceinline__ bool is_zero(double x) { return (__double_as_longlong(x) << 1) == 0; }
 __device__ __forceinline__ bool is_zero(float x) { return (__float_as_uint(x) << 1) == 0; }
 
-// The same reflector in the unnormalized form H = I + kap v v^T with
-// v = (u, x), u = alpha - beta, kap = 1 / (u beta): the tail x is used as it
-// is (no pass that scales it), and the squared norm can be formed together
-// with the dot products of the rows below.  For xn2 != 0 only.  Double
-// precision: ||(alpha, x)|| = h and 1 / (u beta) = -1 / (a2 + |alpha| h) from
-// single-precision seeds and one third-order correction each (as rsqrt_nr and
-// rcp_nr): 11 FP64 instructions.
+// The same reflector with the tail x left as it is, so the squared norm can be
+// formed together with the dot products of the rows below and no pass scales
+// x: a row (a, y) with dot = y . x becomes (a - w, y - ws x), where
+//   double: H = I + kap v v^T, v = (u, x), u = alpha - beta, kap = 1 / (u beta):
+//     ws = -kap (u a + dot), w = u ws; ||(alpha, x)|| = h and
+//     1 / (u beta) = -1 / (a2 + |alpha| h) from single-precision seeds and one
+//     third-order correction each (as rsqrt_nr and rcp_nr), 11 FP64
+//     instructions of scalars and 2 per row;
+//   float: w = tau (a + scal dot), ws = w scal (kap would leave float's range
+//     for tails below 1e-19).
+// For xn2 != 0 only.
 template <typename T>
-__device__ __forceinline__ void reflector(T alpha, T xn2, T& beta, T& u, T& kap) {
-  if constexpr (std::is_same<T, double>::value) {
+struct Reflector;
+
+template <>
+struct Reflector<double> {
+  double beta, u, kap;
+  __device__ __forceinline__ Reflector(double alpha, double xn2) {
     const double a2 = fma(alpha, alpha, xn2);
     const long long bits = __double_as_longlong(a2);
     const int e = (int)((bits >> 52) & 0x7ff) - 1023;
@@ -161,14 +169,25 @@ __device__ __forceinline__ void reflector(T alpha, T xn2, T& beta, T& u, T& kap)
     const bool neg = ab < 0 && (ab << 1) != 0;
     beta = neg ? h : __longlong_as_double(__double_as_longlong(h) ^ (1LL << 63));
     u = alpha - beta;
-    kap = -rcp_nr(fma(fabs(alpha), h, a2));
-  } else {
-    const T nrm = sqrt(fma(alpha, alpha, xn2));
-    beta = alpha >= T(0) ? -nrm : nrm;
-    u = alpha - beta;
-    kap = T(1) / (u * beta);
+    kap = rcp_nr(fma(fabs(alpha), h, a2));  // -1 / (u beta)
   }
-}
+  // new pivot entry; ws: the multiple of x taken off the row's tail
+  __device__ __forceinline__ double row(double a, double dot, double& ws) const {
+    ws = kap * fma(u, a, dot);
+    return fma(-ws, u, a);
+  }
+};
+
+template <>
+struct Reflector<float> {
+  float beta, tau, scal;
+  __device__ __forceinline__ Reflector(float alpha, float xn2) { householder(alpha, xn2, beta, tau, scal); }
+  __device__ __forceinline__ float row(float a, float dot, float& ws) const {
+    const float w = tau * fmaf(scal, dot, a);
+    ws = w * scal;
+    return a - w;
+  }
+};
 
 // C(MxN) = A(MxK) * B(KxN)
 template <typename T, int M, int K, int N, int LDA, int LDB, int LDC>

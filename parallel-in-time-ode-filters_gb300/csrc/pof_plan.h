@@ -28,6 +28,9 @@ struct Plan {
   // means test of the convergence criterion: isclose(old, new, mrtol, matol)
   // (pof/convergence_criteria.py:10 uses rtol 1e-13 and numpy's atol 1e-8)
   double mrtol = 1e-13, matol = 1e-8;
+  // compute the filter objective: reported by the filter/smoother entry
+  // points, read by nobody in the solve loops
+  bool fobj = true;
   int64_t cnt[kMaxLevels] = {0};  // cnt[l], l = 1..nlev (cnt[nlev] <= kTop)
   size_t felem[kMaxLevels] = {0}, fstate[kMaxLevels] = {0}, gelem[kMaxLevels] = {0}, gend[kMaxLevels] = {0};
   size_t selem = 0, partials = 0, scalars = 0, scale = 0;
@@ -100,6 +103,7 @@ inline Plan make_plan(int64_t n, int D, int DY, int esz, bool with_solver, int C
   p.D = D;
   p.DY = DY;
   p.esz = esz;
+  p.fobj = !with_solver;
   p.team = team_lanes(D, !narrow);  // level 0: narrow unless told otherwise
   p.team_up = team_lanes(D, false);
   p.C0 = C0 > 0 ? C0 : pick_c0(n, l0_lanes(D, !narrow));

@@ -76,105 +76,6 @@ __device__ __forceinline__ void t_mv(const Team<TS>& tm, const T* A, const T* x,
   }
 }
 
-// In-place tria of an M x NC matrix X (M <= NC) stacked with MB more rows Y
-// (Y gets the same reflectors; pass MB = 0 for plain tria).  Same
-// reflectors and sign conventions as pof::tria (LAPACK dgeqr2/dlarfg).
-// The norm is a team reduction over columns; the row updates run one row per
-// lane.  Zeroes X's tails at the end.
-//
-// wlow > 0 declares X = [X1, X2] with X2 = X[:, wlow:] lower-triangular and
-// Y[:, wlow:] zero (the shape of every tria([A, L]) of the filter and
-// smoother: [F L, QL], [U1^T Z2, I], [M^T, U2], [E L, D], ...).  Reflector j
-// then has no entry beyond column wlow + j (row j of X2 starts with j + 1
-// nonzeros and the earlier reflectors only fill columns below wlow + j), so
-// its norm, the dot products and the row updates stop there: the same
-// arithmetic without the exact zeros.  ncut < NC declares the columns from
-// ncut on zero in every row (the observation block [[H Lp, 0], [Lp, 0]] of a
-// noiseless update): they stay zero, and the reflectors from ncut - 1 on
-// have an empty tail (no reflection: LAPACK's tau = 0, beta = alpha), so
-// they are skipped.
-//
-// A team with at least twice as many lanes as a reflector has rows to update
-// (M - 1 + MB) gives each row G = TS / RS lanes (RS: row slots, the next
-// power of two): lane phase p takes the columns j + 1 + p, j + 1 + p + G, ...,
-// the G partial dot products are summed by shuffles, and each lane updates
-// its own columns -- G times fewer FP64 instructions per reflector on the
-// latency-bound combines of the upper levels.
-template <int R, int TS>
-struct RowSlots {
-  static constexpr int p2 = R <= 1 ? 1 : (R <= 2 ? 2 : (R <= 4 ? 4 : (R <= 8 ? 8 : (R <= 16 ? 16 : 32))));
-  static constexpr int v = p2 < TS ? p2 : TS;
-};
-
-template <typename T, int TS, int M, int MB, int NC, int LD, int LDY>
-__device__ __forceinline__ void t_tria(const Team<TS>& tm, T* X, T* Y, int wlow = 0, int ncut = NC) {
-  constexpr int RS = RowSlots<M - 1 + MB, TS>::v;
-  constexpr int G = TS / RS;
-  const int src = (threadIdx.x & 31) / TS * TS;  // lane 0 of this team within the warp
-  const int mlim = (ncut < NC && ncut - 1 < M) ? ncut - 1 : M;
-#pragma unroll 1
-  for (int j = 0; j < mlim; ++j) {
-    T* xj = X + j * LD;
-    int kend = (wlow > 0 && wlow + j + 1 < NC) ? wlow + j + 1 : NC;
-    if (ncut < kend) kend = ncut;
-    tm.sync();
-    // ||x[j, j+1:]||^2: column partials, reduced onto lane 0 (the only one
-    // that uses it) over the lanes that hold partials -- the same additions as
-    // the full butterfly, without the ones of zeros
-    T part = T(0);
-    for (int k = j + 1 + tm.r; k < kend; k += TS) part = fma(xj[k], xj[k], part);
-    int span = 1;
-    while (span < kend - j - 1 && span < TS) span <<= 1;
-    for (int o = span >> 1; o > 0; o >>= 1) part += __shfl_xor_sync(tm.mask, part, o, TS);
-    const T xn2 = part;
-    // the reflector's scalars on one lane (a square root and two divisions
-    // are long FP64 sequences), then broadcast
-    T tau = T(0), scal = T(0), beta = T(0);
-    if (tm.r == 0) householder(xj[j], xn2, beta, tau, scal);
-    tau = __shfl_sync(tm.mask, tau, src);
-    scal = __shfl_sync(tm.mask, scal, src);
-    tm.sync();
-    for (int k = j + 1 + tm.r; k < kend; k += TS) xj[k] *= scal;
-    if (tm.r == 0) xj[j] = beta;
-    tm.sync();
-    // rows below j (X rows j+1..M-1, then Y rows 0..MB-1)
-    if constexpr (G == 1) {  // one row per lane
-      for (int rr = tm.r; rr < (M - j - 1) + MB; rr += TS) {
-        T* xi = (rr < M - j - 1) ? X + (j + 1 + rr) * LD : Y + (rr - (M - j - 1)) * LDY;
-        T w = xi[j];
-        for (int k = j + 1; k < kend; ++k) w = fma(xi[k], xj[k], w);
-        w *= tau;
-        xi[j] -= w;
-        for (int k = j + 1; k < kend; ++k) xi[k] = fma(-w, xj[k], xi[k]);
-      }
-    } else {  // G lanes per row, column phases; the shuffles need every lane
-      const int slot = tm.r % RS, ph = tm.r / RS;
-      const int nrows = (M - j - 1) + MB;
-      for (int base = 0; base < nrows; base += RS) {
-        const int rr = base + slot;
-        const bool act = rr < nrows;
-        T* xi = act ? ((rr < M - j - 1) ? X + (j + 1 + rr) * LD : Y + (rr - (M - j - 1)) * LDY) : X;
-        T part = (act && ph == 0) ? xi[j] : T(0);
-        if (act)
-          for (int k = j + 1 + ph; k < kend; k += G) part = fma(xi[k], xj[k], part);
-#pragma unroll
-        for (int o = RS; o < TS; o <<= 1) part += __shfl_xor_sync(tm.mask, part, o, TS);
-        if (act) {
-          const T w = part * tau;
-          if (ph == 0) xi[j] -= w;
-          for (int k = j + 1 + ph; k < kend; k += G) xi[k] = fma(-w, xj[k], xi[k]);
-        }
-      }
-    }
-  }
-  tm.sync();
-  for (int idx = tm.r; idx < M * NC; idx += TS) {
-    const int i = idx / NC, k = idx % NC;
-    if (k > i) X[i * LD + k] = T(0);
-  }
-  tm.sync();
-}
-
 // ---------------------------------------------------------------------------
 // LQ with a triangular pivot block.  Rows [P | W] (M rows, pivot entry (j, j)
 // of row j in column j, tail columns [kb(j), ke(j)) given by `tail`) and MB
@@ -212,6 +113,25 @@ template <int KB, int KE>
 struct TailFixed {  // the same columns for every reflector
   static constexpr int count = KE - KB;
   __device__ __forceinline__ void operator()(int, int& b, int& e) const { b = KB, e = KE; }
+};
+struct TailRange {  // the same columns for every reflector, found at run time
+  static constexpr int count = 0;  // not a constant
+  int kb, ke;
+  __device__ __forceinline__ void operator()(int, int& b, int& e) const { b = kb, e = ke; }
+};
+// [L | F S] with a block-diagonal F (blocks of Q) and a lower-triangular S of
+// `n` nonzero columns: row j of F S, in block j / Q, has no entry beyond
+// column (j / Q + 1) Q - 1, and the reflectors before j fill no further.
+// Q = 0: no such structure.
+template <int Q>
+struct TailBlocks {
+  static constexpr int count = 0;
+  int kb, n;
+  __device__ __forceinline__ void operator()(int j, int& b, int& e) const {
+    int w = n;
+    if constexpr (Q > 0) w = min((j / Q + 1) * Q, n);
+    b = kb, e = kb + w;
+  }
 };
 struct TailUpper {  // the columns right of the diagonal, up to `n`
   static constexpr int count = 0;  // not a constant
@@ -271,24 +191,23 @@ __device__ __forceinline__ void t_lq(const Team<TS>& tm, T* X, T* Y, const Tail&
     const T xn2 = __shfl_sync(tm.mask, dot[0], src);
     pj = -1;
     if (is_zero(xn2)) continue;
-    T beta, u, kap;
-    reflector(alpha, xn2, beta, u, kap);
-    pend = beta;
+    const Reflector<T> h(alpha, xn2);
+    pend = h.beta;
     pj = j;
 #pragma unroll
     for (int p = 0; p < NP; ++p) {
       const int e = slot + p * RS;
       if (e == 0 || e >= ne) continue;
       T* xi = row[p];
-      const T a = xi[j];
-      const T w = kap * fma(u, a, dot[p]);
-      if (ph == 0) xi[j] = fma(w, u, a);
+      T ws;
+      const T a = h.row(xi[j], dot[p], ws);
+      if (ph == 0) xi[j] = a;
       if constexpr (Tail::count > 0 && Tail::count % G == 0) {
 #pragma unroll
-        for (int t = 0; t < Tail::count; t += G) xi[kb + ph + t] = fma(w, xj[kb + ph + t], xi[kb + ph + t]);
+        for (int t = 0; t < Tail::count; t += G) xi[kb + ph + t] = fma(-ws, xj[kb + ph + t], xi[kb + ph + t]);
       } else {
 #pragma unroll 2
-        for (int k = kb + ph; k < ke; k += G) xi[k] = fma(w, xj[k], xi[k]);
+        for (int k = kb + ph; k < ke; k += G) xi[k] = fma(-ws, xj[k], xi[k]);
       }
     }
   }
@@ -595,16 +514,126 @@ __device__ __forceinline__ void t_smooth_combine(const Team<TS>& tm, SmoTeamWs<T
 }
 
 // state (g1 = m, D1 = L) <- element (g2, E2, D2) applied: m = E m + g, L = tria([E L, D])
+// (L any square root: the terminal state may be the caller's)
 template <typename T, int TS, int D>
 __device__ __forceinline__ void t_smooth_apply(const Team<TS>& tm, SmoTeamWs<T, D>& w) {
   using W = SmoTeamWs<T, D>;
   constexpr int L1 = W::LD1, L2 = W::LD2;
   const T x = t_dotrow<T, TS, D, D>(tm, w.E2, L1, 1, w.g1);
-  t_mm_lowB<T, TS, D, D, L1, L1, L2>(tm, w.E2, w.D1, w.X + D);
+  t_mm<T, TS, D, D, D, L1, L1, L2>(tm, w.E2, w.D1, w.X + D);
   t_copy<T, TS, D, D, L1, L2>(tm, w.D2m, w.X);
   t_lq<T, TS, D, 0, L2, L2>(tm, w.X, w.X, TailFixed<D, 2 * D>{});
   if (tm.r < D) w.g1[tm.r] = x + w.g2[tm.r];
   t_copy<T, TS, D, D, L2, L1>(tm, w.X, w.D1);
+  tm.sync();
+}
+
+// Number of columns of A (M x N, leading dimension LDA) up to the last one with
+// a nonzero entry, and whether A is lower triangular (integer operations only).
+template <typename T, int TS, int M, int N, int LDA>
+__device__ __forceinline__ int t_ncols(const Team<TS>& tm, const T* A, bool* lower = nullptr) {
+  int nc = 0;
+  bool up = false;
+  for (int idx = tm.r; idx < M * N; idx += TS) {
+    const int i = idx / N, j = idx % N;
+    if (!is_zero(A[i * LDA + j])) {
+      nc = max(nc, j + 1);
+      up |= j > i;
+    }
+  }
+  if (lower) *lower = !__any_sync(tm.mask, up);
+  return (int)__reduce_max_sync(tm.mask, (unsigned)nc);
+}
+
+// ---------------------------------------------------------------------------
+// Level-0 smoother operations.  The elements' factors Dm are raw square roots
+// (D x nk, not triangular: see t_kf_step), nk their column count.
+// ---------------------------------------------------------------------------
+
+// C(M x nc) = A(M x N) B, the first nc columns of B
+template <typename T, int TS, int M, int N, int LDA, int LDB, int LDC>
+__device__ __forceinline__ void t_mm_cols(const Team<TS>& tm, const T* A, const T* B, T* C, int nc) {
+  constexpr int RS = Pow2Ceil<M>::v < TS ? Pow2Ceil<M>::v : TS;
+  constexpr int CG = TS / RS;
+#pragma unroll
+  for (int i0 = 0; i0 < M; i0 += RS) {
+    const int i = i0 + tm.r % RS;
+    if (M % RS != 0 && i >= M) continue;
+    T a[N];
+#pragma unroll
+    for (int k = 0; k < N; ++k) a[k] = A[i * LDA + k];
+    for (int j = tm.r / RS; j < nc; j += CG) {
+      T s = T(0);
+#pragma unroll
+      for (int k = 0; k < N; ++k) s = fma(a[k], B[k * LDB + j], s);
+      C[i * LDC + j] = s;
+    }
+  }
+}
+
+// Dm <- its triangular form
+template <typename T, int TS, int D>
+__device__ __forceinline__ void t_smooth_tria(const Team<TS>& tm, SmoTeamWs<T, D>& w) {
+  using W = SmoTeamWs<T, D>;
+  constexpr int L1 = W::LD1;
+  const int nk = t_ncols<T, TS, D, D, L1>(tm, w.D2m);
+  t_lq<T, TS, D, 0, L1, L1>(tm, w.D2m, w.D2m, TailUpper{nk});
+  for (int idx = tm.r; idx < D * D; idx += TS) {
+    const int i = idx / D, k = idx % D;
+    if (k > i) w.D2m[i * L1 + k] = T(0);
+  }
+  tm.sync();
+}
+
+// t_smooth_combine with a raw D1; `first`: the composite's D2 is raw too.
+template <typename T, int TS, int D>
+__device__ __forceinline__ void t_smooth_combine_raw(const Team<TS>& tm, SmoTeamWs<T, D>& w, bool first) {
+  using W = SmoTeamWs<T, D>;
+  constexpr int L1 = W::LD1, L2 = W::LD2;
+  const int n1 = t_ncols<T, TS, D, D, L1>(tm, w.D1);
+  const T x = t_dotrow<T, TS, D, D>(tm, w.E2, L1, 1, w.g1);
+  t_mm<T, TS, D, D, D, L1, L1, L1>(tm, w.E2, w.E1, w.En);
+  if (first) {  // [E2 D1 | D2], both dense
+    const int n2 = t_ncols<T, TS, D, D, L1>(tm, w.D2m);
+    t_mm_cols<T, TS, D, D, L1, L1, L2>(tm, w.E2, w.D1, w.X, n1);
+    for (int idx = tm.r; idx < D * D; idx += TS) {
+      const int i = idx / D, k = idx % D;
+      if (n1 + k < 2 * D) w.X[i * L2 + n1 + k] = w.D2m[i * L1 + k];  // zero from column n1 + n2 on
+    }
+    t_lq<T, TS, D, 0, L2, L2>(tm, w.X, w.X, TailUpper{n1 + n2});
+  } else {  // [D2 | E2 D1]
+    t_mm_cols<T, TS, D, D, L1, L1, L2>(tm, w.E2, w.D1, w.X + D, n1);
+    t_copy<T, TS, D, D, L1, L2>(tm, w.D2m, w.X);
+    t_lq<T, TS, D, 0, L2, L2>(tm, w.X, w.X, TailRange{D, D + n1});
+  }
+  if (tm.r < D) w.g2[tm.r] += x;
+  t_copy<T, TS, D, D, L1, L1>(tm, w.En, w.E2);
+  for (int idx = tm.r; idx < D * D; idx += TS) {
+    const int i = idx / D, k = idx % D;
+    w.D2m[i * L1 + k] = k <= i ? w.X[i * L2 + k] : T(0);
+  }
+  tm.sync();
+}
+
+// t_smooth_apply with a raw D2: L = tria([E L, D2]); `lower`: L is lower
+// triangular (every state but a caller's terminal one).
+template <typename T, int TS, int D>
+__device__ __forceinline__ void t_smooth_apply_raw(const Team<TS>& tm, SmoTeamWs<T, D>& w, bool lower) {
+  using W = SmoTeamWs<T, D>;
+  constexpr int L1 = W::LD1, L2 = W::LD2;
+  const int nk = t_ncols<T, TS, D, D, L1>(tm, w.D2m);
+  const T x = t_dotrow<T, TS, D, D>(tm, w.E2, L1, 1, w.g1);
+  if (lower)
+    t_mm_lowB<T, TS, D, D, L1, L1, L2>(tm, w.E2, w.D1, w.X);
+  else
+    t_mm<T, TS, D, D, D, L1, L1, L2>(tm, w.E2, w.D1, w.X);
+  t_copy<T, TS, D, D, L1, L2>(tm, w.D2m, w.X + D);
+  t_lq<T, TS, D, 0, L2, L2>(tm, w.X, w.X, TailUpper{D + nk});
+  if (tm.r < D) w.g1[tm.r] = x + w.g2[tm.r];
+  for (int idx = tm.r; idx < D * D; idx += TS) {
+    const int i = idx / D, k = idx % D;
+    w.D1[i * L1 + k] = k <= i ? w.X[i * L2 + k] : T(0);
+  }
   tm.sync();
 }
 
@@ -613,13 +642,31 @@ __device__ __forceinline__ void t_smooth_apply(const Team<TS>& tm, SmoTeamWs<T, 
 namespace pof {
 
 // ---------------------------------------------------------------------------
-// Level-0 (per time step) operations, team-parallel.  Same formulas as
+// Level-0 (per time step) operations, team-parallel.  Same quantities as
 // kf_step / cond_fold_step of pof_ops.cuh.
+//
+// Level 0 is bound by the FP64 pipe (every FP64 instruction of a warp holds
+// it for 64 cycles), so a step's triangularizations leave out what is zero:
+//   [QL | F L]: L has nl nonzero columns -- D - d after a noiseless update,
+//     none at the start of a conditional fold -- and with a block-diagonal F
+//     (the IWP prior) row j of F L ends with its block (TailBlocks): tails of
+//     4 and 6 columns at D = 8, d = 2 instead of 8;
+//   Psi = [[H Lp, R], [Lp, 0]] without noise (no R, or a step whose R is
+//     zero) ends with the last column h that H reaches (its E0 and E1
+//     columns): D - q + 1 of D + d columns, and Psi22 has D - d columns;
+//   Phi22, the smoother element's factor, is left as the D x nl matrix that
+//     the reflectors of [QL | F L] leave below them: it enters only
+//     triangularizations that take any square root;
+//   [Z | W^T]: the tail is W^T's d columns.
+// The structure is found when the model is loaded (integer operations: it is
+// the caller's data and need not have any); sums over it leave out exact
+// zeros.  D = 8, d = 2: 8 + 5 reflectors per Kalman step instead of 8 + 9 + 7.
 // ---------------------------------------------------------------------------
 template <typename T, int D, int DY>
 struct StepDims {
   static constexpr int D2 = 2 * D;
   static constexpr int DP = D + DY;
+  static constexpr int Q1 = D % DY == 0 ? D / DY : 0;  // block size of the IWP prior
   static constexpr int LD2 = Ld<D2>::v;
   static constexpr int LD1 = Ld<D>::v;
   static constexpr int LDP = Ld<DP>::v;
@@ -634,10 +681,9 @@ struct StepKFWs : StepDims<T, D, DY> {
   using B = StepDims<T, D, DY>;
   T H[DY * B::LD1], c[DY], R[DY * DY];          // observation model of the step
   T m[D], L[D * B::LD1];                        // filtered state
-  T X[D * B::LD2], Y[D * B::LD2];               // [F L, QL], [L, 0]
+  T X[D * B::LD2], Y[D * B::LD2];               // [QL | F L], [0 | L]
   T P[B::DP * B::LDP];                          // Psi
   T E[D * B::LD1], g[D], mp[D];                 // smoother element, predicted mean
-  T sc[4];                                      // scalars: ssq term, nll term
 };
 
 // ... for the conditional fold (and the plain Kalman step of a first chunk).
@@ -645,208 +691,327 @@ template <typename T, int D, int DY>
 struct StepFoldWs : StepDims<T, D, DY> {
   using B = StepDims<T, D, DY>;
   T H[DY * B::LD1], c[DY], R[DY * DY];
-  T m[D], L[D * B::LD1];                        // conditional L (or the filtered state)
-  T X[D * B::LD2];                              // [F L, QL]
+  T m[D], L[D * B::LD1];                        // mean (of x = 0 in the fold) and conditional L
+  T X[D * B::LD2];                              // [QL | F L]
   T P[B::DP * B::LDP];
   T mp[D];
-  T A[D * B::LD1], b[D], eta[D], Z[D * B::LD1];  // conditional fold state
-  T FA[D * B::LD1], Fb[D], W[DY * B::LD1], w[DY], ZX[D * B::LDZ];
-  T sc[4];
+  T ZX[D * B::LDZ];                             // [Z | W^T]
 };
 
-template <typename T, int TS, int D, int DY, typename WS>
-__device__ __forceinline__ void t_load_step(const Team<TS>& tm, WS& w, const T* H, const T* c, const T* R) {
-  constexpr int L1 = Ld<D>::v;
-  for (int f = tm.r; f < DY * D; f += TS) w.H[(f / D) * L1 + f % D] = H[f];
-  for (int f = tm.r; f < DY; f += TS) w.c[f] = c[f];
-  for (int f = tm.r; f < DY * DY; f += TS) w.R[f] = R ? R[f] : T(0);
-}
-
-// Psi = tria([[H Lp, R], [Lp, 0]]) with Lp = X[:, :D]; then r = H mp + c,
-// ssq / nll terms, m <- mp + Psi21 Psi11^{-1} (-r), L <- Psi22.  rzero: R is
-// zero (noiseless observation, the EK1 model), so Psi's last DY columns are.
-template <typename T, int TS, int D, int DY, bool UPDATE_STATE, typename WS>
-__device__ __forceinline__ void t_update(const Team<TS>& tm, WS& w, bool rzero) {
-  using W = StepDims<T, D, DY>;
-  constexpr int L1 = W::LD1, L2 = W::LD2, LP = W::LDP, DP = W::DP;
-  // rows 0..DY-1: [H Lp, R]; rows DY..: [Lp, 0]
-  for (int idx = tm.r; idx < DY * D; idx += TS) {
-    const int i = idx / D, j = idx % D;
-    T s = T(0);
-#pragma unroll
-    for (int k = 0; k < D; ++k) s = fma(w.H[i * L1 + k], w.X[k * L2 + j], s);
-    w.P[i * LP + j] = s;
-  }
-  for (int idx = tm.r; idx < DY * DY; idx += TS) w.P[(idx / DY) * LP + D + idx % DY] = w.R[idx];
-  for (int idx = tm.r; idx < D * DP; idx += TS) {
-    const int i = idx / DP, j = idx % DP;
-    w.P[(DY + i) * LP + j] = (j < D) ? w.X[i * L2 + j] : T(0);
-  }
-  tm.sync();
-  t_tria<T, TS, DP, 0, DP, LP, LP>(tm, w.P, w.P, 0, rzero ? D : DP);
-  if constexpr (UPDATE_STATE) {
-    // the DY x DY solves are tiny: every lane does them redundantly
-    T r[DY], wv[DY], wq[DY];
-#pragma unroll
-    for (int i = 0; i < DY; ++i) {
-      T s = w.c[i];
-#pragma unroll
-      for (int k = 0; k < D; ++k) s = fma(w.H[i * L1 + k], w.mp[k], s);
-      r[i] = s;
-      wv[i] = -s;
-      wq[i] = s;
-    }
-    trsv_l<T, DY, LP>(w.P, wv);
-    trsv_lt<T, DY, LP>(w.P, wq);
-    T ss = T(0), yy = T(0);
-#pragma unroll
-    for (int i = 0; i < DY; ++i) {
-      ss = fma(wq[i], wq[i], ss);
-      yy = fma(wv[i], wv[i], yy);
-    }
-    // log |Psi11_ii| on lane i (the DY logarithms run side by side)
-    const T ld = tm.sum(tm.r < DY ? T(log(fabs(w.P[tm.r * LP + tm.r]))) : T(0));
-    if (tm.r == 0) {
-      w.sc[0] = ss;
-      w.sc[1] = T(0.5) * yy + ld + T(DY) * Log2Pi<T>::half;
-    }
-    for (int i = tm.r; i < D; i += TS) {
-      T acc = w.mp[i];
-#pragma unroll
-      for (int k = 0; k < DY; ++k) acc = fma(w.P[(DY + i) * LP + k], wv[k], acc);
-      w.m[i] = acc;
-    }
-    t_copy<T, TS, D, D, LP, L1>(tm, w.P + DY * LP + DY, w.L);
-    tm.sync();
-  }
-}
-
-// Zero structure of a step's transition model, found when the model is
-// loaded (it is the caller's data: a TransitionModel need not have any).
-//   wq: D when QL is lower-triangular (t_tria's wlow for [F L, QL]), else 0;
-//   wf: Q when F is block-diagonal with upper-triangular Q x Q blocks (the
-//       IWP prior, I_d (x) A_1 with A_1 upper-triangular), else 0;
-//   rzero: the observation noise R is zero (noiseless EK1 model).
+// Zero structure of a step's transition model (D - by - D F and QL):
+//   qlow: QL is lower triangular; wf: the block size Q when F is
+//   block-diagonal with upper-triangular Q x Q blocks (the IWP prior), else 0.
 struct StepStruct {
-  int wq, wf;
+  bool qlow;
+  int wf;
+};
+
+// What a step's observation model leaves out: h1 columns of H up to its last
+// nonzero one, no noise.
+struct StepObs {
+  int h1;
   bool rzero;
 };
 
-// C(D x N) = F B with F's zeros skipped when wf > 0: row i of F has its
-// nonzeros in columns i .. (i / wf + 1) wf - 1.  The skipped terms are exact
-// zeros, so the result is the dense product's.
-template <typename T, int TS, int D, int N, int LDA, int LDB, int LDC>
-__device__ __forceinline__ void t_mm_f(const Team<TS>& tm, const T* F, const T* B, T* C, int wf) {
-  for (int idx = tm.r; idx < D * N; idx += TS) {
-    const int i = idx / N, j = idx % N;
-    const int k0 = wf ? i : 0, k1 = wf ? (i / wf + 1) * wf : D;
-    T s = T(0);
-    for (int k = k0; k < k1; ++k) s = fma(F[i * LDA + k], B[k * LDB + j], s);
-    C[i * LDC + j] = s;
+template <typename T, int TS, int D, int DY, typename WS>
+__device__ __forceinline__ StepObs t_load_step(const Team<TS>& tm, WS& w, const T* H, const T* c, const T* R) {
+  constexpr int L1 = Ld<D>::v;
+  int h1 = 0;
+  bool noise = false;
+  for (int f = tm.r; f < DY * D; f += TS) {
+    const T v = H[f];
+    w.H[(f / D) * L1 + f % D] = v;
+    if (!is_zero(v)) h1 = max(h1, f % D + 1);
   }
+  for (int f = tm.r; f < DY; f += TS) w.c[f] = c[f];
+  if (R) {
+    for (int f = tm.r; f < DY * DY; f += TS) {
+      const T v = R[f];
+      w.R[f] = v;
+      noise |= !is_zero(v);
+    }
+    noise = __any_sync(tm.mask, noise);
+  }
+  return StepObs{(int)__reduce_max_sync(tm.mask, (unsigned)h1), !noise};
 }
 
-// y(D) = F x, F's zeros skipped when wf > 0 (as t_mm_f).
-template <typename T, int TS, int D, int LDA>
-__device__ __forceinline__ void t_mv_f(const Team<TS>& tm, const T* F, const T* x, T* y, int wf) {
-  for (int i = tm.r; i < D; i += TS) {
-    const int k0 = wf ? i : 0, k1 = wf ? (i / wf + 1) * wf : D;
-    T s = T(0);
-    for (int k = k0; k < k1; ++k) s = fma(F[i * LDA + k], x[k], s);
-    y[i] = s;
+// Running log of a product of |x| (the observation factor's diagonal over a
+// chunk's steps): mantissas multiplied, exponents added, one logarithm at the
+// end instead of one per step (about 25 FP64 instructions each).
+struct LogProd {
+  double p = 1.0, extra = 0.0;
+  long long e = 0;
+  __device__ __forceinline__ void mul(double x) {
+    const long long b = __double_as_longlong(x) & 0x7fffffffffffffffLL;
+    const int ex = (int)(b >> 52);
+    if (ex == 0 || ex == 0x7ff) {
+      extra += log(fabs(x));  // zero, subnormal, infinite, NaN
+      return;
+    }
+    p *= __longlong_as_double((b & 0xfffffffffffffLL) | (1023LL << 52));  // p in [1, 4)
+    const long long pb = __double_as_longlong(p);
+    e += (ex - 1023) + ((int)(pb >> 52) - 1023);
+    p = __longlong_as_double((pb & 0xfffffffffffffLL) | (1023LL << 52));
   }
-}
+  __device__ __forceinline__ void mul(float x) { extra += (double)logf(fabsf(x)); }
+  __device__ __forceinline__ double value() const {
+    return log(p) + (double)e * 0.69314718055994530941723212145818 + extra;
+  }
+};
 
-// One square-root KF step from the filtered state (m, L) at grid s, fused with
-// the smoother element (g, E, Dm = Y[:, D:]) of grid s when SMOOTH.  F and
-// QL (D x D, leading dimension Ld<D>) are the step's transition model, ss
-// its zero structure.
+// [QL | F L] in w.X and, when SMOOTH, [0 | L] in w.Y; their reflectors.
 template <typename T, int TS, int D, int DY, bool SMOOTH, typename WS>
-__device__ __forceinline__ void t_kf_step(const Team<TS>& tm, WS& w, const T* F, const T* QL, StepStruct ss) {
+__device__ __forceinline__ void t_predict(const Team<TS>& tm, WS& w, const T* F, const T* QL, StepStruct ss, int nl,
+                                          bool lower) {
   using W = StepDims<T, D, DY>;
-  constexpr int L1 = W::LD1, L2 = W::LD2, D2 = W::D2;
-  const int wq = ss.wq;
-  const bool rzero = ss.rzero;
-  t_mm_f<T, TS, D, D, L1, L1, L2>(tm, F, w.L, w.X, ss.wf);
-  t_copy<T, TS, D, D, L1, L2>(tm, QL, w.X + D);
-  t_mv_f<T, TS, D, L1>(tm, F, w.m, w.mp, ss.wf);
-  if constexpr (SMOOTH) {
-    t_copy<T, TS, D, D, L1, L2>(tm, w.L, w.Y);
-    t_fill<T, TS, D, D, L2>(tm, w.Y + D, T(0), T(0));
-    tm.sync();
-    t_tria<T, TS, D, D, D2, L2, L2>(tm, w.X, w.Y, wq);  // Phi11, Phi21
-    t_tria<T, TS, D, 0, D, L2, L2>(tm, w.Y + D, w.Y);  // Phi22
-    // E^T = Phi11^{-T} Phi21^T  (E stored transposed in w.E, fixed below)
-    t_copy<T, TS, D, D, L2, L1, true>(tm, w.Y, w.E);
-    tm.sync();
-    t_trsm_lt<T, TS, D, D, L2, L1>(tm, w.X, w.E);
-    tm.sync();
-    // g = m - E mp = m - (E^T)^T mp
-    t_mv<T, TS, D, D, L1, true>(tm, w.E, w.mp, w.g);
-    tm.sync();
-    for (int i = tm.r; i < D; i += TS) w.g[i] = w.m[i] - w.g[i];
-  } else {
-    tm.sync();
-    t_tria<T, TS, D, 0, D2, L2, L2>(tm, w.X, w.X, wq);
-  }
-  t_update<T, TS, D, DY, true>(tm, w, rzero);
-}
-
-// One step of the conditional fold (cond_fold_step of pof_ops.cuh).
-template <typename T, int TS, int D, int DY>
-__device__ __forceinline__ void t_cond_fold_step(const Team<TS>& tm, StepFoldWs<T, D, DY>& w, const T* F,
-                                                 const T* QL, StepStruct ss) {
-  using W = StepDims<T, D, DY>;
-  constexpr int L1 = W::LD1, L2 = W::LD2, LP = W::LDP, LZ = W::LDZ, D2 = W::D2;
-  const int wq = ss.wq;
-  const bool rzero = ss.rzero;
-  t_mm_f<T, TS, D, D, L1, L1, L2>(tm, F, w.L, w.X, ss.wf);
-  t_copy<T, TS, D, D, L1, L2>(tm, QL, w.X + D);
-  t_mm_f<T, TS, D, D, L1, L1, L1>(tm, F, w.A, w.FA, ss.wf);
-  t_mv_f<T, TS, D, L1>(tm, F, w.b, w.Fb, ss.wf);
-  tm.sync();
-  t_tria<T, TS, D, 0, D2, L2, L2>(tm, w.X, w.X, wq);
-  t_update<T, TS, D, DY, false>(tm, w, rzero);
-  // W = H FA (DY x D), w = H Fb + c, then Psi11^{-1} on both
-  t_mm<T, TS, DY, D, D, L1, L1, L1>(tm, w.H, w.FA, w.W);
-  for (int i = tm.r; i < DY; i += TS) {
-    T s = w.c[i];
-#pragma unroll
-    for (int k = 0; k < D; ++k) s = fma(w.H[i * L1 + k], w.Fb[k], s);
-    w.w[i] = s;
-  }
-  tm.sync();
-  t_trsm_l<T, TS, DY, D, LP, L1>(tm, w.P, w.W);
-  tm.sync();
-  if (tm.r == 0) trsv_l<T, DY, LP>(w.P, w.w);
-  tm.sync();
-  // A = FA - Psi21 W ; b = Fb - Psi21 w ; eta -= W^T w ; ZX = [Z, W^T]
+  constexpr int L1 = W::LD1, L2 = W::LD2;
+  t_copy<T, TS, D, D, L1, L2>(tm, QL, w.X);
   for (int idx = tm.r; idx < D * D; idx += TS) {
     const int i = idx / D, j = idx % D;
-    T acc = w.FA[i * L1 + j];
+    if (j >= nl) continue;
+    const int k0 = ss.wf ? i : 0, k1 = ss.wf ? (i / ss.wf + 1) * ss.wf : D;
+    T s = T(0);
+    for (int k = k0; k < k1; ++k) s = fma(F[i * L1 + k], w.L[k * L1 + j], s);
+    w.X[i * L2 + D + j] = s;
+  }
+  T* Y = w.X;
+  if constexpr (SMOOTH) {
+    Y = w.Y;
+    t_fill<T, TS, D, D, L2>(tm, w.Y, T(0), T(0));
+    t_copy<T, TS, D, D, L1, L2>(tm, w.L, w.Y + D);
+  }
+  constexpr int MB = SMOOTH ? D : 0;
+  if (ss.qlow) {
+    if (ss.wf && lower)
+      t_lq<T, TS, D, MB, L2, L2>(tm, w.X, Y, TailBlocks<W::Q1>{D, nl});
+    else
+      t_lq<T, TS, D, MB, L2, L2>(tm, w.X, Y, TailBlocks<0>{D, nl});
+  } else {  // a caller's QL that is not triangular: no pivot block
+    t_lq<T, TS, D, MB, L2, L2>(tm, w.X, Y, TailUpper{D + nl});
+    for (int idx = tm.r; idx < D * D; idx += TS) {
+      const int i = idx / D, k = idx % D;
+      if (k > i) w.X[i * L2 + k] = T(0);
+    }
+    tm.sync();
+  }
+}
+
+// Psi = tria([[H Lp, R], [Lp, 0]]) with Lp = X[:, :D] in w.P.
+template <typename T, int TS, int D, int DY, typename WS>
+__device__ __forceinline__ void t_psi(const Team<TS>& tm, WS& w, StepObs ob) {
+  using W = StepDims<T, D, DY>;
+  constexpr int L1 = W::LD1, L2 = W::LD2, LP = W::LDP, DP = W::DP;
+  for (int idx = tm.r; idx < DY * D; idx += TS) {
+    const int i = idx / D, j = idx % D;
+    T s = T(0);
+    for (int k = 0; k < ob.h1; ++k) s = fma(w.H[i * L1 + k], w.X[k * L2 + j], s);
+    w.P[i * LP + j] = s;
+  }
+  if (!ob.rzero)
+    for (int idx = tm.r; idx < DY * DY; idx += TS) w.P[(idx / DY) * LP + D + idx % DY] = w.R[idx];
+  for (int idx = tm.r; idx < D * DP; idx += TS) {
+    const int i = idx / DP, j = idx % DP;
+    w.P[(DY + i) * LP + j] = (j <= i) ? w.X[i * L2 + j] : T(0);
+  }
+  const int nc = ob.rzero ? ob.h1 : DP;  // columns with entries right of the diagonal
+  t_lq<T, TS, DP, 0, LP, LP>(tm, w.P, w.P, TailUpper{nc}, nc < DP ? nc : DP);
+}
+
+// L <- Psi22 (columns beyond Psi's are zero; right of the diagonal the
+// reflected tails are left out)
+template <typename T, int TS, int D, int DY, typename WS>
+__device__ __forceinline__ void t_psi22(const Team<TS>& tm, WS& w, StepObs ob) {
+  using W = StepDims<T, D, DY>;
+  constexpr int L1 = W::LD1, LP = W::LDP, DP = W::DP;
+  const int nc = ob.rzero ? D : DP;
+  for (int idx = tm.r; idx < D * D; idx += TS) {
+    const int i = idx / D, k = idx % D;
+    w.L[i * L1 + k] = (k <= i && DY + k < nc) ? w.P[(DY + i) * LP + DY + k] : T(0);
+  }
+}
+
+// wv = -Psi11^{-1} (H x + c) (every lane has all of it), the lane's share
+// being one row; rdv[i] = 1 / Psi11_ii, r the residual.
+template <typename T, int TS, int D, int DY, typename WS>
+__device__ __forceinline__ void t_innovation(const Team<TS>& tm, WS& w, const T* x, int h1, T (&r)[DY], T (&rdv)[DY],
+                                             T (&wv)[DY]) {
+  using W = StepDims<T, D, DY>;
+  constexpr int L1 = W::LD1, LP = W::LDP;
+  const int src = (threadIdx.x & 31) / TS * TS;
+  const int i = tm.r % DY;
+  T s = w.c[i];
+  for (int k = 0; k < h1; ++k) s = fma(w.H[i * L1 + k], x[k], s);
+  const T rd = rcp(w.P[i * LP + i]);
 #pragma unroll
-    for (int k = 0; k < DY; ++k) acc = fma(-w.P[(DY + i) * LP + k], w.W[k * L1 + j], acc);
-    w.A[i * L1 + j] = acc;
+  for (int a = 0; a < DY; ++a) {
+    r[a] = __shfl_sync(tm.mask, s, src + a);
+    rdv[a] = __shfl_sync(tm.mask, rd, src + a);
+  }
+#pragma unroll
+  for (int a = 0; a < DY; ++a) {
+    T v = -r[a];
+#pragma unroll
+    for (int k = 0; k < a; ++k) v = fma(-w.P[a * LP + k], wv[k], v);
+    wv[a] = v * rdv[a];
+  }
+}
+
+// One square-root KF step from the filtered state (m, L), L with nl nonzero
+// columns, at grid s, fused with the smoother element of grid s when SMOOTH:
+// g, E, and its factor in Y[:, D : D + nl] (a D x nl square root of
+// Phi22 Phi22^T, not triangular).  Adds ||Psi11^{-T} r||^2 to ssq (whiten
+// quirk, pof/utils.py:110-112), ||Psi11^{-1} r||^2 to yy and |Psi11_ii| to
+// lane i's lp; returns the column count of the new L.
+template <typename T, int TS, int D, int DY, bool SMOOTH, typename WS>
+__device__ __forceinline__ int t_kf_step(const Team<TS>& tm, WS& w, const T* F, const T* QL, StepStruct ss,
+                                         StepObs ob, int nl, bool lower, double& ssq, double& yy, LogProd& lp) {
+  using W = StepDims<T, D, DY>;
+  constexpr int L1 = W::LD1, L2 = W::LD2, LP = W::LDP;
+  static_assert(D <= TS && DY <= TS, "one row of the state per lane");
+  for (int i = tm.r; i < D; i += TS) {
+    const int k0 = ss.wf ? i : 0, k1 = ss.wf ? (i / ss.wf + 1) * ss.wf : D;
+    T s = T(0);
+    for (int k = k0; k < k1; ++k) s = fma(F[i * L1 + k], w.m[k], s);
+    w.mp[i] = s;
+  }
+  t_predict<T, TS, D, DY, SMOOTH>(tm, w, F, QL, ss, nl, lower);  // Phi11 = X[:, :D], Phi21 = Y[:, :D]
+  if constexpr (SMOOTH) {
+    // E = Phi21 Phi11^{-1}, lane j solves for row j; g = m - E mp
+    const int src = (threadIdx.x & 31) / TS * TS;
+    const T rd = t_recip_diag<T, TS, D, L2>(tm, w.X);
+    const int j = tm.r < D ? tm.r : 0;
+    T x[D];
+#pragma unroll
+    for (int i = D - 1; i >= 0; --i) {
+      T s = w.Y[j * L2 + i];
+#pragma unroll
+      for (int k = i + 1; k < D; ++k) s = fma(-w.X[k * L2 + i], x[k], s);
+      x[i] = s * __shfl_sync(tm.mask, rd, src + i);
+    }
+    T gj = w.m[j];
+#pragma unroll
+    for (int i = 0; i < D; ++i) gj = fma(-x[i], w.mp[i], gj);
+    if (tm.r < D) {
+      w.g[j] = gj;
+#pragma unroll
+      for (int i = 0; i < D; ++i) w.E[j * L1 + i] = x[i];
+    }
+  }
+  t_psi<T, TS, D, DY>(tm, w, ob);
+  T r[DY], rdv[DY], wv[DY], wq[DY];
+  t_innovation<T, TS, D, DY>(tm, w, w.mp, ob.h1, r, rdv, wv);
+  T s2 = T(0), y2 = T(0);
+#pragma unroll
+  for (int i = DY - 1; i >= 0; --i) {
+    T v = r[i];
+#pragma unroll
+    for (int k = i + 1; k < DY; ++k) v = fma(-w.P[k * LP + i], wq[k], v);
+    wq[i] = v * rdv[i];
+    s2 = fma(wq[i], wq[i], s2);
+    y2 = fma(wv[i], wv[i], y2);
+  }
+  ssq += (double)s2;
+  yy += (double)y2;
+  if (tm.r < DY) lp.mul(w.P[tm.r * LP + tm.r]);
+  for (int i = tm.r; i < D; i += TS) {
+    T acc = w.mp[i];
+#pragma unroll
+    for (int k = 0; k < DY; ++k) acc = fma(w.P[(DY + i) * LP + k], wv[k], acc);
+    w.m[i] = acc;
+  }
+  t_psi22<T, TS, D, DY>(tm, w, ob);
+  tm.sync();
+  return ob.rzero && DY < D ? D - DY : D;
+}
+
+// Conditional fold of a chunk (cond_fold_step of pof_ops.cuh): lane j holds
+// column j of A and entry j of eta; b is w.m, U is w.L, Z is w.ZX[:, :D].
+template <typename T, int D>
+struct FoldRegs {
+  T a[D], eta;
+};
+
+template <typename T, int TS, int D, int DY>
+__device__ __forceinline__ void t_fold_start(const Team<TS>& tm, StepFoldWs<T, D, DY>& w, FoldRegs<T, D>& fr) {
+  using W = StepDims<T, D, DY>;
+#pragma unroll
+  for (int i = 0; i < D; ++i) fr.a[i] = T(i == tm.r ? 1 : 0);
+  fr.eta = T(0);
+  t_fill<T, TS, D, D, W::LD1>(tm, w.L, T(0), T(0));
+  t_fill<T, TS, D, D, W::LDZ>(tm, w.ZX, T(0), T(0));
+  for (int i = tm.r; i < D; i += TS) w.m[i] = T(0);
+}
+
+template <typename T, int TS, int D, int DY>
+__device__ __forceinline__ int t_cond_fold_step(const Team<TS>& tm, StepFoldWs<T, D, DY>& w, FoldRegs<T, D>& fr,
+                                                const T* F, const T* QL, StepStruct ss, StepObs ob, int nl) {
+  using W = StepDims<T, D, DY>;
+  constexpr int L1 = W::LD1, LP = W::LDP, LZ = W::LDZ, Q1 = W::Q1;
+  static_assert(D <= TS && DY <= TS, "one column of A per lane");
+  t_predict<T, TS, D, DY, false>(tm, w, F, QL, ss, nl, true);
+  t_psi<T, TS, D, DY>(tm, w, ob);
+  // FA (lane's column) and Fb
+  T fa[D];
+  if (Q1 > 0 && ss.wf) {
+#pragma unroll
+    for (int i = 0; i < D; ++i) {
+      T s = T(0);
+#pragma unroll
+      for (int k = i; k < (i / (Q1 > 0 ? Q1 : 1) + 1) * Q1; ++k) s = fma(F[i * L1 + k], fr.a[k], s);
+      fa[i] = s;
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < D; ++i) {
+      T s = T(0);
+#pragma unroll
+      for (int k = 0; k < D; ++k) s = fma(F[i * L1 + k], fr.a[k], s);
+      fa[i] = s;
+    }
   }
   for (int i = tm.r; i < D; i += TS) {
-    T acc = w.Fb[i];
-#pragma unroll
-    for (int k = 0; k < DY; ++k) acc = fma(-w.P[(DY + i) * LP + k], w.w[k], acc);
-    w.b[i] = acc;
-    T e = w.eta[i];
-#pragma unroll
-    for (int k = 0; k < DY; ++k) e = fma(-w.W[k * L1 + i], w.w[k], e);
-    w.eta[i] = e;
+    const int k0 = ss.wf ? i : 0, k1 = ss.wf ? (i / ss.wf + 1) * ss.wf : D;
+    T s = T(0);
+    for (int k = k0; k < k1; ++k) s = fma(F[i * L1 + k], w.m[k], s);
+    w.mp[i] = s;
   }
-  for (int idx = tm.r; idx < D * (D + DY); idx += TS) {
-    const int i = idx / (D + DY), j = idx % (D + DY);
-    w.ZX[i * LZ + j] = (j < D) ? w.Z[i * L1 + j] : w.W[(j - D) * L1 + i];
+  tm.sync();
+  // w = Psi11^{-1} (H Fb + c) = -wv, W = Psi11^{-1} H FA (lane's column)
+  T r[DY], rdv[DY], wv[DY], wc[DY];
+  t_innovation<T, TS, D, DY>(tm, w, w.mp, ob.h1, r, rdv, wv);
+#pragma unroll
+  for (int i = 0; i < DY; ++i) {
+    T s = T(0);
+#pragma unroll
+    for (int k = 0; k < D; ++k)
+      if (k < ob.h1) s = fma(w.H[i * L1 + k], fa[k], s);
+#pragma unroll
+    for (int k = 0; k < i; ++k) s = fma(-w.P[i * LP + k], wc[k], s);
+    wc[i] = s * rdv[i];
   }
-  t_copy<T, TS, D, D, LP, L1>(tm, w.P + DY * LP + DY, w.L);
-  tm.sync();
-  t_tria<T, TS, D, 0, D + DY, LZ, LZ>(tm, w.ZX, w.ZX);
-  t_copy<T, TS, D, D, LZ, L1>(tm, w.ZX, w.Z);
-  tm.sync();
+  // A = FA - Psi21 W; b = Fb - Psi21 w; eta -= W^T w; [Z | W^T]
+#pragma unroll
+  for (int i = 0; i < D; ++i) {
+    T acc = fa[i];
+#pragma unroll
+    for (int k = 0; k < DY; ++k) acc = fma(-w.P[(DY + i) * LP + k], wc[k], acc);
+    fr.a[i] = acc;
+  }
+#pragma unroll
+  for (int k = 0; k < DY; ++k) fr.eta = fma(wc[k], wv[k], fr.eta);
+  if (tm.r < D) {
+#pragma unroll
+    for (int k = 0; k < DY; ++k) w.ZX[tm.r * LZ + D + k] = wc[k];
+  }
+  for (int i = tm.r; i < D; i += TS) {
+    T acc = w.mp[i];
+#pragma unroll
+    for (int k = 0; k < DY; ++k) acc = fma(w.P[(DY + i) * LP + k], wv[k], acc);
+    w.m[i] = acc;
+  }
+  t_psi22<T, TS, D, DY>(tm, w, ob);
+  t_lq<T, TS, D, 0, LZ, LZ>(tm, w.ZX, w.ZX, TailFixed<D, D + DY>{});
+  return ob.rzero && DY < D ? D - DY : D;
 }
 
 }  // namespace pof

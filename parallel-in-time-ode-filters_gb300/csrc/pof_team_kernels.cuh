@@ -360,7 +360,7 @@ __global__ void k_smo_ks_team(const T* __restrict__ in, int64_t K, int64_t s, in
 template <typename T, int D>
 struct FQ {
   T F[D * Ld<D>::v], QL[D * Ld<D>::v], QLi[D * Ld<D>::v];
-  int wq;  // D when QL is lower-triangular (t_tria's wlow for [F L, QL]), else 0
+  int wq;  // 1 when QL is lower-triangular (the pivot block of [QL | F L]), else 0
   int wf;  // Q when F is block-diagonal with upper-triangular Q x Q blocks, else 0
 };
 
@@ -368,7 +368,7 @@ struct FQ {
 // the block-upper-triangular pattern with blocks of Q (Q = 0: no pattern)
 template <typename T>
 __device__ __forceinline__ bool breaks_fblocks(T v, int i, int k, int Q) {
-  return Q <= 0 || (v != T(0) && (k < i || k >= (i / Q + 1) * Q));
+  return Q <= 0 || (!is_zero(v) && (k < i || k >= (i / Q + 1) * Q));
 }
 
 template <typename Base, typename T, int D, bool PS>
@@ -430,13 +430,13 @@ __device__ __forceinline__ void t_load_FQ(const Team<TS>& tm, FQ<T, D>& q, const
   for (int f = tm.r; f < D * D; f += TS) {
     q.F[(f / D) * L1 + f % D] = F[f];
     q.QL[(f / D) * L1 + f % D] = QL[f];
-    upper |= (f % D > f / D) && QL[f] != T(0);
+    upper |= (f % D > f / D) && !is_zero(QL[f]);
     fdense |= breaks_fblocks(F[f], f / D, f % D, Q);
   }
   const bool any_upper = __any_sync(tm.mask, upper);
   const bool any_fdense = __any_sync(tm.mask, fdense);
   if (tm.r == 0) {
-    q.wq = any_upper ? 0 : D;
+    q.wq = any_upper ? 0 : 1;
     q.wf = any_fdense ? 0 : Q;
   }
 }
@@ -460,13 +460,13 @@ __device__ __forceinline__ void load_fq_block(const Team<TS>& tm, FQ<T, D>& q, c
   for (int f = threadIdx.x; f < D * D; f += blockDim.x) {
     q.F[(f / D) * L1 + f % D] = F[f];
     q.QL[(f / D) * L1 + f % D] = QL[f];
-    upper |= (f % D > f / D) && QL[f] != T(0);
+    upper |= (f % D > f / D) && !is_zero(QL[f]);
     fdense |= breaks_fblocks(F[f], f / D, f % D, Q);
   }
   upper = __syncthreads_or(upper);
   fdense = __syncthreads_or(fdense);
   if (threadIdx.x == 0) {
-    q.wq = upper ? 0 : D;
+    q.wq = upper ? 0 : 1;
     q.wf = fdense ? 0 : Q;
   }
   if (threadIdx.x < TS) t_inv_lower<T, TS, D>(tm, q.QL, q.QLi);
@@ -474,14 +474,15 @@ __device__ __forceinline__ void load_fq_block(const Team<TS>& tm, FQ<T, D>& q, c
 }
 
 // || QL^{-1} (a - F b) ||^2 with QLi = QL^{-1}; every lane gets the value.
+// wf > 0: F is block-diagonal with blocks of wf (its zeros are skipped).
 template <typename T, int TS, int D>
 __device__ __forceinline__ T t_objective(const Team<TS>& tm, const T* F, const T* QLi, const T* a, const T* b,
-                                         T* r) {
+                                         T* r, int wf) {
   constexpr int L1 = Ld<D>::v;
   for (int i = tm.r; i < D; i += TS) {
+    const int k0 = wf ? i : 0, k1 = wf ? (i / wf + 1) * wf : D;
     T s = a[i];
-#pragma unroll
-    for (int k = 0; k < D; ++k) s = fma(-F[i * L1 + k], b[k], s);
+    for (int k = k0; k < k1; ++k) s = fma(-F[i * L1 + k], b[k], s);
     r[i] = s;
   }
   tm.sync();
@@ -530,66 +531,129 @@ __device__ __forceinline__ void fq_step(const Team<TS>& tm, FQ<T, D>& q, const S
   }
 }
 
+// the fold's element (columns of A and eta in lane registers) to SoA
+template <typename T, int TS, int D, int DY>
+__device__ __forceinline__ void t_store_fold(const Team<TS>& tm, T* base, int64_t n, int64_t e,
+                                             const StepFoldWs<T, D, DY>& w, const FoldRegs<T, D>& fr) {
+  if (!POF_IN(e, n)) return;
+  using FL = FiltLayout<D>;
+  constexpr int L1 = Ld<D>::v, LZ = StepDims<T, D, DY>::LDZ;
+  if (tm.r < D) {
+#pragma unroll
+    for (int i = 0; i < D; ++i) base[(FL::A + i * D + tm.r) * n + e] = fr.a[i];
+    base[(FL::B + tm.r) * n + e] = w.m[tm.r];
+    base[(FL::ETA + tm.r) * n + e] = fr.eta;
+  }
+  for (int f = tm.r; f < D * D; f += TS) {
+    const int i = f / D, j = f % D;
+    base[(FL::U + f) * n + e] = w.L[i * L1 + j];
+    base[(FL::Z + f) * n + e] = w.ZX[i * LZ + j];
+  }
+}
+
+// Level-0 fold.  Chunk 0 runs the Kalman filter from x0 (its element is the
+// filtering state: A, eta and Z are zero); it has a block of its own, so no
+// warp runs both kinds of step.
 template <typename T, int D, int DY, int TS, bool PS>
 __global__ void k_filt_l0_reduce_team(int64_t n, int C0, StepModel sm, const T* __restrict__ x0m,
                                       const T* __restrict__ x0L, T* __restrict__ out, int64_t n1) {
   using WS = L0FoldWs<T, D, DY, PS>;
-  POF_L0_PROLOGUE(WS, PS)
+  constexpr int HB_ = FQHeader<T, D, PS>::bytes;
+  using B_ = TeamBlockH<WS, TS, HB_>;
+  extern __shared__ __align__(16) unsigned char smem_raw_[];
+  const int team_in_block = threadIdx.x / TS;
+  WS& ws_ = *reinterpret_cast<WS*>(smem_raw_ + HB_ + team_in_block * B_::stride);
+  // block 0: chunk 0 in its first team; block b > 0: chunks 1 + (b - 1) teams ..
+  const int64_t t = blockIdx.x == 0 ? (team_in_block == 0 ? 0 : n1)
+                                    : 1 + (int64_t)(blockIdx.x - 1) * B_::teams + team_in_block;
+  Team<TS> tm;
+  FQ<T, D>& fq = fq_ref<PS, T, D>(ws_, smem_raw_);
   if constexpr (!PS)
-    load_fq_block<T, TS, D>(tm, fq, static_cast<const T*>(sm.F), static_cast<const T*>(sm.QL), D / DY);
+    load_fq_block<T, TS, D>(tm, fq, static_cast<const T*>(sm.F), static_cast<const T*>(sm.QL),
+                            StepDims<T, D, DY>::Q1);
   if (t >= n1) return;
   StepFoldWs<T, D, DY>& w = ws_.s;
-  constexpr int L1 = Ld<D>::v;
+  constexpr int L1 = Ld<D>::v, LZ = StepDims<T, D, DY>::LDZ;
   const int64_t s0 = t * C0;
   const int64_t s1 = (s0 + C0 < n) ? s0 + C0 : n;
+  FoldRegs<T, D> fr;
   if (t == 0) {
     t_load_state_plain<T, TS, D>(tm, x0m, x0L, w.m, w.L);
+    tm.sync();
+    bool lower;
+    int nl = t_ncols<T, TS, D, D, L1>(tm, w.L, &lower);
+    double ssq = 0.0, yy = 0.0;
+    LogProd lp;
     for (int64_t s = s0; s < s1; ++s) {
       if (!POF_IN(s, n)) break;
-      fq_step<PS, T, TS, D>(tm, fq, sm, s, false, D / DY);
+      fq_step<PS, T, TS, D>(tm, fq, sm, s, false, StepDims<T, D, DY>::Q1);
       StepView<T, D, DY> v(sm, s);
-      t_load_step<T, TS, D, DY>(tm, w, v.H, v.c, v.R);
+      const StepObs ob = t_load_step<T, TS, D, DY>(tm, w, v.H, v.c, v.R);
       tm.sync();
-      t_kf_step<T, TS, D, DY, false>(tm, w, fq.F, fq.QL, StepStruct{fq.wq, fq.wf, sm.R == nullptr});
+      nl = t_kf_step<T, TS, D, DY, false>(tm, w, fq.F, fq.QL, StepStruct{fq.wq != 0, fq.wf}, ob, nl, lower, ssq, yy,
+                                          lp);
+      lower = true;
     }
-    t_fill<T, TS, D, D, L1>(tm, w.A, T(0), T(0));
-    t_fill<T, TS, D, D, L1>(tm, w.Z, T(0), T(0));
-    for (int i = tm.r; i < D; i += TS) w.eta[i] = T(0);
-    tm.sync();
-    t_store_filt<T, TS, D>(tm, out, n1, t, w.A, w.m, w.L, w.eta, w.Z);
+#pragma unroll
+    for (int i = 0; i < D; ++i) fr.a[i] = T(0);
+    fr.eta = T(0);
+    t_fill<T, TS, D, D, LZ>(tm, w.ZX, T(0), T(0));
   } else {
-    t_fill<T, TS, D, D, L1>(tm, w.A, T(0), T(1));
-    t_fill<T, TS, D, D, L1>(tm, w.L, T(0), T(0));
-    t_fill<T, TS, D, D, L1>(tm, w.Z, T(0), T(0));
-    for (int i = tm.r; i < D; i += TS) {
-      w.b[i] = T(0);
-      w.eta[i] = T(0);
-    }
+    t_fold_start<T, TS, D, DY>(tm, w, fr);
+    int nl = 0;
     for (int64_t s = s0; s < s1; ++s) {
       if (!POF_IN(s, n)) break;
-      fq_step<PS, T, TS, D>(tm, fq, sm, s, false, D / DY);
+      fq_step<PS, T, TS, D>(tm, fq, sm, s, false, StepDims<T, D, DY>::Q1);
       StepView<T, D, DY> v(sm, s);
-      t_load_step<T, TS, D, DY>(tm, w, v.H, v.c, v.R);
+      const StepObs ob = t_load_step<T, TS, D, DY>(tm, w, v.H, v.c, v.R);
       tm.sync();
-      t_cond_fold_step<T, TS, D, DY>(tm, w, fq.F, fq.QL, StepStruct{fq.wq, fq.wf, sm.R == nullptr});
+      nl = t_cond_fold_step<T, TS, D, DY>(tm, w, fr, fq.F, fq.QL, StepStruct{fq.wq != 0, fq.wf}, ob, nl);
     }
-    tm.sync();
-    t_store_filt<T, TS, D>(tm, out, n1, t, w.A, w.b, w.L, w.eta, w.Z);
+  }
+  tm.sync();
+  t_store_fold<T, TS, D, DY>(tm, out, n1, t, w, fr);
+}
+
+// Smoother element of a step, t_kf_step's g, E and raw factor, to SoA.
+template <typename T, int TS, int D, int DY>
+__device__ __forceinline__ void t_store_selem(const Team<TS>& tm, T* base, int64_t n, int64_t s,
+                                              const StepKFWs<T, D, DY>& w, int nl) {
+  using GL = SmoLayout<D>;
+  constexpr int L1 = Ld<D>::v, L2 = Ld<2 * D>::v;
+  for (int f = tm.r; f < D; f += TS) base[f * n + s] = w.g[f];
+  for (int f = tm.r; f < D * D; f += TS) {
+    const int i = f / D, j = f % D;
+    base[(GL::E + f) * n + s] = w.E[i * L1 + j];
+    base[(GL::DM + f) * n + s] = j < nl ? w.Y[i * L2 + D + j] : T(0);
+  }
+}
+
+// The chunk's partial sums: sigma^2 terms, NLL (the constant of its steps and
+// the logarithms added here) and filter objective.
+template <int TS, int DY>
+__device__ __forceinline__ void t_store_partials(const Team<TS>& tm, double* partials, int64_t n1, int64_t t,
+                                                 double ssq, double yy, const LogProd& lp, int64_t steps,
+                                                 double fobj) {
+  const double ld = tm.sum(tm.r < DY ? lp.value() : 0.0);
+  if (tm.r == 0) {
+    partials[P_SSQ * n1 + t] = ssq;
+    partials[P_NLL * n1 + t] = 0.5 * yy + ld + (double)(steps * DY) * Log2Pi<double>::half;
+    partials[P_FOBJ * n1 + t] = fobj;
   }
 }
 
 template <typename T, int D, int DY, int TS, bool PS>
 __global__ void k_filt_l0_down_team(int64_t n, int C0, StepModel sm, const T* __restrict__ states1, int64_t n1,
                                     T* __restrict__ means, T* __restrict__ chols, T* __restrict__ selems,
-                                    double* __restrict__ partials) {
+                                    double* __restrict__ partials, bool want_fobj) {
   using WS = L0KFWs<T, D, DY, PS>;
   POF_L0_PROLOGUE(WS, PS)
   if constexpr (!PS)
-    load_fq_block<T, TS, D>(tm, fq, static_cast<const T*>(sm.F), static_cast<const T*>(sm.QL), D / DY);
+    load_fq_block<T, TS, D>(tm, fq, static_cast<const T*>(sm.F), static_cast<const T*>(sm.QL),
+                            StepDims<T, D, DY>::Q1);
   if (t >= n1) return;
   StepKFWs<T, D, DY>& w = ws_.s;
-  using GL = SmoLayout<D>;
-  constexpr int L1 = Ld<D>::v, L2 = Ld<2 * D>::v;
+  constexpr int L1 = Ld<D>::v;
   const int64_t s0 = t * C0;
   const int64_t s1 = (s0 + C0 < n) ? s0 + C0 : n;
   t_load_state<T, TS, D>(tm, states1, n1, t, w.m, w.L);
@@ -602,29 +666,23 @@ __global__ void k_filt_l0_down_team(int64_t n, int C0, StepModel sm, const T* __
         chols[f - D] = w.L[((f - D) / D) * L1 + (f - D) % D];
     }
   }
-  double ssq = 0.0, nll = 0.0, fobj = 0.0;
+  bool lower;
+  int nl = t_ncols<T, TS, D, D, L1>(tm, w.L, &lower);
+  double ssq = 0.0, yy = 0.0, fobj = 0.0;
+  LogProd lp;
   for (int64_t s = s0; s < s1; ++s) {
     if (!POF_IN(s, n)) break;
-    fq_step<PS, T, TS, D>(tm, fq, sm, s, true, D / DY);
+    fq_step<PS, T, TS, D>(tm, fq, sm, s, want_fobj, StepDims<T, D, DY>::Q1);
     StepView<T, D, DY> v(sm, s);
-    t_load_step<T, TS, D, DY>(tm, w, v.H, v.c, v.R);
-    for (int i = tm.r; i < D; i += TS) ws_.mold[i] = w.m[i];
+    const StepObs ob = t_load_step<T, TS, D, DY>(tm, w, v.H, v.c, v.R);
+    if (want_fobj)
+      for (int i = tm.r; i < D; i += TS) ws_.mold[i] = w.m[i];
     tm.sync();
-    t_kf_step<T, TS, D, DY, true>(tm, w, fq.F, fq.QL, StepStruct{fq.wq, fq.wf, sm.R == nullptr});
-    ssq += (double)w.sc[0];
-    nll += (double)w.sc[1];
-    fobj += (double)t_objective<T, TS, D>(tm, fq.F, fq.QLi, ws_.mold, w.m, ws_.r);
-    // smoother element of grid s: g, E (stored transposed in w.E), Dm = Y[:, D:]
-    for (int f = tm.r; f < GL::NG; f += TS) {
-      T val;
-      if (f < GL::E)
-        val = w.g[f];
-      else if (f < GL::DM)
-        val = w.E[((f - GL::E) % D) * L1 + (f - GL::E) / D];
-      else
-        val = w.Y[((f - GL::DM) / D) * L2 + D + (f - GL::DM) % D];
-      selems[f * n + s] = val;
-    }
+    const int nk = nl;
+    nl = t_kf_step<T, TS, D, DY, true>(tm, w, fq.F, fq.QL, StepStruct{fq.wq != 0, fq.wf}, ob, nl, lower, ssq, yy, lp);
+    lower = true;
+    if (want_fobj) fobj += (double)t_objective<T, TS, D>(tm, fq.F, fq.QLi, ws_.mold, w.m, ws_.r, fq.wf);
+    t_store_selem<T, TS, D, DY>(tm, selems, n, s, w, nk);
     for (int f = tm.r; f < D + D * D; f += TS) {
       if (f < D)
         means[(s + 1) * D + f] = w.m[f];
@@ -633,22 +691,40 @@ __global__ void k_filt_l0_down_team(int64_t n, int C0, StepModel sm, const T* __
     }
     tm.sync();
   }
-  if (tm.r == 0) {
-    partials[P_SSQ * n1 + t] = ssq;
-    partials[P_NLL * n1 + t] = nll;
-    partials[P_FOBJ * n1 + t] = fobj;
+  t_store_partials<TS, DY>(tm, partials, n1, t, ssq, yy, lp, s1 - s0, fobj);
+}
+
+// Smoother level 0, up-sweep: composite of each chunk's elements, whose
+// factors are raw square roots; the composite's is triangular.
+template <typename T, int D, int TS>
+__global__ void k_smo_l0_reduce_team(const T* __restrict__ in, int64_t nin, int C, T* __restrict__ out,
+                                     int64_t nout) {
+  using WS = SmoTeamWs<T, D>;
+  POF_TEAM_PROLOGUE(WS)
+  if (t >= nout) return;
+  const int64_t i0 = t * C;
+  const int64_t i1 = (i0 + C < nin) ? i0 + C : nin;
+  t_load_smo<T, TS, D>(tm, in, nin, i0, w.g2, w.E2, w.D2m);
+  for (int64_t i = i0 + 1; i < i1; ++i) {
+    t_load_smo<T, TS, D>(tm, in, nin, i, w.g1, w.E1, w.D1);
+    tm.sync();
+    t_smooth_combine_raw<T, TS, D>(tm, w, i == i0 + 1);
   }
+  tm.sync();
+  if (i1 - i0 == 1) t_smooth_tria<T, TS, D>(tm, w);
+  t_store_smo<T, TS, D>(tm, out, nout, t, w.g2, w.E2, w.D2m);
 }
 
 template <typename T, int D, int TS, bool PS>
 __global__ void k_smo_l0_down_team(int64_t n, int C0, const T* __restrict__ F, const T* __restrict__ QL,
-                                   int64_t ft_stride, const T* __restrict__ selems, const T* __restrict__ ends1,
-                                   int64_t n1, T* __restrict__ means, T* __restrict__ chols,
-                                   const T* __restrict__ scale, const T* __restrict__ means_old, double c_mrtol,
-                                   double c_matol, double* __restrict__ partials) {
+                                   int64_t ft_stride, int Q, const T* __restrict__ selems,
+                                   const T* __restrict__ ends1, int64_t n1, T* __restrict__ means,
+                                   T* __restrict__ chols, const T* __restrict__ scale,
+                                   const T* __restrict__ means_old, double c_mrtol, double c_matol,
+                                   double* __restrict__ partials) {
   using WS = SmoL0Ws<T, D, PS>;
   POF_L0_PROLOGUE(WS, PS)
-  if constexpr (!PS) load_fq_block<T, TS, D>(tm, fq, F, QL, 0);
+  if constexpr (!PS) load_fq_block<T, TS, D>(tm, fq, F, QL, Q);
   if (t >= n1) return;
   SmoTeamWs<T, D>& w = ws_.s;
   constexpr int L1 = Ld<D>::v;
@@ -658,7 +734,10 @@ __global__ void k_smo_l0_down_team(int64_t n, int C0, const T* __restrict__ F, c
   const StepModel sm{F, QL, ft_stride, nullptr, nullptr, nullptr, 0};
   t_load_state<T, TS, D>(tm, ends1, n1, t, w.g1, w.D1);
   tm.sync();
-  double sobj = 0.0, notclose = 0.0;
+  bool lower;
+  t_ncols<T, TS, D, D, L1>(tm, w.D1, &lower);
+  double sobj = 0.0;
+  int notclose = 0;
   auto close_count = [&](int64_t k) {
     if (!means_old) return;
     for (int i = tm.r; i < D; i += TS) {
@@ -668,7 +747,7 @@ __global__ void k_smo_l0_down_team(int64_t n, int C0, const T* __restrict__ F, c
         ok = fabs(a - b) <= c_matol + c_mrtol * fabs(b);
       else
         ok = (a == b);
-      notclose += ok ? 0.0 : 1.0;
+      notclose += ok ? 0 : 1;
     }
   };
   if (s1 == n) {
@@ -678,25 +757,27 @@ __global__ void k_smo_l0_down_team(int64_t n, int C0, const T* __restrict__ F, c
   }
   for (int64_t k = s1 - 1; k >= s0; --k) {
     if (!POF_IN(k, n)) break;
-    fq_step<PS, T, TS, D>(tm, fq, sm, k, true, 0);
+    fq_step<PS, T, TS, D>(tm, fq, sm, k, true, Q);
     for (int i = tm.r; i < D; i += TS) ws_.mnext[i] = w.g1[i];
     t_load_smo<T, TS, D>(tm, selems, n, k, w.g2, w.E2, w.D2m);
     tm.sync();
-    t_smooth_apply<T, TS, D>(tm, w);
-    sobj += (double)t_objective<T, TS, D>(tm, fq.F, fq.QLi, w.g1, ws_.mnext, ws_.r);
+    t_smooth_apply_raw<T, TS, D>(tm, w, lower);
+    lower = true;
+    sobj += (double)t_objective<T, TS, D>(tm, fq.F, fq.QLi, w.g1, ws_.mnext, ws_.r, fq.wf);
     close_count(k);
     for (int f = tm.r; f < D + D * D; f += TS) {
       if (f < D)
         means[k * D + f] = w.g1[f];
       else
-        chols[k * D * D + f - D] = w.D1[((f - D) / D) * L1 + (f - D) % D] * sc;
+        chols[k * D * D + f - D] = scale ? w.D1[((f - D) / D) * L1 + (f - D) % D] * sc
+                                         : w.D1[((f - D) / D) * L1 + (f - D) % D];
     }
     tm.sync();
   }
-  notclose = (double)tm.sum(notclose);
+  notclose = (int)__reduce_add_sync(tm.mask, (unsigned)notclose);
   if (tm.r == 0) {
     partials[P_SOBJ * n1 + t] = sobj;
-    partials[P_NOTCLOSE * n1 + t] = notclose;
+    partials[P_NOTCLOSE * n1 + t] = (double)notclose;
   }
 }
 
