@@ -149,6 +149,34 @@ inline void launch_team(void (*kern)(KArgs...), int64_t nteams, cudaStream_t st,
 // row, more outputs per t_mm step).  POF_WIDE_LANES overrides.
 int wide_lane_limit();
 
+// Smoother elements from given filtered states (used by pof_smoothing, where
+// the filtered trajectory comes from the caller), one thread per step, for
+// the small shapes.
+template <typename T, int D>
+__global__ void __launch_bounds__(64) k_smo_elements(int64_t n, const T* __restrict__ F, const T* __restrict__ QL,
+                                                     int64_t ft_stride, const T* __restrict__ fmeans,
+                                                     const T* __restrict__ fchols, T* __restrict__ selems) {
+  using GL = SmoLayout<D>;
+  constexpr int D2 = 2 * D;
+  const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  const T* Fk = F + k * ft_stride;
+  const T* Qk = QL + k * ft_stride;
+  const T* m = fmeans + k * D;
+  const T* L = fchols + k * D * D;
+  T X[D2 * D2];
+  mm<T, D, D, D, D, D, D2>(Fk, L, X);
+  copy<T, D, D, D, D2>(Qk, X + D);
+  copy<T, D, D, D, D2>(L, X + D * D2);
+  zero<T, D, D, D2>(X + D * D2 + D);
+  lq_rows<T, D, D2, D2, D2>(X);
+  T ge[GL::NG], mp[D];
+  mv<T, D, D, D>(Fk, m, mp);
+  gain<T, D, D2, D2>(X, X + D * D2, m, mp, ge + GL::G, ge + GL::E);
+  copy<T, D, D, D2, D>(X + D * D2 + D, ge + GL::DM);
+  st_soa<T, GL::NG>(selems, n, k, ge);
+}
+
 template <typename T, int D, int DY>
 struct Driver {
   static constexpr int kBlock = 64;
@@ -221,8 +249,8 @@ struct Driver {
                                                           p.C0, sm, x0m, x0L, b.template at<T>(p.felem[1]), n1);
       }
       else
-        k_filt_l0_reduce<T, D, DY><<<grid_for(n1, kBlock), kBlock, 0, st>>>(n, p.C0, sm, x0m, x0L,
-                                                                             b.template at<T>(p.felem[1]), n1);
+        k_filt_l0_reduce<T, D, DY><<<1 + grid_for(n1 - 1, kBlock), kBlock, 0, st>>>(
+            n, p.C0, sm, x0m, x0L, b.template at<T>(p.felem[1]), n1);
     }
     const int64_t wide = wide_lane_limit() / TSX;  // teams up to which the widest teams run
     for (int l = 1; l < p.nlev; ++l) {
@@ -280,7 +308,7 @@ struct Driver {
       else
         k_filt_l0_down<T, D, DY><<<grid_for(n1, kBlock), kBlock, 0, st>>>(
             n, p.C0, sm, b.template at<T>(p.fstate[1]), n1, means, chols, b.template at<T>(p.selem),
-            b.template at<double>(p.partials));
+            b.template at<double>(p.partials), p.fobj);
     }
     {
       ProfScope ps(PK_FILT_FINALIZE, st);
@@ -305,8 +333,8 @@ struct Driver {
         launch_team<SWS, TS>(k_smo_l0_reduce_team<T, D, TS>, n1, st, (const T*)b.template at<T>(p.selem), n, p.C0,
                              b.template at<T>(p.gelem[1]), n1);
       else
-        k_smo_reduce<T, D><<<grid_for(n1, kBlock), kBlock, 0, st>>>(b.template at<T>(p.selem), n, p.C0,
-                                                                    b.template at<T>(p.gelem[1]), n1);
+        k_smo_l0_reduce<T, D, DY><<<grid_for(n1, kBlock), kBlock, 0, st>>>(b.template at<T>(p.selem), n, p.C0,
+                                                                           b.template at<T>(p.gelem[1]), n1);
     }
     const int64_t wide = wide_lane_limit() / TSX;
     for (int l = 1; l < p.nlev; ++l) {
@@ -370,7 +398,7 @@ struct Driver {
                                                      means_old, p.mrtol, p.matol, b.template at<double>(p.partials));
       }
       else
-        k_smo_l0_down<T, D><<<grid_for(n1, kBlock), kBlock, 0, st>>>(
+        k_smo_l0_down<T, D, DY><<<grid_for(n1, kBlock), kBlock, 0, st>>>(
             n, p.C0, F, QL, ft_stride, b.template at<T>(p.selem), b.template at<T>(p.gend[1]), n1, means, chols,
             scl, means_old, p.mrtol, p.matol, b.template at<double>(p.partials));
     }
@@ -386,47 +414,21 @@ struct Driver {
     ProfScope ps(PK_LINEARIZE, st);
     k_linearize<T, D, DY><<<grid_for(n, 128), 128, 0, st>>>(n, field, params, p0, p1, means, H, c);
   }
-};
 
-// Smoother elements from given filtered states (used by pof_smoothing, where
-// the filtered trajectory comes from the caller).
-template <typename T, int D>
-__global__ void __launch_bounds__(64) k_smo_elements(int64_t n, const T* __restrict__ F, const T* __restrict__ QL,
-                                                     int64_t ft_stride, const T* __restrict__ fmeans,
-                                                     const T* __restrict__ fchols, T* __restrict__ selems) {
-  using GL = SmoLayout<D>;
-  constexpr int D2 = 2 * D;
-  const int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (k >= n) return;
-  const T* Fk = F + k * ft_stride;
-  const T* Qk = QL + k * ft_stride;
-  const T* m = fmeans + k * D;
-  const T* L = fchols + k * D * D;
-  T X[D * D2], Y[D * D2];
-  mm<T, D, D, D, D, D, D2>(Fk, L, X);
-  copy<T, D, D, D, D2>(Qk, X + D);
-  copy<T, D, D, D, D2>(L, Y);
-  zero<T, D, D, D2>(Y + D);
-  tria_top<T, D, D, D2, D2, D2>(X, Y);
-  tria<T, D, D, D2>(Y + D);
-  T ge[GL::NG];
-  T Et[D * D];
-#pragma unroll
-  for (int i = 0; i < D; ++i)
-#pragma unroll
-    for (int j = 0; j < D; ++j) Et[i * D + j] = Y[j * D2 + i];
-  trsm_lt<T, D, D, D2, D>(X, Et);
-#pragma unroll
-  for (int i = 0; i < D; ++i)
-#pragma unroll
-    for (int j = 0; j < D; ++j) ge[GL::E + i * D + j] = Et[j * D + i];
-  T mm_[D], Emp[D];
-  mv<T, D, D, D>(Fk, m, mm_);
-  mv<T, D, D, D>(ge + GL::E, mm_, Emp);
-#pragma unroll
-  for (int i = 0; i < D; ++i) ge[GL::G + i] = m[i] - Emp[i];
-  copy<T, D, D, D2, D>(Y + D, ge + GL::DM);
-  st_soa<T, GL::NG>(selems, n, k, ge);
-}
+  // smoother elements of the filtered states fm, fL (n + 1 of them)
+  static void smo_elements(int64_t n, const T* F, const T* QL, int64_t fts, const T* fm, const T* fL, T* selems,
+                           cudaStream_t st) {
+    if constexpr (kTeamL0) {
+      if (fts)
+        launch_l0<TSN, true, L0KFWs<T, D, DY, true>>(k_smo_elements_team<T, D, DY, TSN, true>, n, st, n, F, QL, fts,
+                                                     fm, fL, selems);
+      else
+        launch_l0<TSN, false, L0KFWs<T, D, DY, false>>(k_smo_elements_team<T, D, DY, TSN, false>, n, st, n, F, QL,
+                                                       fts, fm, fL, selems);
+    } else {
+      k_smo_elements<T, D><<<grid_for(n, 64), 64, 0, st>>>(n, F, QL, fts, fm, fL, selems);
+    }
+  }
+};
 
 }  // namespace pof

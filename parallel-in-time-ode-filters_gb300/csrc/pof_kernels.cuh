@@ -3,7 +3,8 @@
 // Time steps s = 0..n-1 (step s maps grid point s to s+1).  Level-0 chunks
 // hold C0 consecutive steps; chunk totals form level 1; levels l >= 1 fold C
 // consecutive elements into level l+1 until at most a few remain (the top).
-// Every kernel assigns one thread to one chunk.
+// These level-0 kernels assign one thread to one chunk (small D); the team
+// kernels (pof_team_kernels.cuh) take larger D and every level above.
 //
 // Internal buffers are structure-of-arrays: field f of element e of a level
 // with n elements lives at base[f * n + e], so a warp touching 32
@@ -126,35 +127,74 @@ __global__ void k_linearize(int64_t n, int field, const T* __restrict__ params, 
 }
 
 // ---------------------------------------------------------------------------
+// Level 0 with one thread per chunk (small D: the state fits registers).  A
+// step with the prior's structure (is_prior, is_exact_obs) takes the forms that
+// leave out its zeros; the transition model is tested once, per step only when
+// it varies.
+// ---------------------------------------------------------------------------
+template <typename T, int D, int DY>
+struct ChunkModel {
+  const StepModel& sm;
+  bool prior;
+  __device__ __forceinline__ explicit ChunkModel(const StepModel& sm_) : sm(sm_) {
+    prior = sm.ft_stride == 0 && is_prior<T, D, DY>(static_cast<const T*>(sm.F), static_cast<const T*>(sm.QL));
+  }
+  // whether step v takes the prior's form
+  __device__ __forceinline__ bool exact(const StepView<T, D, DY>& v) const {
+    const bool p = sm.ft_stride == 0 ? prior : is_prior<T, D, DY>(v.F, v.QL);
+    return p && is_exact_obs<T, D, DY>(v.H, v.R);
+  }
+};
+
+// kf_step in the form that fits; `thin`: the last DY columns of L are zero,
+// `lower`: L is lower triangular.
+template <typename T, int D, int DY, bool SMOOTH>
+__device__ __forceinline__ void kf_step_any(const StepView<T, D, DY>& v, bool exact, bool& thin, bool& lower, T* m,
+                                            T* L, double& ssq, double& yy, LogProd& lp, T* g, T* E, T* Dm) {
+  if constexpr (PriorDims<D, DY>::ok) {
+    if (exact && lower) {
+      if (thin)
+        kf_step_prior<T, D, DY, D - DY, SMOOTH>(v.F, v.QL, v.H, v.c, m, L, ssq, yy, lp, g, E, Dm);
+      else
+        kf_step_prior<T, D, DY, D, SMOOTH>(v.F, v.QL, v.H, v.c, m, L, ssq, yy, lp, g, E, Dm);
+      thin = true;
+      return;
+    }
+  }
+  kf_step<T, D, DY, SMOOTH>(v.F, v.QL, v.H, v.c, v.R, m, L, ssq, yy, lp, g, E, Dm);
+  thin = false;
+  lower = true;
+}
+
 // Filter, phase 1 (level 0): chunk totals.  Chunk 0 runs the filter from x0
 // and stores the filtering state as an element with A = 0, eta = 0, Z = 0
 // (the operator of filter.py:117-142 reads only b and U of a left operand
-// that holds x0).  Other chunks run the conditional fold.
-// ---------------------------------------------------------------------------
+// that holds x0); it has a block of its own, so no warp runs both kinds of
+// step.  Other chunks run the conditional fold.
 template <typename T, int D, int DY>
 __global__ void __launch_bounds__(64) k_filt_l0_reduce(int64_t n, int C0, StepModel sm, const T* __restrict__ x0m,
                                                        const T* __restrict__ x0L, T* __restrict__ out, int64_t n1) {
   using FL = FiltLayout<D>;
-  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int64_t t = blockIdx.x == 0 ? (threadIdx.x == 0 ? 0 : n1)
+                                    : 1 + (blockIdx.x - 1) * (int64_t)blockDim.x + threadIdx.x;
   if (t >= n1) return;
   const int64_t s0 = t * C0;
   const int64_t s1 = (s0 + C0 < n) ? s0 + C0 : n;
+  const ChunkModel<T, D, DY> cm(sm);
   T e[FL::NF];
+#pragma unroll
+  for (int i = 0; i < FL::NF; ++i) e[i] = T(0);
   if (t == 0) {
     T m[D], L[D * D];
     ld<T, D>(x0m, m);
     ld<T, D * D>(x0L, L);
-    T ss, nn;
-    {
-      StepView<T, D, DY> v(sm, 0);
-      kf_step<T, D, DY, false, false>(v.F, v.QL, v.H, v.c, v.R, m, L, ss, nn, nullptr, nullptr, nullptr);
-    }
-    for (int64_t s = 1; s < s1; ++s) {
+    double ssq = 0.0, yy = 0.0;
+    LogProd lp;
+    bool thin = false, lower = false;
+    for (int64_t s = 0; s < s1; ++s) {
       StepView<T, D, DY> v(sm, s);
-      kf_step<T, D, DY, false, true>(v.F, v.QL, v.H, v.c, v.R, m, L, ss, nn, nullptr, nullptr, nullptr);
+      kf_step_any<T, D, DY, false>(v, cm.exact(v), thin, lower, m, L, ssq, yy, lp, nullptr, nullptr, nullptr);
     }
-#pragma unroll
-    for (int i = 0; i < FL::NF; ++i) e[i] = T(0);
     st<T, D>(e + FL::B, m);
     st<T, D * D>(e + FL::U, L);
   } else {
@@ -164,84 +204,31 @@ __global__ void __launch_bounds__(64) k_filt_l0_reduce(int64_t n, int C0, StepMo
     T* eta = e + FL::ETA;
     T* Z = e + FL::Z;
 #pragma unroll
-    for (int i = 0; i < FL::NF; ++i) e[i] = T(0);
-#pragma unroll
     for (int i = 0; i < D; ++i) A[i * D + i] = T(1);
+    int nl = 0;  // columns of U: none at the start, D - DY after a step of the prior's form
     for (int64_t s = s0; s < s1; ++s) {
       if (!POF_IN(s, n)) break;
       StepView<T, D, DY> v(sm, s);
-      cond_fold_step<T, D, DY>(v.F, v.QL, v.H, v.c, v.R, A, b, U, eta, Z);
+      bool done = false;
+      if constexpr (PriorDims<D, DY>::ok) {
+        if (cm.exact(v)) {
+          if (nl == 0)
+            cond_fold_prior<T, D, DY, 0>(v.F, v.QL, v.H, v.c, A, b, U, eta, Z);
+          else if (nl == 1)
+            cond_fold_prior<T, D, DY, D - DY>(v.F, v.QL, v.H, v.c, A, b, U, eta, Z);
+          else
+            cond_fold_prior<T, D, DY, D>(v.F, v.QL, v.H, v.c, A, b, U, eta, Z);
+          nl = 1;
+          done = true;
+        }
+      }
+      if (!done) {
+        cond_fold_step<T, D, DY>(v.F, v.QL, v.H, v.c, v.R, A, b, U, eta, Z);
+        nl = 2;
+      }
     }
   }
   st_soa<T, FL::NF>(out, n1, t, e);
-}
-
-// Filter, phase 2 up-sweep: fold C consecutive general elements.
-template <typename T, int D>
-__global__ void __launch_bounds__(64) k_filt_reduce(const T* __restrict__ in, int64_t nin, int C, T* __restrict__ out,
-                                                    int64_t nout) {
-  using FL = FiltLayout<D>;
-  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (t >= nout) return;
-  const int64_t i0 = t * C;
-  const int64_t i1 = (i0 + C < nin) ? i0 + C : nin;
-  T a[FL::NF], b[FL::NF];
-  ld_soa<T, FL::NF>(in, nin, i0, a);
-  for (int64_t i = i0 + 1; i < i1; ++i) {
-    ld_soa<T, FL::NF>(in, nin, i, b);
-    filt_combine<T, D>(a + FL::A, a + FL::B, a + FL::U, a + FL::ETA, a + FL::Z, b + FL::A, b + FL::B, b + FL::U,
-                       b + FL::ETA, b + FL::Z);
-  }
-  st_soa<T, FL::NF>(out, nout, t, a);
-}
-
-// Advance a filtering state over element e (element 0 of every level holds x0
-// and is absolute: the state after it is its own (b, U)).
-template <typename T, int D>
-__device__ __forceinline__ void filt_advance(const T* __restrict__ elems, int64_t n, int64_t i, T* m, T* L) {
-  using FL = FiltLayout<D>;
-  T e[FL::NF];
-  ld_soa<T, FL::NF>(elems, n, i, e);
-  if (i == 0) {
-    ld<T, D>(e + FL::B, m);
-    ld<T, D * D>(e + FL::U, L);
-  } else {
-    filt_apply<T, D>(m, L, e + FL::A, e + FL::B, e + FL::U, e + FL::ETA, e + FL::Z);
-  }
-}
-
-// Filter, top of phase 2: the state before each top-level element (one thread).
-template <typename T, int D>
-__global__ void k_filt_top(const T* __restrict__ elems, int64_t n, const T* __restrict__ x0m,
-                           const T* __restrict__ x0L, T* __restrict__ states) {
-  using SL = StateLayout<D>;
-  if (blockIdx.x * blockDim.x + threadIdx.x != 0) return;
-  T st_[SL::NS];
-  ld<T, D>(x0m, st_ + SL::M);
-  ld<T, D * D>(x0L, st_ + SL::L);
-  for (int64_t i = 0; i < n; ++i) {
-    st_soa<T, SL::NS>(states, n, i, st_);
-    if (i + 1 < n) filt_advance<T, D>(elems, n, i, st_ + SL::M, st_ + SL::L);
-  }
-}
-
-// Filter, phase 2 down-sweep at level l >= 1: states before every element of
-// chunk t from the state before the chunk.
-template <typename T, int D>
-__global__ void __launch_bounds__(64) k_filt_down(const T* __restrict__ elems, int64_t n, int C,
-                                                  const T* __restrict__ states_up, int64_t nup,
-                                                  T* __restrict__ states) {
-  using SL = StateLayout<D>;
-  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (t >= nup) return;
-  const int64_t i0 = t * C;
-  const int64_t i1 = (i0 + C < n) ? i0 + C : n;
-  T st_[SL::NS];
-  ld_soa<T, SL::NS>(states_up, nup, t, st_);
-  for (int64_t i = i0; i < i1; ++i) {
-    st_soa<T, SL::NS>(states, n, i, st_);
-    if (i + 1 < i1) filt_advance<T, D>(elems, n, i, st_ + SL::M, st_ + SL::L);
-  }
 }
 
 // Filter, phase 3 (level 0): the square-root KF inside chunk t from the state
@@ -251,13 +238,15 @@ __global__ void __launch_bounds__(64) k_filt_down(const T* __restrict__ elems, i
 template <typename T, int D, int DY>
 __global__ void __launch_bounds__(64) k_filt_l0_down(int64_t n, int C0, StepModel sm, const T* __restrict__ states1,
                                                      int64_t n1, T* __restrict__ means, T* __restrict__ chols,
-                                                     T* __restrict__ selems, double* __restrict__ partials) {
+                                                     T* __restrict__ selems, double* __restrict__ partials,
+                                                     bool want_fobj) {
   using SL = StateLayout<D>;
   using GL = SmoLayout<D>;
   const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (t >= n1) return;
   const int64_t s0 = t * C0;
   const int64_t s1 = (s0 + C0 < n) ? s0 + C0 : n;
+  const ChunkModel<T, D, DY> cm(sm);
   T st_[SL::NS];
   ld_soa<T, SL::NS>(states1, n1, t, st_);
   T* m = st_ + SL::M;
@@ -266,39 +255,37 @@ __global__ void __launch_bounds__(64) k_filt_l0_down(int64_t n, int C0, StepMode
     st<T, D>(means, m);
     st<T, D * D>(chols, L);
   }
-  double ssq = 0.0, nll = 0.0, fobj = 0.0;
+  double ssq = 0.0, yy = 0.0, fobj = 0.0;
+  LogProd lp;
+  bool thin = false, lower = t != 0;  // chunk 0 starts from x0, whose chol may be any square root
   T ge[GL::NG];
   for (int64_t s = s0; s < s1; ++s) {
     if (!POF_IN(s, n)) break;
     StepView<T, D, DY> v(sm, s);
     T mold[D];
     ld<T, D>(m, mold);
-    T ss, nn;
-    if (s == 0)
-      kf_step<T, D, DY, true, false>(v.F, v.QL, v.H, v.c, v.R, m, L, ss, nn, ge + GL::G, ge + GL::E, ge + GL::DM);
-    else
-      kf_step<T, D, DY, true, true>(v.F, v.QL, v.H, v.c, v.R, m, L, ss, nn, ge + GL::G, ge + GL::E, ge + GL::DM);
-    ssq += (double)ss;
-    nll += (double)nn;
-    fobj += (double)objective_term<T, D>(v.F, v.QL, mold, m);
+    kf_step_any<T, D, DY, true>(v, cm.exact(v), thin, lower, m, L, ssq, yy, lp, ge + GL::G, ge + GL::E, ge + GL::DM);
+    if (want_fobj) fobj += (double)objective_term<T, D>(v.F, v.QL, mold, m);
     st_soa<T, GL::NG>(selems, n, s, ge);
     st<T, D>(means + (s + 1) * D, m);
     st<T, D * D>(chols + (s + 1) * D * D, L);
   }
   partials[P_SSQ * n1 + t] = ssq;
-  partials[P_NLL * n1 + t] = nll;
+  partials[P_NLL * n1 + t] = 0.5 * yy + lp.value() + (double)((s1 - s0) * DY) * Log2Pi<double>::half;
   partials[P_FOBJ * n1 + t] = fobj;
 }
 
 // ---------------------------------------------------------------------------
 // Smoother.  Element k (grid point k = 0..n-1) maps the smoothed state at
 // k+1 to the one at k; composites of a range [k0, k1) map the state at k1 to
-// the state at k0.
+// the state at k0.  The elements' factors are raw square roots, D - DY columns
+// after a step of the prior's form; the composites' are triangular.
 // ---------------------------------------------------------------------------
-template <typename T, int D>
-__global__ void __launch_bounds__(64) k_smo_reduce(const T* __restrict__ in, int64_t nin, int C, T* __restrict__ out,
-                                                   int64_t nout) {
+template <typename T, int D, int DY>
+__global__ void __launch_bounds__(64) k_smo_l0_reduce(const T* __restrict__ in, int64_t nin, int C,
+                                                      T* __restrict__ out, int64_t nout) {
   using GL = SmoLayout<D>;
+  constexpr int NT = DY < D ? D - DY : D;
   const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (t >= nout) return;
   const int64_t i0 = t * C;
@@ -307,58 +294,35 @@ __global__ void __launch_bounds__(64) k_smo_reduce(const T* __restrict__ in, int
   ld_soa<T, GL::NG>(in, nin, i0, a);
   for (int64_t i = i0 + 1; i < i1; ++i) {
     ld_soa<T, GL::NG>(in, nin, i, b);
-    smooth_combine<T, D>(b + GL::G, b + GL::E, b + GL::DM, a + GL::G, a + GL::E, a + GL::DM);
+    const bool thin = NT < D && last_cols_zero<T, D, D - NT>(b + GL::DM);
+    if (i == i0 + 1) {
+      if (thin)
+        smooth_combine<T, D, NT, true>(b + GL::G, b + GL::E, b + GL::DM, a + GL::G, a + GL::E, a + GL::DM);
+      else
+        smooth_combine<T, D, D, true>(b + GL::G, b + GL::E, b + GL::DM, a + GL::G, a + GL::E, a + GL::DM);
+    } else {
+      if (thin)
+        smooth_combine<T, D, NT, false>(b + GL::G, b + GL::E, b + GL::DM, a + GL::G, a + GL::E, a + GL::DM);
+      else
+        smooth_combine<T, D, D, false>(b + GL::G, b + GL::E, b + GL::DM, a + GL::G, a + GL::E, a + GL::DM);
+    }
+  }
+  if (i1 - i0 == 1) {
+    T* X = a + GL::DM;
+    lq_rows<T, D, D, D, D>(X);
+#pragma unroll
+    for (int i = 0; i < D; ++i)
+#pragma unroll
+      for (int j = i + 1; j < D; ++j) X[i * D + j] = T(0);
   }
   st_soa<T, GL::NG>(out, nout, t, a);
-}
-
-// Top of the smoother hierarchy: the smoothed state after every top-level
-// element, starting from the terminal (filtered) state (one thread).
-template <typename T, int D>
-__global__ void k_smo_top(const T* __restrict__ elems, int64_t n, const T* __restrict__ mT,
-                          const T* __restrict__ LT, T* __restrict__ ends) {
-  using SL = StateLayout<D>;
-  using GL = SmoLayout<D>;
-  if (blockIdx.x * blockDim.x + threadIdx.x != 0) return;
-  T st_[SL::NS];
-  ld<T, D>(mT, st_ + SL::M);
-  ld<T, D * D>(LT, st_ + SL::L);
-  for (int64_t i = n - 1; i >= 0; --i) {
-    st_soa<T, SL::NS>(ends, n, i, st_);
-    if (i > 0) {
-      T e[GL::NG];
-      ld_soa<T, GL::NG>(elems, n, i, e);
-      smooth_apply<T, D>(e + GL::G, e + GL::E, e + GL::DM, st_ + SL::M, st_ + SL::L);
-    }
-  }
-}
-
-template <typename T, int D>
-__global__ void __launch_bounds__(64) k_smo_down(const T* __restrict__ elems, int64_t n, int C,
-                                                 const T* __restrict__ ends_up, int64_t nup, T* __restrict__ ends) {
-  using SL = StateLayout<D>;
-  using GL = SmoLayout<D>;
-  const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (t >= nup) return;
-  const int64_t i0 = t * C;
-  const int64_t i1 = (i0 + C < n) ? i0 + C : n;
-  T st_[SL::NS];
-  ld_soa<T, SL::NS>(ends_up, nup, t, st_);
-  for (int64_t i = i1 - 1; i >= i0; --i) {
-    st_soa<T, SL::NS>(ends, n, i, st_);
-    if (i > i0) {
-      T e[GL::NG];
-      ld_soa<T, GL::NG>(elems, n, i, e);
-      smooth_apply<T, D>(e + GL::G, e + GL::E, e + GL::DM, st_ + SL::M, st_ + SL::L);
-    }
-  }
 }
 
 // Smoother, phase 3 (level 0): backward recursion inside chunk t from the
 // smoothed state at its end.  Writes smoothed means and chols (chols scaled
 // by *scale when scale != nullptr), and partial sums of the smoother
 // objective and of the convergence test against means_old.
-template <typename T, int D>
+template <typename T, int D, int DY>
 __global__ void __launch_bounds__(64) k_smo_l0_down(int64_t n, int C0, const T* __restrict__ F,
                                                     const T* __restrict__ QL, int64_t ft_stride,
                                                     const T* __restrict__ selems, const T* __restrict__ ends1,
@@ -367,6 +331,7 @@ __global__ void __launch_bounds__(64) k_smo_l0_down(int64_t n, int C0, const T* 
                                                     double c_mrtol, double c_matol, double* __restrict__ partials) {
   using SL = StateLayout<D>;
   using GL = SmoLayout<D>;
+  constexpr int NT = DY < D ? D - DY : D;
   const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (t >= n1) return;
   const int64_t s0 = t * C0;
@@ -376,7 +341,8 @@ __global__ void __launch_bounds__(64) k_smo_l0_down(int64_t n, int C0, const T* 
   ld_soa<T, SL::NS>(ends1, n1, t, st_);
   T* m = st_ + SL::M;
   T* L = st_ + SL::L;
-  double sobj = 0.0, notclose = 0.0;
+  double sobj = 0.0;
+  int notclose = 0;
   auto close_count = [&](int64_t k, const T* mk) {
     if (!means_old) return;
 #pragma unroll
@@ -387,7 +353,7 @@ __global__ void __launch_bounds__(64) k_smo_l0_down(int64_t n, int C0, const T* 
         ok = fabs(a - b) <= c_matol + c_mrtol * fabs(b);
       else
         ok = (a == b);
-      notclose += ok ? 0.0 : 1.0;
+      notclose += ok ? 0 : 1;
     }
   };
   if (s1 == n) {  // the terminal grid point n belongs to the last chunk
@@ -398,20 +364,29 @@ __global__ void __launch_bounds__(64) k_smo_l0_down(int64_t n, int C0, const T* 
     }
   }
   T ge[GL::NG];
+  bool lower = s1 != n;  // the terminal state may be the caller's, with any square root
   for (int64_t k = s1 - 1; k >= s0; --k) {
     if (!POF_IN(k, n)) break;
     T mnext[D];
     ld<T, D>(m, mnext);
     ld_soa<T, GL::NG>(selems, n, k, ge);
-    smooth_apply<T, D>(ge + GL::G, ge + GL::E, ge + GL::DM, m, L);
+    if (lower && NT < D && last_cols_zero<T, D, D - NT>(ge + GL::DM))
+      smooth_apply<T, D, NT, true>(ge + GL::G, ge + GL::E, ge + GL::DM, m, L);
+    else
+      smooth_apply<T, D, D, false>(ge + GL::G, ge + GL::E, ge + GL::DM, m, L);
+    lower = true;
     sobj += (double)objective_term<T, D>(F + k * ft_stride, QL + k * ft_stride, m, mnext);
     close_count(k, m);
     st<T, D>(means + k * D, m);
+    if (scale) {
 #pragma unroll
-    for (int i = 0; i < D * D; ++i) chols[k * D * D + i] = L[i] * sc;
+      for (int i = 0; i < D * D; ++i) chols[k * D * D + i] = L[i] * sc;
+    } else {
+      st<T, D * D>(chols + k * D * D, L);
+    }
   }
   partials[P_SOBJ * n1 + t] = sobj;
-  partials[P_NOTCLOSE * n1 + t] = notclose;
+  partials[P_NOTCLOSE * n1 + t] = (double)notclose;
 }
 
 // Fixed-order sum of per-chunk partials (deterministic: the same sums in the

@@ -204,51 +204,6 @@ __device__ __forceinline__ void mm(const T* __restrict__ A, const T* __restrict_
   }
 }
 
-// C(MxN) = A(MxK) * B(KxN) with B lower-triangular (K == N): skips B's zeros.
-template <typename T, int M, int K, int LDA, int LDB, int LDC>
-__device__ __forceinline__ void mm_lowerB(const T* __restrict__ A, const T* __restrict__ B, T* __restrict__ C) {
-#pragma unroll
-  for (int i = 0; i < M; ++i) {
-#pragma unroll
-    for (int j = 0; j < K; ++j) {
-      T s = T(0);
-#pragma unroll
-      for (int k = j; k < K; ++k) s = fma(A[i * LDA + k], B[k * LDB + j], s);
-      C[i * LDC + j] = s;
-    }
-  }
-}
-
-// C(MxN) = A^T * B with A (KxM), B (KxN)
-template <typename T, int M, int K, int N, int LDA, int LDB, int LDC>
-__device__ __forceinline__ void mtm(const T* __restrict__ A, const T* __restrict__ B, T* __restrict__ C) {
-#pragma unroll
-  for (int i = 0; i < M; ++i) {
-#pragma unroll
-    for (int j = 0; j < N; ++j) {
-      T s = T(0);
-#pragma unroll
-      for (int k = 0; k < K; ++k) s = fma(A[k * LDA + i], B[k * LDB + j], s);
-      C[i * LDC + j] = s;
-    }
-  }
-}
-
-// C(MxN) = A(MxK) * B^T with B (NxK)
-template <typename T, int M, int K, int N, int LDA, int LDB, int LDC>
-__device__ __forceinline__ void mmt(const T* __restrict__ A, const T* __restrict__ B, T* __restrict__ C) {
-#pragma unroll
-  for (int i = 0; i < M; ++i) {
-#pragma unroll
-    for (int j = 0; j < N; ++j) {
-      T s = T(0);
-#pragma unroll
-      for (int k = 0; k < K; ++k) s = fma(A[i * LDA + k], B[j * LDB + k], s);
-      C[i * LDC + j] = s;
-    }
-  }
-}
-
 // y(M) = A(MxN) x(N)
 template <typename T, int M, int N, int LDA>
 __device__ __forceinline__ void mv(const T* __restrict__ A, const T* __restrict__ x, T* __restrict__ y) {
@@ -273,89 +228,73 @@ __device__ __forceinline__ void mtv(const T* __restrict__ A, const T* __restrict
   }
 }
 
-// In-place lower-triangular square root of an M x NC matrix X (M <= NC):
-// on return X[:, :M] holds L (lower triangular) with L L^T = X X^T, and
-// X[:, M:] and the strict upper triangle are zero.
+// The LQ factorisation by Householder reflectors of the first M of the MX
+// rows of X (NC columns): afterwards X[:M, :M] holds L in its lower triangle
+// (L L^T = the M rows' X X^T) and the rows below are multiplied by the same
+// orthogonal matrix; what lies right of the diagonal in the M rows is left as
+// it is and must not be read.
 //
-// This is the LQ factorisation X = L Q computed as LAPACK's dgeqr2 computes
-// the R factor of X^T: one Householder reflector per row, in row order, with
-// dlarfg's conventions -- beta = -sign(alpha) * ||(alpha, x)||, and no
-// reflection (tau = 0, R_jj = alpha) when the tail x is exactly zero.  The
-// reference computes tria as qr(A^T, mode="r")^T (pof/utils.py:33-41), so
-// the diagonal signs of L match LAPACK's for the same input.
-template <typename T, int M, int NC, int LD>
-__device__ __forceinline__ void tria(T* X) {
-  static_assert(M <= NC, "tria needs M <= NC");
+// LAPACK's dgeqr2 computes the R factor of X^T so: one reflector per row, in
+// row order, with dlarfg's conventions -- beta = -sign(alpha) * ||(alpha, x)||,
+// and no reflection (tau = 0, R_jj = alpha) when the tail x is exactly zero.
+// The reference computes tria as qr(A^T, mode="r")^T (pof/utils.py:33-41).
+template <typename T, int M, int MX, int NC, int LD>
+__device__ __forceinline__ void lq_rows(T* X) {
 #pragma unroll
   for (int j = 0; j < M; ++j) {
     T* xj = X + j * LD;
-    const T alpha = xj[j];
     T xn2 = T(0);
 #pragma unroll
     for (int k = j + 1; k < NC; ++k) xn2 = fma(xj[k], xj[k], xn2);
-    T beta, tau, scal;
-    householder(alpha, xn2, beta, tau, scal);
+    if (!is_zero(xn2)) {
+      const Reflector<T> h(xj[j], xn2);
+      xj[j] = h.beta;
 #pragma unroll
-    for (int k = j + 1; k < NC; ++k) xj[k] *= scal;  // reflector v (v_j = 1)
-    xj[j] = beta;
+      for (int i = j + 1; i < MX; ++i) {
+        T* xi = X + i * LD;
+        T dot = T(0), ws;
 #pragma unroll
-    for (int i = j + 1; i < M; ++i) {
-      T* xi = X + i * LD;
-      T w = xi[j];
+        for (int k = j + 1; k < NC; ++k) dot = fma(xi[k], xj[k], dot);
+        xi[j] = h.row(xi[j], dot, ws);
 #pragma unroll
-      for (int k = j + 1; k < NC; ++k) w = fma(xi[k], xj[k], w);
-      w *= tau;
-      xi[j] -= w;
-#pragma unroll
-      for (int k = j + 1; k < NC; ++k) xi[k] = fma(-w, xj[k], xi[k]);
+        for (int k = j + 1; k < NC; ++k) xi[k] = fma(-ws, xj[k], xi[k]);
+      }
     }
-#pragma unroll
-    for (int k = j + 1; k < NC; ++k) xj[k] = T(0);
   }
 }
 
-// Same reflectors as tria<M, NC>, additionally applied to the MB rows of a
-// second block Y (MB x NC, leading dim LDY) that sits below X.  Equivalent to
-// the first M reflectors of tria on the stacked (M+MB) x NC matrix [X; Y].
-template <typename T, int M, int MB, int NC, int LD, int LDY>
-__device__ __forceinline__ void tria_top(T* X, T* Y) {
-  static_assert(M <= NC, "tria_top needs M <= NC");
+// LQ with a triangular pivot block (t_lq of pof_team.cuh, one thread): rows
+// [P | W], P lower triangular M x M, W with NW columns, over MB rows [Yp | Yw]:
+// P becomes L with L L^T = P P^T + W W^T, the rows below are multiplied by the
+// same orthogonal matrix.  Q > 0: row j of W ends with column (j / Q + 1) Q - 1
+// (W = F S, F block-diagonal, S lower triangular).  W is left as it is.
+template <typename T, int M, int NW, int MB, int Q, int LDP, int LDW, int LDYP, int LDYW>
+__device__ __forceinline__ void lq_pivot(T* P, T* W, T* Yp, T* Yw) {
 #pragma unroll
   for (int j = 0; j < M; ++j) {
-    T* xj = X + j * LD;
-    const T alpha = xj[j];
+    const int nw = Q > 0 ? ((j / (Q > 0 ? Q : 1) + 1) * Q < NW ? (j / (Q > 0 ? Q : 1) + 1) * Q : NW) : NW;
+    T* wj = W + j * LDW;
     T xn2 = T(0);
 #pragma unroll
-    for (int k = j + 1; k < NC; ++k) xn2 = fma(xj[k], xj[k], xn2);
-    T beta, tau, scal;
-    householder(alpha, xn2, beta, tau, scal);
+    for (int k = 0; k < NW; ++k)
+      if (k < nw) xn2 = fma(wj[k], wj[k], xn2);
+    if (!is_zero(xn2)) {
+      const Reflector<T> h(P[j * LDP + j], xn2);
+      P[j * LDP + j] = h.beta;
 #pragma unroll
-    for (int k = j + 1; k < NC; ++k) xj[k] *= scal;
-    xj[j] = beta;
+      for (int i = j + 1; i < M + MB; ++i) {
+        T* y = i < M ? W + i * LDW : Yw + (i - M) * LDYW;
+        T& a = i < M ? P[i * LDP + j] : Yp[(i - M) * LDYP + j];
+        T dot = T(0), ws;
 #pragma unroll
-    for (int i = j + 1; i < M; ++i) {
-      T* xi = X + i * LD;
-      T w = xi[j];
+        for (int k = 0; k < NW; ++k)
+          if (k < nw) dot = fma(y[k], wj[k], dot);
+        a = h.row(a, dot, ws);
 #pragma unroll
-      for (int k = j + 1; k < NC; ++k) w = fma(xi[k], xj[k], w);
-      w *= tau;
-      xi[j] -= w;
-#pragma unroll
-      for (int k = j + 1; k < NC; ++k) xi[k] = fma(-w, xj[k], xi[k]);
+        for (int k = 0; k < NW; ++k)
+          if (k < nw) y[k] = fma(-ws, wj[k], y[k]);
+      }
     }
-#pragma unroll
-    for (int i = 0; i < MB; ++i) {
-      T* yi = Y + i * LDY;
-      T w = yi[j];
-#pragma unroll
-      for (int k = j + 1; k < NC; ++k) w = fma(yi[k], xj[k], w);
-      w *= tau;
-      yi[j] -= w;
-#pragma unroll
-      for (int k = j + 1; k < NC; ++k) yi[k] = fma(-w, xj[k], yi[k]);
-    }
-#pragma unroll
-    for (int k = j + 1; k < NC; ++k) xj[k] = T(0);
   }
 }
 
@@ -394,22 +333,6 @@ __device__ __forceinline__ void trsm_l(const T* __restrict__ L, T* B) {
       T s = B[i * LDB + j];
 #pragma unroll
       for (int k = 0; k < i; ++k) s = fma(-L[i * LDL + k], B[k * LDB + j], s);
-      B[i * LDB + j] = s * inv;
-    }
-  }
-}
-
-// B(M x NR) <- L^{-T} B
-template <typename T, int M, int NR, int LDL, int LDB>
-__device__ __forceinline__ void trsm_lt(const T* __restrict__ L, T* B) {
-#pragma unroll
-  for (int i = M - 1; i >= 0; --i) {
-    const T inv = rcp(L[i * LDL + i]);
-#pragma unroll
-    for (int j = 0; j < NR; ++j) {
-      T s = B[i * LDB + j];
-#pragma unroll
-      for (int k = i + 1; k < M; ++k) s = fma(-L[k * LDL + i], B[k * LDB + j], s);
       B[i * LDB + j] = s * inv;
     }
   }

@@ -14,43 +14,17 @@ template <typename T, int D>
 __device__ __forceinline__ void seq_smooth_step(const T* __restrict__ F, const T* __restrict__ QL,
                                                 const T* __restrict__ mf, const T* __restrict__ Lf, T* ms, T* Ls) {
   constexpr int D2 = 2 * D;
-  T X[D * D2], Y[D * D2];
+  T X[D2 * D2];
   mm<T, D, D, D, D, D, D2>(F, Lf, X);
   copy<T, D, D, D, D2>(QL, X + D);
-  copy<T, D, D, D, D2>(Lf, Y);
-  zero<T, D, D, D2>(Y + D);
-  tria_top<T, D, D, D2, D2, D2>(X, Y);
-  tria<T, D, D, D2>(Y + D);
-  // gain^T = Phi11^{-T} Phi21^T
-  T Gt[D * D];
-#pragma unroll
-  for (int i = 0; i < D; ++i)
-#pragma unroll
-    for (int j = 0; j < D; ++j) Gt[i * D + j] = Y[j * D2 + i];
-  trsm_lt<T, D, D, D2, D>(X, Gt);
-  T Fm[D], diff[D];
+  copy<T, D, D, D, D2>(Lf, X + D * D2);
+  zero<T, D, D, D2>(X + D * D2 + D);
+  lq_rows<T, D, D2, D2, D2>(X);
+  T Fm[D], g[D], E[D * D], Dm[D * D];
   mv<T, D, D, D>(F, mf, Fm);
-#pragma unroll
-  for (int i = 0; i < D; ++i) diff[i] = ms[i] - Fm[i];
-  T mn[D];
-  mtv<T, D, D, D>(Gt, diff, mn);
-#pragma unroll
-  for (int i = 0; i < D; ++i) mn[i] += mf[i];
-  // [Phi22, gain Ls]
-  T Z[D * D2];
-  copy<T, D, D, D2, D2>(Y + D, Z);
-#pragma unroll
-  for (int i = 0; i < D; ++i)
-#pragma unroll
-    for (int j = 0; j < D; ++j) {
-      T s = T(0);
-#pragma unroll
-      for (int k = 0; k < D; ++k) s = fma(Gt[k * D + i], Ls[k * D + j], s);
-      Z[i * D2 + D + j] = s;
-    }
-  tria<T, D, D2, D2>(Z);
-  ld<T, D>(mn, ms);
-  copy<T, D, D, D2, D>(Z, Ls);
+  gain<T, D, D2, D2>(X, X + D * D2, mf, Fm, g, E);
+  copy<T, D, D, D2, D>(X + D * D2 + D, Dm);
+  smooth_apply<T, D, D, false>(g, E, Dm, ms, Ls);
 }
 
 // Whole sequential filter (+ smoother when `smooth`) of one trajectory.  FIELD >= 1: EKF,
@@ -70,7 +44,8 @@ __global__ void k_seq_filtsmooth(int64_t n, StepModel sm, int field, const T* __
   ld<T, D * D>(x0L, L);
   st<T, D>(means, m);
   st<T, D * D>(chols, L);
-  double ssq = 0.0, ell = 0.0;
+  double ssq = 0.0, yy = 0.0;
+  LogProd lp;
   for (int64_t s = 0; s < n; ++s) {
     const T* F = static_cast<const T*>(sm.F) + s * sm.ft_stride;
     const T* QL = static_cast<const T*>(sm.QL) + s * sm.ft_stride;
@@ -108,16 +83,11 @@ __global__ void k_seq_filtsmooth(int64_t n, StepModel sm, int field, const T* __
       H = Hb;
       c = cb;
     }
-    T ss, nn;
-    if (s == 0)
-      kf_step<T, D, DY, false, false>(F, QL, H, c, R, m, L, ss, nn, nullptr, nullptr, nullptr);
-    else
-      kf_step<T, D, DY, false, true>(F, QL, H, c, R, m, L, ss, nn, nullptr, nullptr, nullptr);
-    ssq += (double)ss;
-    ell -= (double)nn;
+    kf_step<T, D, DY, false>(F, QL, H, c, R, m, L, ssq, yy, lp, nullptr, nullptr, nullptr);
     st<T, D>(means + (s + 1) * D, m);
     st<T, D * D>(chols + (s + 1) * D * D, L);
   }
+  const double ell = -(0.5 * yy + lp.value() + (double)(n * DY) * Log2Pi<double>::half);
   // backward pass (pof/sequential_filtsmooth/smoother.py:8-28)
   double obj = 0.0;
   for (int64_t k = n - 1; smooth && k >= 0; --k) {

@@ -35,9 +35,8 @@ struct OpsImpl {
   }
   static void smo_elements(int64_t n, const void* F, const void* QL, int64_t fts, const void* fm, const void* fL,
                            void* selems, cudaStream_t st) {
-    k_smo_elements<T, D><<<grid_for(n, 64), 64, 0, st>>>(n, static_cast<const T*>(F), static_cast<const T*>(QL),
-                                                         fts, static_cast<const T*>(fm),
-                                                         static_cast<const T*>(fL), static_cast<T*>(selems));
+    Driver<T, D, DY>::smo_elements(n, static_cast<const T*>(F), static_cast<const T*>(QL), fts,
+                                   static_cast<const T*>(fm), static_cast<const T*>(fL), static_cast<T*>(selems), st);
   }
   static void linearize(int64_t n, int field, const void* params, double p0, double p1, const void* means, void* H,
                         void* c, cudaStream_t st) {

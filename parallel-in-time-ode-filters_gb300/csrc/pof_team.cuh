@@ -17,7 +17,7 @@
 // cols) so the lanes of a team reading one column hit distinct banks.
 #pragma once
 
-#include "pof_linalg.cuh"
+#include "pof_ops.cuh"
 
 namespace pof {
 
@@ -735,30 +735,6 @@ __device__ __forceinline__ StepObs t_load_step(const Team<TS>& tm, WS& w, const 
   return StepObs{(int)__reduce_max_sync(tm.mask, (unsigned)h1), !noise};
 }
 
-// Running log of a product of |x| (the observation factor's diagonal over a
-// chunk's steps): mantissas multiplied, exponents added, one logarithm at the
-// end instead of one per step (about 25 FP64 instructions each).
-struct LogProd {
-  double p = 1.0, extra = 0.0;
-  long long e = 0;
-  __device__ __forceinline__ void mul(double x) {
-    const long long b = __double_as_longlong(x) & 0x7fffffffffffffffLL;
-    const int ex = (int)(b >> 52);
-    if (ex == 0 || ex == 0x7ff) {
-      extra += log(fabs(x));  // zero, subnormal, infinite, NaN
-      return;
-    }
-    p *= __longlong_as_double((b & 0xfffffffffffffLL) | (1023LL << 52));  // p in [1, 4)
-    const long long pb = __double_as_longlong(p);
-    e += (ex - 1023) + ((int)(pb >> 52) - 1023);
-    p = __longlong_as_double((pb & 0xfffffffffffffLL) | (1023LL << 52));
-  }
-  __device__ __forceinline__ void mul(float x) { extra += (double)logf(fabsf(x)); }
-  __device__ __forceinline__ double value() const {
-    return log(p) + (double)e * 0.69314718055994530941723212145818 + extra;
-  }
-};
-
 // [QL | F L] in w.X and, when SMOOTH, [0 | L] in w.Y; their reflectors.
 template <typename T, int TS, int D, int DY, bool SMOOTH, typename WS>
 __device__ __forceinline__ void t_predict(const Team<TS>& tm, WS& w, const T* F, const T* QL, StepStruct ss, int nl,
@@ -856,17 +832,14 @@ __device__ __forceinline__ void t_innovation(const Team<TS>& tm, WS& w, const T*
   }
 }
 
-// One square-root KF step from the filtered state (m, L), L with nl nonzero
-// columns, at grid s, fused with the smoother element of grid s when SMOOTH:
-// g, E, and its factor in Y[:, D : D + nl] (a D x nl square root of
-// Phi22 Phi22^T, not triangular).  Adds ||Psi11^{-T} r||^2 to ssq (whiten
-// quirk, pof/utils.py:110-112), ||Psi11^{-1} r||^2 to yy and |Psi11_ii| to
-// lane i's lp; returns the column count of the new L.
+// Predicted mean and factor from the state (m, L), L with nl nonzero columns,
+// and the smoother element of that state when SMOOTH: g, E, and its factor in
+// Y[:, D : D + nl] (a D x nl square root of Phi22 Phi22^T, not triangular).
 template <typename T, int TS, int D, int DY, bool SMOOTH, typename WS>
-__device__ __forceinline__ int t_kf_step(const Team<TS>& tm, WS& w, const T* F, const T* QL, StepStruct ss,
-                                         StepObs ob, int nl, bool lower, double& ssq, double& yy, LogProd& lp) {
+__device__ __forceinline__ void t_predict_gain(const Team<TS>& tm, WS& w, const T* F, const T* QL, StepStruct ss,
+                                               int nl, bool lower) {
   using W = StepDims<T, D, DY>;
-  constexpr int L1 = W::LD1, L2 = W::LD2, LP = W::LDP;
+  constexpr int L1 = W::LD1, L2 = W::LD2;
   static_assert(D <= TS && DY <= TS, "one row of the state per lane");
   for (int i = tm.r; i < D; i += TS) {
     const int k0 = ss.wf ? i : 0, k1 = ss.wf ? (i / ss.wf + 1) * ss.wf : D;
@@ -897,6 +870,18 @@ __device__ __forceinline__ int t_kf_step(const Team<TS>& tm, WS& w, const T* F, 
       for (int i = 0; i < D; ++i) w.E[j * L1 + i] = x[i];
     }
   }
+}
+
+// One square-root KF step from the filtered state (m, L) at grid s
+// (t_predict_gain, then the update).  Adds ||Psi11^{-T} r||^2 to ssq (whiten
+// quirk, pof/utils.py:110-112), ||Psi11^{-1} r||^2 to yy and |Psi11_ii| to
+// lane i's lp; returns the column count of the new L.
+template <typename T, int TS, int D, int DY, bool SMOOTH, typename WS>
+__device__ __forceinline__ int t_kf_step(const Team<TS>& tm, WS& w, const T* F, const T* QL, StepStruct ss,
+                                         StepObs ob, int nl, bool lower, double& ssq, double& yy, LogProd& lp) {
+  using W = StepDims<T, D, DY>;
+  constexpr int LP = W::LDP;
+  t_predict_gain<T, TS, D, DY, SMOOTH>(tm, w, F, QL, ss, nl, lower);
   t_psi<T, TS, D, DY>(tm, w, ob);
   T r[DY], rdv[DY], wv[DY], wq[DY];
   t_innovation<T, TS, D, DY>(tm, w, w.mp, ob.h1, r, rdv, wv);

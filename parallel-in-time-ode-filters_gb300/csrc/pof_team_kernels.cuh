@@ -628,6 +628,28 @@ __device__ __forceinline__ void t_store_selem(const Team<TS>& tm, T* base, int64
   }
 }
 
+// Smoother elements of given filtered states (pof_smoothing), one team per
+// step; the states' factors may be any square roots.
+template <typename T, int D, int DY, int TS, bool PS>
+__global__ void k_smo_elements_team(int64_t n, const T* __restrict__ F, const T* __restrict__ QL, int64_t ft_stride,
+                                    const T* __restrict__ fmeans, const T* __restrict__ fchols,
+                                    T* __restrict__ selems) {
+  using WS = L0KFWs<T, D, DY, PS>;
+  POF_L0_PROLOGUE(WS, PS)
+  if constexpr (!PS) load_fq_block<T, TS, D>(tm, fq, F, QL, StepDims<T, D, DY>::Q1);
+  if (t >= n) return;
+  StepKFWs<T, D, DY>& w = ws_.s;
+  const StepModel sm{F, QL, ft_stride, nullptr, nullptr, nullptr, 0};
+  fq_step<PS, T, TS, D>(tm, fq, sm, t, false, StepDims<T, D, DY>::Q1);
+  t_load_state_plain<T, TS, D>(tm, fmeans + t * D, fchols + t * D * D, w.m, w.L);
+  tm.sync();
+  bool lower;
+  const int nl = t_ncols<T, TS, D, D, Ld<D>::v>(tm, w.L, &lower);
+  t_predict_gain<T, TS, D, DY, true>(tm, w, fq.F, fq.QL, StepStruct{fq.wq != 0, fq.wf}, nl, lower);
+  tm.sync();
+  t_store_selem<T, TS, D, DY>(tm, selems, n, t, w, nl);
+}
+
 // The chunk's partial sums: sigma^2 terms, NLL (the constant of its steps and
 // the logarithms added here) and filter objective.
 template <int TS, int DY>
