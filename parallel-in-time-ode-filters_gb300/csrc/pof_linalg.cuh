@@ -42,53 +42,63 @@ __device__ __forceinline__ bool pof_check_fail(int line) {
 // Reciprocal and reciprocal square root of a double, for the scalars of the
 // Householder reflectors and the diagonal solves.
 //
-// GB300 runs FP64 at 1/64 of the FP32 rate and a warp instruction holds an
-// SM sub-partition's FP64 pipe for the same time however many of its lanes
-// are active, so the instruction sequences of IEEE double division and
-// square root -- computed once per reflector, often on one lane -- are a
-// large share of a small factorization's FP64 instructions.  These take a
-// single-precision hardware approximation of the exponent-normalized
-// argument as the seed (the float operand and the widened result are built
-// with integer operations, so no FP64 conversion is issued), then ONE
-// third-order correction in double precision (Householder's iteration of
-// order 3; Halley's method for the square root):
+// GB300 runs FP64 at 1/64 of the FP32 rate: an FP64 instruction of a warp
+// holds its SM sub-partition's FP64 pipe for 64 cycles, whatever its lanes
+// do, so the instruction sequences of IEEE double division and square root
+// -- computed once per reflector -- are a large share of a small
+// factorization's time.  These take a single-precision hardware
+// approximation of the argument's leading 21 significand bits as the seed
+// (the float operand and the widened result are built with 32-bit integer
+// operations, so no FP64 conversion is issued), then ONE third-order
+// correction in double precision (Householder's iteration of order 3;
+// Halley's method for the square root):
 //   1/a:       r = 1 - a y,     y <- y (1 + r + r^2)
 //   1/sqrt(a): r = 1 - a y^2,   y <- y (1 + r/2 + 3 r^2/8)
-// which cubes the seed's relative error (below ~4e-7: truncation of the
-// argument to 23 fraction bits plus the approximation) to below 1e-19, so
-// the result is within a few units in the last place of the correctly
-// rounded value: 3 and 5 FP64 instructions.  Arguments whose binary
-// exponent is beyond +-1000 (zero, subnormals, infinities, NaN included)
-// take the IEEE operations.
+// which cubes the seed's relative error (below ~1.2e-6: truncation of the
+// argument plus the approximation) to below 2e-18, so the result is within a
+// few units in the last place of the correctly rounded value: 3 and 5 FP64
+// instructions.  Arguments whose binary exponent is beyond +-1000 (zero,
+// subnormals, infinities, NaN included) take the IEEE operations.
 // ---------------------------------------------------------------------------
+__device__ __forceinline__ float approx_rcp(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float approx_rsqrt(float x) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
 
-// double with the sign bit `sign`, binary exponent `e` and the fraction of
-// the float f (exact)
-__device__ __forceinline__ double widen_with_exp(float f, int e, long long sign) {
-  const unsigned fb = __float_as_uint(f);
-  const long long ex = (long long)((int)((fb >> 23) & 0xff) - 127 + e + 1023) << 52;
-  return __longlong_as_double(sign | ex | ((long long)(fb & 0x7fffff) << 29));
+// high word of a double whose binary exponent is within +-1000
+__device__ __forceinline__ bool exp_in_range(int hi) {
+  return (unsigned)(((hi >> 20) & 0x7ff) - 23) <= 2000u;
+}
+// the leading significand bits of the double with high word hi, times 2^p
+__device__ __forceinline__ float lead_float(int hi, int p) {
+  return __int_as_float((((hi << 3) & 0x007ffff8) | 0x3f800000) + (p << 23));
+}
+// the float f > 0 times 2^e as a double (exact; no FP64 instruction)
+__device__ __forceinline__ double widen_with_exp(float f, int e) {
+  const int b = __float_as_int(f);
+  return __hiloint2double((b >> 3) + ((896 + e) << 20), b << 29);
 }
 
 __device__ __forceinline__ double rcp_nr(double a) {
-  const long long bits = __double_as_longlong(a);
-  const int e = (int)((bits >> 52) & 0x7ff) - 1023;
-  if (e < -1000 || e > 1000) return 1.0 / a;
-  // |a| = m 2^e, m in [1, 2): seed 1/m in single precision, times 2^-e
-  const float mf = __int_as_float(0x3f800000 | (int)((bits >> 29) & 0x7fffff));
-  const double y = widen_with_exp(__frcp_rn(mf), -e, bits & (1LL << 63));
+  const int hi = __double2hiint(a);
+  if (!exp_in_range(hi)) return 1.0 / a;
+  const double ym = widen_with_exp(approx_rcp(lead_float(hi, 0)), 1023 - ((hi >> 20) & 0x7ff));
+  const double y = __hiloint2double(__double2hiint(ym) | (hi & 0x80000000), __double2loint(ym));
   const double r = fma(-a, y, 1.0);
   return fma(y, fma(r, r, r), y);
 }
 
 __device__ __forceinline__ double rsqrt_nr(double a) {
-  const long long bits = __double_as_longlong(a);
-  const int e = (int)((bits >> 52) & 0x7ff) - 1023;
-  if (e < -1000 || e > 1000 || bits < 0) return 1.0 / sqrt(a);
-  // a = m 4^k with m in [1, 4): seed 1/sqrt(m) in single precision, times 2^-k
-  const int k = e >> 1;
-  const float mf = __int_as_float(((127 + e - 2 * k) << 23) | (int)((bits >> 29) & 0x7fffff));
-  const double y = widen_with_exp(rsqrtf(mf), -k, 0);
+  const int hi = __double2hiint(a);
+  if (!exp_in_range(hi) || hi < 0) return 1.0 / sqrt(a);
+  const int t = hi - 0x3ff00000, k = t >> 21;  // a = m 4^k with m in [1, 4)
+  const double y = widen_with_exp(approx_rsqrt(lead_float(hi, (t >> 20) & 1)), -k);
   const double r = fma(-(a * y), y, 1.0);
   return fma(y, r * fma(r, 0.375, 0.5), y);
 }
@@ -139,7 +149,8 @@ __device__ __forceinline__ bool is_zero(float x) { return (__float_as_uint(x) <<
 //     ws = -kap (u a + dot), w = u ws; ||(alpha, x)|| = h and
 //     1 / (u beta) = -1 / (a2 + |alpha| h) from single-precision seeds and one
 //     third-order correction each (as rsqrt_nr and rcp_nr), 11 FP64
-//     instructions of scalars and 2 per row;
+//     instructions of scalars and 2 per row; measured alone on a warp
+//     1399 cycles with 64-bit integer seeds one after the other;
 //   float: w = tau (a + scal dot), ws = w scal (kap would leave float's range
 //     for tails below 1e-19).
 // For xn2 != 0 only.
@@ -151,25 +162,31 @@ struct Reflector<double> {
   double beta, u, kap;
   __device__ __forceinline__ Reflector(double alpha, double xn2) {
     const double a2 = fma(alpha, alpha, xn2);
-    const long long bits = __double_as_longlong(a2);
-    const int e = (int)((bits >> 52) & 0x7ff) - 1023;
+    const int hi = __double2hiint(a2), ahi = __double2hiint(alpha) & 0x7fffffff;
     double h;
-    if (e < -1000 || e > 1000) {
-      h = sqrt(a2);
-    } else {
-      const int k = e >> 1;
-      const float mf = __int_as_float(((127 + e - 2 * k) << 23) | (int)((bits >> 29) & 0x7fffff));
-      const double y = widen_with_exp(rsqrtf(mf), -k, 0);
+    if (exp_in_range(hi)) {
+      const int t = hi - 0x3ff00000, k = t >> 21;  // a2 = m 4^k with m in [1, 4)
+      const float mf = lead_float(hi, (t >> 20) & 1);
+      const float yf = approx_rsqrt(mf);
+      const double y = widen_with_exp(yf, -k);
+      // the seed of 1 / (a2 + |alpha| h) from single precision too (|alpha| 2^-k
+      // and m^(1/2)), while the square root's correction is in the FP64 pipe
+      const int av = ahi - ((896 + k) << 20);
+      const float af = __int_as_float(av > 0 ? av << 3 : 0);
+      const double z = widen_with_exp(approx_rcp(fmaf(af, mf * yf, mf)), -2 * k);
       const double g = a2 * y;
       const double r = fma(-g, y, 1.0);
       h = fma(g, r * fma(r, 0.375, 0.5), g);
+      const double s = fma(-fma(fabs(alpha), h, a2), z, 1.0);
+      kap = fma(z, fma(s, s, s), z);  // -1 / (u beta)
+    } else {
+      h = sqrt(a2);
+      kap = 1.0 / fma(fabs(alpha), h, a2);
     }
     // sign(0) = +, so alpha = -0 reflects like +0
-    const long long ab = __double_as_longlong(alpha);
-    const bool neg = ab < 0 && (ab << 1) != 0;
-    beta = neg ? h : __longlong_as_double(__double_as_longlong(h) ^ (1LL << 63));
+    const bool neg = __double2hiint(alpha) < 0 && !is_zero(alpha);
+    beta = neg ? h : __hiloint2double(__double2hiint(h) ^ 0x80000000, __double2loint(h));
     u = alpha - beta;
-    kap = rcp_nr(fma(fabs(alpha), h, a2));  // -1 / (u beta)
   }
   // new pivot entry; ws: the multiple of x taken off the row's tail
   __device__ __forceinline__ double row(double a, double dot, double& ws) const {

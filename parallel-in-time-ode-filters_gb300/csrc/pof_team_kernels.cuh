@@ -22,26 +22,53 @@ struct TeamBlock {
   static constexpr int threads = teams * TS;
 };
 
-// SoA element <-> team workspace slot
+// SoA element <-> team workspace slot.  A lane's fields are all requested
+// before the first is put into shared memory, so an element costs one trip to
+// L2 instead of one per field (7 at D = 8 with 32 lanes).
+template <typename T, int TS, int NF>
+struct LaneFields {
+  static constexpr int N = (NF + TS - 1) / TS;
+  T v[N];
+  __device__ __forceinline__ void load(const Team<TS>& tm, const T* base, int64_t n, int64_t e) {
+#pragma unroll
+    for (int u = 0; u < N; ++u) {
+      const int f = tm.r + u * TS;
+      if (NF % TS == 0 || f < NF) v[u] = base[f * n + e];
+    }
+  }
+  template <typename Put>
+  __device__ __forceinline__ void put(const Team<TS>& tm, Put&& put_field) const {
+#pragma unroll
+    for (int u = 0; u < N; ++u) {
+      const int f = tm.r + u * TS;
+      if (NF % TS == 0 || f < NF) put_field(f, v[u]);
+    }
+  }
+};
+
+template <typename T, int D>
+__device__ __forceinline__ void put_filt(int f, T v, T* A, T* b, T* U, T* eta, T* Z) {
+  using FL = FiltLayout<D>;
+  constexpr int L1 = Ld<D>::v;
+  if (f < FL::B)
+    A[(f / D) * L1 + f % D] = v;
+  else if (f < FL::U)
+    b[f - FL::B] = v;
+  else if (f < FL::ETA)
+    U[((f - FL::U) / D) * L1 + (f - FL::U) % D] = v;
+  else if (f < FL::Z)
+    eta[f - FL::ETA] = v;
+  else
+    Z[((f - FL::Z) / D) * L1 + (f - FL::Z) % D] = v;
+}
+
 template <typename T, int TS, int D>
 __device__ __forceinline__ void t_load_filt(const Team<TS>& tm, const T* base, int64_t n, int64_t e, T* A, T* b,
                                             T* U, T* eta, T* Z) {
   if (!POF_IN(e, n)) return;
-  using FL = FiltLayout<D>;
-  constexpr int L1 = Ld<D>::v;
-  for (int f = tm.r; f < FL::NF; f += TS) {
-    const T v = base[f * n + e];
-    if (f < FL::B)
-      A[(f / D) * L1 + f % D] = v;
-    else if (f < FL::U)
-      b[f - FL::B] = v;
-    else if (f < FL::ETA)
-      U[((f - FL::U) / D) * L1 + (f - FL::U) % D] = v;
-    else if (f < FL::Z)
-      eta[f - FL::ETA] = v;
-    else
-      Z[((f - FL::Z) / D) * L1 + (f - FL::Z) % D] = v;
-  }
+  LaneFields<T, TS, FiltLayout<D>::NF> x;
+  x.load(tm, base, n, e);
+  x.put(tm, [&](int f, T v) { put_filt<T, D>(f, v, A, b, U, eta, Z); });
 }
 
 template <typename T, int TS, int D>
@@ -67,17 +94,20 @@ __device__ __forceinline__ void t_store_filt(const Team<TS>& tm, T* base, int64_
 }
 
 // state (m, L) <-> slot
+template <typename T, int D>
+__device__ __forceinline__ void put_state(int f, T v, T* m, T* L) {
+  constexpr int L1 = Ld<D>::v;
+  if (f < D)
+    m[f] = v;
+  else
+    L[((f - D) / D) * L1 + (f - D) % D] = v;
+}
 template <typename T, int TS, int D>
 __device__ __forceinline__ void t_load_state(const Team<TS>& tm, const T* base, int64_t n, int64_t e, T* m, T* L) {
   if (!POF_IN(e, n)) return;
-  constexpr int L1 = Ld<D>::v;
-  for (int f = tm.r; f < D + D * D; f += TS) {
-    const T v = base[f * n + e];
-    if (f < D)
-      m[f] = v;
-    else
-      L[((f - D) / D) * L1 + (f - D) % D] = v;
-  }
+  LaneFields<T, TS, D + D * D> x;
+  x.load(tm, base, n, e);
+  x.put(tm, [&](int f, T v) { put_state<T, D>(f, v, m, L); });
 }
 template <typename T, int TS, int D>
 __device__ __forceinline__ void t_store_state(const Team<TS>& tm, T* base, int64_t n, int64_t e, const T* m,
@@ -98,21 +128,24 @@ __device__ __forceinline__ void t_load_state_plain(const Team<TS>& tm, const T* 
 }
 
 // smoother element (g, E, Dm) <-> slot
+template <typename T, int D>
+__device__ __forceinline__ void put_smo(int f, T v, T* g, T* E, T* Dm) {
+  using GL = SmoLayout<D>;
+  constexpr int L1 = Ld<D>::v;
+  if (f < GL::E)
+    g[f] = v;
+  else if (f < GL::DM)
+    E[((f - GL::E) / D) * L1 + (f - GL::E) % D] = v;
+  else
+    Dm[((f - GL::DM) / D) * L1 + (f - GL::DM) % D] = v;
+}
 template <typename T, int TS, int D>
 __device__ __forceinline__ void t_load_smo(const Team<TS>& tm, const T* base, int64_t n, int64_t e, T* g, T* E,
                                            T* Dm) {
   if (!POF_IN(e, n)) return;
-  using GL = SmoLayout<D>;
-  constexpr int L1 = Ld<D>::v;
-  for (int f = tm.r; f < GL::NG; f += TS) {
-    const T v = base[f * n + e];
-    if (f < GL::E)
-      g[f] = v;
-    else if (f < GL::DM)
-      E[((f - GL::E) / D) * L1 + (f - GL::E) % D] = v;
-    else
-      Dm[((f - GL::DM) / D) * L1 + (f - GL::DM) % D] = v;
-  }
+  LaneFields<T, TS, SmoLayout<D>::NG> x;
+  x.load(tm, base, n, e);
+  x.put(tm, [&](int f, T v) { put_smo<T, D>(f, v, g, E, Dm); });
 }
 template <typename T, int TS, int D>
 __device__ __forceinline__ void t_store_smo(const Team<TS>& tm, T* base, int64_t n, int64_t e, const T* g,
@@ -148,9 +181,12 @@ __global__ void k_filt_reduce_team(const T* __restrict__ in, int64_t nin, int C,
   if (t >= nout) return;
   const int64_t i0 = t * C;
   const int64_t i1 = (i0 + C < nin) ? i0 + C : nin;
+  LaneFields<T, TS, FiltLayout<D>::NF> nx;  // the next element, on its way while the one before is put
+  if (i0 + 1 < i1) nx.load(tm, in, nin, i0 + 1);
   t_load_filt<T, TS, D>(tm, in, nin, i0, w.A1, w.b1, w.U1, w.e1, w.Z1);
   for (int64_t i = i0 + 1; i < i1; ++i) {
-    t_load_filt<T, TS, D>(tm, in, nin, i, w.A2, w.b2, w.U2, w.e2, w.Z2);
+    nx.put(tm, [&](int f, T v) { put_filt<T, D>(f, v, w.A2, w.b2, w.U2, w.e2, w.Z2); });
+    if (i + 1 < i1) nx.load(tm, in, nin, i + 1);
     tm.sync();
     t_filt_combine<T, TS, D>(tm, w);
   }
@@ -182,12 +218,26 @@ __global__ void k_filt_down_team(const T* __restrict__ elems, int64_t n, int C, 
   if (t >= nup) return;
   const int64_t i0 = t * C;
   const int64_t i1 = (i0 + C < n) ? i0 + C : n;
+  LaneFields<T, TS, FiltLayout<D>::NF> nx;  // the next element, requested together with the state
+  if (i0 + 1 < i1) nx.load(tm, elems, n, i0);
   t_load_state<T, TS, D>(tm, states_up, nup, t, w.b1, w.U1);
   tm.sync();
   for (int64_t i = i0; i < i1; ++i) {
     t_store_state<T, TS, D>(tm, states, n, i, w.b1, w.U1);
     tm.sync();
-    if (i + 1 < i1) t_filt_advance<T, D, TS>(tm, w, elems, n, i);
+    if (i + 1 < i1) {
+      if (i == 0) {  // absolute: the state after it is its own (b, U)
+        nx.put(tm, [&](int f, T v) { put_filt<T, D>(f, v, w.M, w.b1, w.U1, w.v1, w.M); });
+        tm.sync();
+      } else {
+        nx.put(tm, [&](int f, T v) { put_filt<T, D>(f, v, w.A2, w.b2, w.U2, w.e2, w.Z2); });
+        if (i + 2 < i1) nx.load(tm, elems, n, i + 1);
+        tm.sync();
+        t_filt_apply<T, TS, D>(tm, w);
+        continue;
+      }
+      if (i + 2 < i1) nx.load(tm, elems, n, i + 1);
+    }
   }
 }
 
@@ -214,9 +264,12 @@ __global__ void k_smo_reduce_team(const T* __restrict__ in, int64_t nin, int C, 
   if (t >= nout) return;
   const int64_t i0 = t * C;
   const int64_t i1 = (i0 + C < nin) ? i0 + C : nin;
+  LaneFields<T, TS, SmoLayout<D>::NG> nx;
+  if (i0 + 1 < i1) nx.load(tm, in, nin, i0 + 1);
   t_load_smo<T, TS, D>(tm, in, nin, i0, w.g2, w.E2, w.D2m);
   for (int64_t i = i0 + 1; i < i1; ++i) {
-    t_load_smo<T, TS, D>(tm, in, nin, i, w.g1, w.E1, w.D1);
+    nx.put(tm, [&](int f, T v) { put_smo<T, D>(f, v, w.g1, w.E1, w.D1); });
+    if (i + 1 < i1) nx.load(tm, in, nin, i + 1);
     tm.sync();
     t_smooth_combine<T, TS, D>(tm, w);
   }
@@ -232,12 +285,15 @@ __global__ void k_smo_down_team(const T* __restrict__ elems, int64_t n, int C, c
   if (t >= nup) return;
   const int64_t i0 = t * C;
   const int64_t i1 = (i0 + C < n) ? i0 + C : n;
+  LaneFields<T, TS, SmoLayout<D>::NG> nx;
+  if (i1 - 1 > i0) nx.load(tm, elems, n, i1 - 1);
   t_load_state<T, TS, D>(tm, ends_up, nup, t, w.g1, w.D1);
   tm.sync();
   for (int64_t i = i1 - 1; i >= i0; --i) {
     t_store_state<T, TS, D>(tm, ends, n, i, w.g1, w.D1);
     if (i > i0) {
-      t_load_smo<T, TS, D>(tm, elems, n, i, w.g2, w.E2, w.D2m);
+      nx.put(tm, [&](int f, T v) { put_smo<T, D>(f, v, w.g2, w.E2, w.D2m); });
+      if (i - 1 > i0) nx.load(tm, elems, n, i - 1);
       tm.sync();
       t_smooth_apply<T, TS, D>(tm, w);
     }
