@@ -154,7 +154,7 @@ __global__ void kb_filt_top(BView v, const T* __restrict__ x0m, const T* __restr
   if (v.frozen[b]) return;
   for (int f = tm.r; f < D + D * D; f += TS) {
     const T val = (f < D) ? x0m[(int64_t)b * D + f] : x0L[(int64_t)b * D * D + f - D];
-    states[f * v.Ba + t] = val;
+    states[element_index<D, D + D * D>(f, t, v.Ba)] = val;
   }
 }
 
@@ -290,7 +290,7 @@ __global__ void kb_smo_top(BView v, const T* __restrict__ means, const T* __rest
   const int64_t g = v.gb[b] + v.ns[b];
   for (int f = tm.r; f < D + D * D; f += TS) {
     const T val = (f < D) ? means[g * D + f] : chols[g * D * D + f - D];
-    ends[f * v.Ba + t] = val;
+    ends[element_index<D, D + D * D>(f, t, v.Ba)] = val;
   }
 }
 

@@ -6,9 +6,14 @@
 // These level-0 kernels assign one thread to one chunk (small D); the team
 // kernels (pof_team_kernels.cuh) take larger D and every level above.
 //
-// Internal buffers are structure-of-arrays: field f of element e of a level
-// with n elements lives at base[f * n + e], so a warp touching 32
-// consecutive elements issues one coalesced access per field.
+// Internal buffers of the small shapes (D < 6, one thread per chunk) are
+// structure-of-arrays: field f of element e of a level with n elements lives
+// at base[f * n + e], so a warp touching 32 consecutive elements issues one
+// coalesced access per field.  From D = 6 on a team works on one element, and
+// an element's fields are contiguous (base[e * fields + f]): a team then reads
+// whole lines, where a field of its own per 32-byte sector cost four times the
+// L2 traffic (the sectors' other elements are read steps later, and shared
+// memory leaves L1 too small to keep them).  element_index is the rule.
 //
 // Caller-facing arrays (x0, F, QL, H, c, R, means, chols) keep the
 // reference's row-major layouts: H (n, DY, D), c (n, DY), means (n+1, D),
@@ -47,6 +52,11 @@ struct StateLayout {
   static constexpr int M = 0, L = D;
   static constexpr int NS = D + D * D;
 };
+
+template <int D, int FIELDS>
+__host__ __device__ __forceinline__ int64_t element_index(int f, int64_t e, int64_t n) {
+  return D >= 6 ? e * FIELDS + f : f * n + e;
+}
 
 // per-chunk partial sums (double accumulators for every T)
 enum Partial : int { P_SSQ = 0, P_NLL = 1, P_FOBJ = 2, P_SOBJ = 3, P_NOTCLOSE = 4, P_COUNT = 5 };

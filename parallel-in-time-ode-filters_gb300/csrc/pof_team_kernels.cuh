@@ -22,10 +22,10 @@ struct TeamBlock {
   static constexpr int threads = teams * TS;
 };
 
-// SoA element <-> team workspace slot.  A lane's fields are all requested
+// Stored element <-> team workspace slot.  A lane's fields are all requested
 // before the first is put into shared memory, so an element costs one trip to
 // L2 instead of one per field (7 at D = 8 with 32 lanes).
-template <typename T, int TS, int NF>
+template <typename T, int TS, int D, int NF>
 struct LaneFields {
   static constexpr int N = (NF + TS - 1) / TS;
   T v[N];
@@ -33,7 +33,7 @@ struct LaneFields {
 #pragma unroll
     for (int u = 0; u < N; ++u) {
       const int f = tm.r + u * TS;
-      if (NF % TS == 0 || f < NF) v[u] = base[f * n + e];
+      if (NF % TS == 0 || f < NF) v[u] = base[element_index<D, NF>(f, e, n)];
     }
   }
   template <typename Put>
@@ -66,7 +66,7 @@ template <typename T, int TS, int D>
 __device__ __forceinline__ void t_load_filt(const Team<TS>& tm, const T* base, int64_t n, int64_t e, T* A, T* b,
                                             T* U, T* eta, T* Z) {
   if (!POF_IN(e, n)) return;
-  LaneFields<T, TS, FiltLayout<D>::NF> x;
+  LaneFields<T, TS, D, FiltLayout<D>::NF> x;
   x.load(tm, base, n, e);
   x.put(tm, [&](int f, T v) { put_filt<T, D>(f, v, A, b, U, eta, Z); });
 }
@@ -89,7 +89,7 @@ __device__ __forceinline__ void t_store_filt(const Team<TS>& tm, T* base, int64_
       v = eta[f - FL::ETA];
     else
       v = Z[((f - FL::Z) / D) * L1 + (f - FL::Z) % D];
-    base[f * n + e] = v;
+    base[element_index<D, FL::NF>(f, e, n)] = v;
   }
 }
 
@@ -105,7 +105,7 @@ __device__ __forceinline__ void put_state(int f, T v, T* m, T* L) {
 template <typename T, int TS, int D>
 __device__ __forceinline__ void t_load_state(const Team<TS>& tm, const T* base, int64_t n, int64_t e, T* m, T* L) {
   if (!POF_IN(e, n)) return;
-  LaneFields<T, TS, D + D * D> x;
+  LaneFields<T, TS, D, D + D * D> x;
   x.load(tm, base, n, e);
   x.put(tm, [&](int f, T v) { put_state<T, D>(f, v, m, L); });
 }
@@ -114,7 +114,8 @@ __device__ __forceinline__ void t_store_state(const Team<TS>& tm, T* base, int64
                                               const T* L) {
   if (!POF_IN(e, n)) return;
   constexpr int L1 = Ld<D>::v;
-  for (int f = tm.r; f < D + D * D; f += TS) base[f * n + e] = (f < D) ? m[f] : L[((f - D) / D) * L1 + (f - D) % D];
+  for (int f = tm.r; f < D + D * D; f += TS)
+    base[element_index<D, D + D * D>(f, e, n)] = (f < D) ? m[f] : L[((f - D) / D) * L1 + (f - D) % D];
 }
 template <typename T, int TS, int D>
 __device__ __forceinline__ void t_load_state_plain(const Team<TS>& tm, const T* m0, const T* L0, T* m, T* L) {
@@ -143,7 +144,7 @@ template <typename T, int TS, int D>
 __device__ __forceinline__ void t_load_smo(const Team<TS>& tm, const T* base, int64_t n, int64_t e, T* g, T* E,
                                            T* Dm) {
   if (!POF_IN(e, n)) return;
-  LaneFields<T, TS, SmoLayout<D>::NG> x;
+  LaneFields<T, TS, D, SmoLayout<D>::NG> x;
   x.load(tm, base, n, e);
   x.put(tm, [&](int f, T v) { put_smo<T, D>(f, v, g, E, Dm); });
 }
@@ -161,7 +162,7 @@ __device__ __forceinline__ void t_store_smo(const Team<TS>& tm, T* base, int64_t
       v = E[((f - GL::E) / D) * L1 + (f - GL::E) % D];
     else
       v = Dm[((f - GL::DM) / D) * L1 + (f - GL::DM) % D];
-    base[f * n + e] = v;
+    base[element_index<D, GL::NG>(f, e, n)] = v;
   }
 }
 
@@ -181,7 +182,7 @@ __global__ void k_filt_reduce_team(const T* __restrict__ in, int64_t nin, int C,
   if (t >= nout) return;
   const int64_t i0 = t * C;
   const int64_t i1 = (i0 + C < nin) ? i0 + C : nin;
-  LaneFields<T, TS, FiltLayout<D>::NF> nx;  // the next element, on its way while the one before is put
+  LaneFields<T, TS, D, FiltLayout<D>::NF> nx;  // the next element, on its way while the one before is put
   if (i0 + 1 < i1) nx.load(tm, in, nin, i0 + 1);
   t_load_filt<T, TS, D>(tm, in, nin, i0, w.A1, w.b1, w.U1, w.e1, w.Z1);
   for (int64_t i = i0 + 1; i < i1; ++i) {
@@ -218,7 +219,7 @@ __global__ void k_filt_down_team(const T* __restrict__ elems, int64_t n, int C, 
   if (t >= nup) return;
   const int64_t i0 = t * C;
   const int64_t i1 = (i0 + C < n) ? i0 + C : n;
-  LaneFields<T, TS, FiltLayout<D>::NF> nx;  // the next element, requested together with the state
+  LaneFields<T, TS, D, FiltLayout<D>::NF> nx;  // the next element, requested together with the state
   if (i0 + 1 < i1) nx.load(tm, elems, n, i0);
   t_load_state<T, TS, D>(tm, states_up, nup, t, w.b1, w.U1);
   tm.sync();
@@ -264,7 +265,7 @@ __global__ void k_smo_reduce_team(const T* __restrict__ in, int64_t nin, int C, 
   if (t >= nout) return;
   const int64_t i0 = t * C;
   const int64_t i1 = (i0 + C < nin) ? i0 + C : nin;
-  LaneFields<T, TS, SmoLayout<D>::NG> nx;
+  LaneFields<T, TS, D, SmoLayout<D>::NG> nx;
   if (i0 + 1 < i1) nx.load(tm, in, nin, i0 + 1);
   t_load_smo<T, TS, D>(tm, in, nin, i0, w.g2, w.E2, w.D2m);
   for (int64_t i = i0 + 1; i < i1; ++i) {
@@ -285,7 +286,7 @@ __global__ void k_smo_down_team(const T* __restrict__ elems, int64_t n, int C, c
   if (t >= nup) return;
   const int64_t i0 = t * C;
   const int64_t i1 = (i0 + C < n) ? i0 + C : n;
-  LaneFields<T, TS, SmoLayout<D>::NG> nx;
+  LaneFields<T, TS, D, SmoLayout<D>::NG> nx;
   if (i1 - 1 > i0) nx.load(tm, elems, n, i1 - 1);
   t_load_state<T, TS, D>(tm, ends_up, nup, t, w.g1, w.D1);
   tm.sync();
@@ -587,7 +588,7 @@ __device__ __forceinline__ void fq_step(const Team<TS>& tm, FQ<T, D>& q, const S
   }
 }
 
-// the fold's element (columns of A and eta in lane registers) to SoA
+// the fold's element (columns of A and eta in lane registers) to its slot
 template <typename T, int TS, int D, int DY>
 __device__ __forceinline__ void t_store_fold(const Team<TS>& tm, T* base, int64_t n, int64_t e,
                                              const StepFoldWs<T, D, DY>& w, const FoldRegs<T, D>& fr) {
@@ -596,14 +597,14 @@ __device__ __forceinline__ void t_store_fold(const Team<TS>& tm, T* base, int64_
   constexpr int L1 = Ld<D>::v, LZ = StepDims<T, D, DY>::LDZ;
   if (tm.r < D) {
 #pragma unroll
-    for (int i = 0; i < D; ++i) base[(FL::A + i * D + tm.r) * n + e] = fr.a[i];
-    base[(FL::B + tm.r) * n + e] = w.m[tm.r];
-    base[(FL::ETA + tm.r) * n + e] = fr.eta;
+    for (int i = 0; i < D; ++i) base[element_index<D, FL::NF>(FL::A + i * D + tm.r, e, n)] = fr.a[i];
+    base[element_index<D, FL::NF>(FL::B + tm.r, e, n)] = w.m[tm.r];
+    base[element_index<D, FL::NF>(FL::ETA + tm.r, e, n)] = fr.eta;
   }
   for (int f = tm.r; f < D * D; f += TS) {
     const int i = f / D, j = f % D;
-    base[(FL::U + f) * n + e] = w.L[i * L1 + j];
-    base[(FL::Z + f) * n + e] = w.ZX[i * LZ + j];
+    base[element_index<D, FL::NF>(FL::U + f, e, n)] = w.L[i * L1 + j];
+    base[element_index<D, FL::NF>(FL::Z + f, e, n)] = w.ZX[i * LZ + j];
   }
 }
 
@@ -670,17 +671,17 @@ __global__ void k_filt_l0_reduce_team(int64_t n, int C0, StepModel sm, const T* 
   t_store_fold<T, TS, D, DY>(tm, out, n1, t, w, fr);
 }
 
-// Smoother element of a step, t_kf_step's g, E and raw factor, to SoA.
+// Smoother element of a step, t_kf_step's g, E and raw factor, to its slot.
 template <typename T, int TS, int D, int DY>
 __device__ __forceinline__ void t_store_selem(const Team<TS>& tm, T* base, int64_t n, int64_t s,
                                               const StepKFWs<T, D, DY>& w, int nl) {
   using GL = SmoLayout<D>;
   constexpr int L1 = Ld<D>::v, L2 = Ld<2 * D>::v;
-  for (int f = tm.r; f < D; f += TS) base[f * n + s] = w.g[f];
+  for (int f = tm.r; f < D; f += TS) base[element_index<D, GL::NG>(f, s, n)] = w.g[f];
   for (int f = tm.r; f < D * D; f += TS) {
     const int i = f / D, j = f % D;
-    base[(GL::E + f) * n + s] = w.E[i * L1 + j];
-    base[(GL::DM + f) * n + s] = j < nl ? w.Y[i * L2 + D + j] : T(0);
+    base[element_index<D, GL::NG>(GL::E + f, s, n)] = w.E[i * L1 + j];
+    base[element_index<D, GL::NG>(GL::DM + f, s, n)] = j < nl ? w.Y[i * L2 + D + j] : T(0);
   }
 }
 
