@@ -177,6 +177,12 @@ int pof_dense_linear_filtsmooth(int32_t which, int32_t dtype, int64_t n_steps, i
                                 void* out_mean, void* out_chol, double* out_scalars, int32_t chunks, void* workspace,
                                 size_t workspace_bytes, void* stream);
 
+/* Taylor-mode initial values of a built-in field (pof/initialization.py:15-22):
+ * the derivatives y^(0..q) at the initial value of y' = f(y), y = y0, into
+ * out (q + 1, d).  params, y0 and out are HOST arrays of doubles (the field's
+ * parameters, d, (q + 1) d); no CUDA call.  q <= 64. */
+int pof_taylor(int32_t field, int32_t d, int32_t q, const double* params, const double* y0, double* out);
+
 /* EK1 linearization of a built-in field at means[1:]
  *   (pof/step.py:12-22, pof/observations.py:35-40) with the Nordsieck-scaled
  * projections of pof/convenience.py:24-28 (step size h): writes

@@ -60,6 +60,7 @@ _SIGS = {
     "pof_shape_supported": (_c.c_int, [_i32, _i32]),
     "pof_filtsmooth_workspace_bytes": (_sz, [_i32, _i64, _i32, _i32]),
     "pof_ieks_workspace_bytes": (_sz, [_i32, _i64, _i32, _i32]),
+    "pof_taylor": (_c.c_int, [_i32, _i32, _i32, _vp, _vp, _vp]),
     "pof_linear_filtsmooth": (
         _c.c_int,
         [_i32, _i64, _i32, _i32, _vp, _vp, _vp, _vp, _i64, _vp, _vp, _vp, _i64, _vp, _vp, _dp, _vp, _sz, _vp],

@@ -1,5 +1,6 @@
 """Solver set-up (pof/convenience.py)."""
 
+import numpy as np
 import torch
 
 from . import initialization as init
@@ -7,9 +8,9 @@ from .observations import NonlinearModel, linearize
 from .transitions import (
     IWP,
     TransitionModel,
+    _nordsieck_1d_np,
+    _preconditioned_1d_np,
     get_transition_model,
-    nordsieck_preconditioner,
-    preconditioned_discretize,
     projection_matrix,
 )
 from .utils import MVNSqrt, default_device, gmul_stack
@@ -24,24 +25,40 @@ def _ts(ts):
     return torch.as_tensor(ts, dtype=torch.float64).to(default_device())
 
 
+def _to_device(arrays, dev):
+    """Small host matrices on the device with one copy, each 256-byte aligned."""
+    sizes = [-(-a.size // 32) * 32 for a in arrays]
+    flat = np.zeros(sum(sizes))
+    at = np.concatenate([[0], np.cumsum(sizes)])
+    for a, o in zip(arrays, at):
+        flat[o:o + a.size] = a.reshape(-1)
+    buf = torch.from_numpy(flat).to(dev)
+    return [buf[o:o + a.size].view(a.shape) for a, o in zip(arrays, at)]
+
+
 def set_up_solver(*, f, y0, ts, order):
     """pof/convenience.py:13-45: preconditioned IWP prior, Nordsieck P/PI,
     projections E0 P and E1 P, the residual model E1 x - f(E0 x) and the
     Taylor-mode x0 (times PI).  The N-1 identical transition models are
     exposed as a stride-0 expand of one (D, D) pair."""
-    ts = _ts(ts)
-    dts = ts[1:] - ts[:-1]
-    dt = float(dts[0])  # uniform grid assumed, as in the reference (its check is commented out)
+    ts = torch.as_tensor(ts, dtype=torch.float64)
+    dt = float(ts[1] - ts[0])  # uniform grid assumed, as in the reference (its check is commented out)
+    dev = default_device()
+    ts = ts.to(dev)
     y0 = torch.as_tensor(y0, dtype=torch.float64)
     d = y0.shape[0]
     n = ts.shape[0] - 1
     iwp = IWP(num_derivatives=order, wiener_process_dimension=d)
-    A, QL = preconditioned_discretize(iwp)
+    x0 = init.taylor_mode_init(f, y0, order, device=torch.device("cpu"))
+    # the set-up matrices are small: formed on the host, one copy to the device
+    A1, QL1 = _preconditioned_1d_np(order)
+    P1, PI1 = _nordsieck_1d_np(order, dt)
+    I = np.eye(d)
+    A, QL, P, PI = (np.kron(I, x) for x in (A1, QL1, P1, PI1))
+    E0, E1 = (np.kron(I, np.eye(1, order + 1, k)) @ P for k in (0, 1))
+    A, QL, P, PI, E0, E1, m0, L0 = _to_device([A, QL, P, PI, E0, E1, PI @ x0.mean.numpy(), PI @ x0.chol.numpy()], dev)
     D = A.shape[0]
     dtm = TransitionModel(A.expand(n, D, D), QL.expand(n, D, D))
-    P, PI = nordsieck_preconditioner(iwp, dt)
-    E0, E1 = projection_matrix(iwp, 0), projection_matrix(iwp, 1)
-    E0, E1 = E0 @ P, E1 @ P
 
     def om_fn(x, f=f, E0=E0, E1=E1):
         return E1 @ x - f(None, E0 @ x)
@@ -60,10 +77,8 @@ def set_up_solver(*, f, y0, ts, order):
         "iwp": iwp,
     }
     om = NonlinearModel(om_fn, field=getattr(f, "pof_field", None), setup=setup)
-    x0 = init.taylor_mode_init(f, y0, order)
-    x0 = MVNSqrt(PI @ x0.mean, PI @ x0.chol)
     setup["om"] = om
-    setup["x0"] = x0
+    setup["x0"] = MVNSqrt(m0, L0)
     return setup
 
 
@@ -97,8 +112,10 @@ def get_initial_trajectory(setup, method="prior"):
         states = init.coarse_ekf_init(y0=y0, order=order, ts=ts, f=f, N=100)
         return gmul_stack(PI, states)
     elif method == "constant":
-        states = init.constant_init(y0=y0, order=order, ts=ts, f=f)
-        return gmul_stack(PI, states)
+        # one row, repeated (PI times a zero chol is zero)
+        row = init.constant_init(y0=y0, order=order, ts=ts[:1], f=f, device=ts.device)
+        N, D = ts.shape[0], row.mean.shape[1]
+        return MVNSqrt((row.mean @ PI.T).repeat(N, 1), torch.zeros((N, D, D), dtype=torch.float64, device=ts.device))
     elif method == "prior":
         return init.prior_init(f=f, y0=y0, order=order, ts=ts)
     else:

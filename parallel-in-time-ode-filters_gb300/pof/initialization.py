@@ -2,16 +2,19 @@
 (pof/initialization.py).
 
 Taylor-mode initialisation: the reference calls tornadox's TaylorMode
-(``jax.experimental.jet``); here the derivatives come from nested
-``torch.func.jvp``: with y_k(t) = sum_{j<k} y^(j) t^j / j!, the k-th
+(``jax.experimental.jet``); here the derivatives of a built-in field come from
+libpof's power series on the host (``pof_taylor``), those of a user field from
+nested ``torch.func.jvp``: with y_k(t) = sum_{j<k} y^(j) t^j / j!, the k-th
 derivative of the solution at t0 is the (k-1)-th time derivative of
 f(y_k(t)) at t0, which only involves y^(0..k-1).
 """
 
 import math
 
+import numpy as np
 import torch
 
+from . import _lib
 from .sequential_filtsmooth.filter import _sqrt_predict
 from .transitions import IWP, discretize_transitions
 from .utils import FORWARD_AD_LOCK, MVNSqrt, default_device
@@ -31,6 +34,16 @@ def _nth_time_derivative(g, n):
 def taylor_derivatives(f, y0, num_derivatives):
     """(q+1, d) array of y^(k)(t0), k = 0..q, for y' = f(t, y) (time-independent f)."""
     y0 = torch.as_tensor(y0, dtype=torch.float64).detach().cpu()
+    field = getattr(f, "pof_field", None)
+    if field is not None and num_derivatives <= 64:
+        name, params = field
+        y = np.ascontiguousarray(y0.numpy())
+        p = np.array(params if params else (0.0,), dtype=np.float64)
+        out = np.empty((num_derivatives + 1, y.shape[0]))
+        rc = _lib.lib().pof_taylor(_lib.FIELDS[name], y.shape[0], num_derivatives, p.ctypes.data, y.ctypes.data,
+                                   out.ctypes.data)
+        _lib.check(rc, "pof_taylor")
+        return torch.from_numpy(out)
     derivs = [y0]
     for k in range(1, num_derivatives + 1):
         coeffs = [dj / math.factorial(j) for j, dj in enumerate(derivs)]
@@ -48,8 +61,11 @@ def taylor_derivatives(f, y0, num_derivatives):
 def taylor_mode_init(f, y0, num_derivatives, device=None):
     """x0 = (y0, y0', ..., y0^(q)) per dimension, chol = 0 (pof/initialization.py:15-22)."""
     d = torch.as_tensor(y0).shape[0]
-    with FORWARD_AD_LOCK:
+    if getattr(f, "pof_field", None) is not None:
         derivs = taylor_derivatives(f, y0, num_derivatives)  # (q+1, d)
+    else:
+        with FORWARD_AD_LOCK:
+            derivs = taylor_derivatives(f, y0, num_derivatives)
     m0 = derivs.T.reshape(-1)
     D = d * (num_derivatives + 1)
     dev = device or default_device()

@@ -41,9 +41,10 @@ def pascal(n):
 
 
 def _preconditioned_1d_np(q):
-    A = np.flip(pascal(q + 1))
-    Q = np.flip(hilbert(q + 1))
-    return np.ascontiguousarray(A), np.linalg.cholesky(np.ascontiguousarray(Q))
+    # flip(lower Pascal), flip(Hilbert): the entries of scipy.linalg.pascal / hilbert, without their host time
+    A = np.array([[math.comb(q - i, q - j) if j >= i else 0 for j in range(q + 1)] for i in range(q + 1)], dtype=float)
+    k = np.arange(q, -1, -1, dtype=float)
+    return A, np.linalg.cholesky(1.0 / (k[:, None] + k + 1.0))
 
 
 def preconditioned_discretize_1d(iwp: IWP, device=None):
