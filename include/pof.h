@@ -194,7 +194,7 @@ int pof_linearize(int32_t dtype, int64_t n_steps, int32_t D, int32_t d, int32_t 
 /* pof.sequential_filtsmooth.linear_filtsmooth(x0, dtm, dom)
  *   (pof/sequential_filtsmooth/__init__.py:13-16): the square-root Kalman
  * filter (filter.py:33-56) and RTS smoother (smoother.py:8-28) step after
- * step on one GPU thread -- the reference's sequential twin.  Writes the
+ * step in one thread block -- the reference's sequential twin.  Writes the
  * smoothed states (the filtered ones when smooth == 0) and
  * out_scalars[POF_S_NLL] = +sum log-likelihood (the sequential twin's sign,
  * filter.py:23-30), [POF_S_OBJ] (0 when smooth == 0), [POF_S_SSQ].

@@ -54,9 +54,10 @@ struct OpsImpl {
                          const void* x0m, const void* x0L, int smooth, void* means, void* chols, double* scalars,
                          cudaStream_t st) {
     ProfScope ps(PK_SEQUENTIAL, st);
-    k_seq_filtsmooth<T, D, DY><<<1, 32, 0, st>>>(n, sm, field, static_cast<const T*>(params), (T)p0, (T)p1,
-                                                 static_cast<const T*>(x0m), static_cast<const T*>(x0L), smooth,
-                                                 static_cast<T*>(means), static_cast<T*>(chols), scalars);
+    static_assert(sizeof(SeqWs<T, D, DY>) <= 48 * 1024, "the default limit of dynamic shared memory");
+    k_seq_filtsmooth<T, D, DY><<<1, 64, sizeof(SeqWs<T, D, DY>), st>>>(
+        n, sm, field, static_cast<const T*>(params), (T)p0, (T)p1, static_cast<const T*>(x0m),
+        static_cast<const T*>(x0L), smooth, static_cast<T*>(means), static_cast<T*>(chols), scalars);
   }
   static const Ops* get() {
     static const Ops ops{&filter, &smoother, &smo_elements, &linearize, &scale_inplace, &sequential};

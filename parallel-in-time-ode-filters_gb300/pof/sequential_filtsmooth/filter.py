@@ -1,7 +1,7 @@
 """Sequential square-root filter (pof/sequential_filtsmooth/filter.py).
 
 ``extended_kalman_filter`` / ``linear_noiseless_filter`` run whole
-trajectories in libpof on one GPU thread (built-in vector fields are
+trajectories in libpof in one thread block (built-in vector fields are
 linearized inside the kernel); the EKF of any other torch vector field runs
 step after step in torch (each step's linearization needs the previous
 step's prediction).  ``_sqrt_predict`` and ``_sqrt_update`` are the one-step

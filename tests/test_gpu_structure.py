@@ -13,7 +13,7 @@ import pytest
 import torch
 
 from oracle import core, filtsmooth as ofs
-from pof import parallel_filtsmooth as pfs
+from pof import parallel_filtsmooth as pfs, sequential_filtsmooth as sfs
 from pof.observations import AffineModel
 from pof.transitions import TransitionModel
 from pof.utils import MVNSqrt
@@ -87,3 +87,28 @@ def test_level0_structure(D, d, prior, noise, full_h, x0, n):
         turn = np.linalg.qr(np.random.default_rng(n).standard_normal((D, D)))[0]
         sm, _ = pfs.smoothing(gdtm, MVNSqrt(filt.mean, filt.chol @ T(turn)))
         assert rel(N_(sm.mean), om) <= tol_m and rel(cov(N_(sm.chol)), cov(oL)) <= tol_c
+
+
+@pytest.mark.parametrize("D,d", SHAPES + [(3, 4)])
+@pytest.mark.parametrize("prior,noise,x0,n", [(True, "none", "point", 12), (True, "some", "full", 5),
+                                              (False, "all", "full", 1), (True, "all", "point", 2)])
+def test_sequential_twin_structure(D, d, prior, noise, x0, n):
+    """The sequential twin (one block, the same step operations) on the same
+    models, filtered and smoothed, within the bound of the test above."""
+    if d > D:  # more rows than states: noise on all of them
+        prior, noise = False, "all"
+    st, (F, QL), dom = model(D, d, n, prior, noise, False, x0, 7 * D + d + n)
+    rep = lambda A: np.broadcast_to(A, (n, D, D)).copy()  # noqa: E731
+    dtm = (rep(F), rep(QL))
+    (om, oL), oell, oobj, _ = ofs.sequential_linear_filtsmooth(st, dtm, dom)
+    (pm, pL), pnll, pobj, _ = ofs.linear_filtsmooth(st, dtm, dom)
+    tol_m = max(TOL, 10 * rel(pm, om))
+    tol_c = max(TOL, 10 * rel(cov(pL), cov(oL)))
+    gx0 = MVNSqrt(T(st[0]), T(st[1]))
+    gdom = AffineModel(T(dom[0]), T(dom[1]), None if noise == "none" else T(dom[2]))
+    shared = TransitionModel(T(F).expand(n, D, D), T(QL).expand(n, D, D))
+    for gdtm in (shared, TransitionModel(T(dtm[0]), T(dtm[1]))):
+        out, ell, obj, _ = sfs.linear_filtsmooth(gx0, gdtm, gdom)
+        assert rel(N_(out.mean), om) <= tol_m and rel(cov(N_(out.chol)), cov(oL)) <= tol_c
+        assert abs(float(ell) - oell) <= max(TOL * abs(oell), 10 * abs(oell + pnll))
+        assert abs(float(obj) - oobj) <= max(TOL * abs(oobj), 10 * abs(oobj - pobj))
