@@ -97,7 +97,7 @@ def test_sequential_twin_structure(D, d, prior, noise, x0, n):
     models, filtered and smoothed, within the bound of the test above."""
     if d > D:  # more rows than states: noise on all of them
         prior, noise = False, "all"
-    st, (F, QL), dom = model(D, d, n, prior, noise, False, x0, 7 * D + d + n)
+    st, (F, QL), dom = model(D, d, n, prior, noise, d > D, x0, 7 * D + d + n)
     rep = lambda A: np.broadcast_to(A, (n, D, D)).copy()  # noqa: E731
     dtm = (rep(F), rep(QL))
     (om, oL), oell, oobj, _ = ofs.sequential_linear_filtsmooth(st, dtm, dom)
