@@ -42,6 +42,7 @@ namespace dense {
 namespace {
 
 constexpr int64_t kMaxGridYZ = 65535;
+constexpr int64_t kSMs = 152;
 constexpr size_t kPanelSmem = 200 * 1024;
 
 int panel_rows(int n, size_t es) {
@@ -64,6 +65,36 @@ constexpr int64_t kClusterMaxBatch = 32;
 // ---------------------------------------------------------------------------
 // launches
 // ---------------------------------------------------------------------------
+// Register panels (k_lq_panel): 16 rows in double (4 warps of 4 rows: a
+// panel's FP64 work grows with its rows squared and runs on one SM), 32 in
+// float (8 warps of 4), up to kRegCols columns.
+template <typename T>
+struct RegPanel;
+template <>
+struct RegPanel<double> {
+  static constexpr int NW = 4, RPW = 4, cols = 768;
+};
+template <>
+struct RegPanel<float> {
+  static constexpr int NW = 8, RPW = 4, cols = 1280;
+};
+
+template <typename T, int NC>
+void launch_lq_panel(int64_t batch, cudaStream_t st, MV<T> W, int i0, int nbb, int np, T* V, T* TT, T* TV,
+                     int64_t vbs, int64_t tbs) {
+  using R = RegPanel<T>;
+  if constexpr (NC * 32 <= R::cols)
+    k_lq_panel<T, R::NW, R::RPW, NC><<<(unsigned)batch, R::NW * 32, 0, st>>>(W, i0, nbb, np, V, TT, TV, vbs, tbs);
+}
+
+// Row blocks of k_wy_apply: their rows and the panel's V fit 200 KB.  double
+// always takes it; float, whose two GEMMs run on the tensor cores, while the
+// row blocks are few (the tree levels above the chunks, where a launch costs
+// its latency).
+constexpr int kWyRows = 16;
+constexpr int64_t kWyMaxBlocksF32 = 4 * kSMs;
+inline size_t wy_smem(int nb, int np, size_t es) { return size_t(kWyRows + nb) * (np | 1) * es; }
+
 template <typename T>
 struct Ctx {
   cudaStream_t st;
@@ -82,14 +113,22 @@ struct Ctx {
     }
     for (int64_t b0 = 0; b0 < batch; b0 += kMaxGridYZ) {
       const int nb = (int)std::min<int64_t>(kMaxGridYZ, batch - b0);
-      if (N <= 16) {
+      if (N == 1) {
+        k_gemv<T><<<dim3(cdiv(M, A.cs == 1 ? 4 : 32), nb), 128, 0, st>>>(M, K, alpha, A, B, beta, C, b0);
+      } else if (N <= 16) {
         k_gemm<T, 128, 16, 16, 4, 2><<<dim3(cdiv(N, 16), cdiv(M, 128), nb), 256, 0, st>>>(M, N, K, alpha, A, B,
                                                                                              beta, C, b0);
-      } else if (M <= 32) {
+      } else if (M <= 32 && (sizeof(T) == 4 || cdiv(N, 128) * nb >= 4 * kSMs)) {
         k_gemm<T, 32, 128, 16, 2, 8><<<dim3(cdiv(N, 128), cdiv(M, 32), nb), 256, 0, st>>>(M, N, K, alpha, A, B,
                                                                                             beta, C, b0);
       } else if (tensor_f32()) {
         gemm_tensor(dim3(cdiv(N, 64), cdiv(M, 64), nb), M, N, K, alpha, A, B, beta, C, b0);
+      } else if (sizeof(T) == 8 && cdiv(N, 64) * cdiv(M, 64) * nb < 4 * kSMs) {
+        // double is FP64-pipe bound whatever the tile (a 64 x 64 tile of K =
+        // 128 holds an SM for 160 us): too few 64 x 64 tiles to fill the SMs
+        // evenly go as 32 x 32 ones
+        k_gemm<T, 32, 32, 16, 4, 2><<<dim3(cdiv(N, 32), cdiv(M, 32), nb), 128, 0, st>>>(M, N, K, alpha, A, B, beta,
+                                                                                          C, b0);
       } else {
         k_gemm<T, 64, 64, 16, 4, 4><<<dim3(cdiv(N, 64), cdiv(M, 64), nb), 256, 0, st>>>(M, N, K, alpha, A, B, beta,
                                                                                           C, b0);
@@ -102,8 +141,10 @@ struct Ctx {
   bool tf32;
   bool tensor_f32() const { return sizeof(T) == 4 && tf32; }
   // D and, when the transition matrix is block-diagonal with blocks of Q1
-  // (checked once per pass), Q1; 0: products with F are GEMMs.
+  // (checked once per pass), Q1; 0: products with F are GEMMs.  qlow: the one
+  // QL of all steps is lower triangular (checked with it).
   int D, fq1;
+  bool qlow;
 
   void fmul(int64_t batch, int K, MV<T> F, MV<T> X, T alpha, T beta, MV<T> Yv) {
     if (batch <= 0 || K <= 0) return;
@@ -141,19 +182,59 @@ struct Ctx {
     }
   }
 
-  // In place: W (m x n, n >= m) -> L in its first m columns, zeros elsewhere.
+  // In place: the first mt of W's m rows (n columns) -> L in their first
+  // columns, zeros right of the diagonal; the rows below are multiplied by the
+  // same reflectors.  low > 0: row j has no entry beyond column low + j (W =
+  // [X | S], S lower triangular from column low on), so a panel and its
+  // reflectors end there.  tria: all rows, no such structure.
   bool cluster_panels;
-  void tria(int64_t batch, int m, int n, MV<T> W) {
+  void tria(int64_t batch, int m, int n, MV<T> W) { tria_rows(batch, m, m, n, W, 0); }
+
+  void tria_rows(int64_t batch, int mt, int m, int n, MV<T> W, int low) {
     if (batch <= 0) return;
-    const bool cl = cluster_panels && n >= kClusterMinCols && batch <= kClusterMaxBatch;
-    const int nb = cl ? panel_rows((n + kClusterSize - 1) / kClusterSize, sizeof(T)) : panel_rows(n, sizeof(T));
-    for (int i0 = 0; i0 < m; i0 += nb) {
-      const int nbb = std::min(nb, m - i0);
-      const int np = n - i0;
+    using R = RegPanel<T>;
+    mt = std::min(mt, n);
+    for (int i0 = 0; i0 < mt;) {
+      const int width = low > 0 ? std::min(n, low + i0 + R::NW * R::RPW) - i0 : n - i0;
+      const bool reg = width <= R::cols;
+      const bool cl = !reg && cluster_panels && n >= kClusterMinCols && batch <= kClusterMaxBatch;
+      const int nb = reg ? R::NW * R::RPW
+                         : (cl ? panel_rows((width + kClusterSize - 1) / kClusterSize, sizeof(T))
+                               : panel_rows(width, sizeof(T)));
+      const int nbb = std::min(nb, mt - i0);
+      const int np = low > 0 ? std::min(n, low + i0 + nbb) - i0 : n - i0;
+      const int mr = m - i0 - nbb;  // rows below
       for (int64_t b0 = 0; b0 < batch; b0 += maxbatch) {
         const int64_t nbt = std::min<int64_t>(maxbatch, batch - b0);
         MV<T> Wb{W.p + b0 * W.bs, W.rs, W.cs, W.bs};
-        if (cl && np >= kClusterMinCols) {
+        MV<T> Wtr = sub(Wb, i0 + nbb, i0);
+        if (reg) {
+          const bool wy = mr > 0 && wy_smem(nb, np, sizeof(T)) <= kPanelSmem &&
+                          (sizeof(T) == 8 || cdiv(mr, kWyRows) * nbt <= kWyMaxBlocksF32);
+          T* tv = (mr > 0 && !wy) ? TV : nullptr;
+          const int nc = (int)cdiv(np, 32);
+          // T (nb x nb) goes to Y's place: k_wy_apply does not use Y, and the
+          // GEMMs that do use T V instead
+          auto go = [&](auto c) { launch_lq_panel<T, decltype(c)::value>(nbt, st, Wb, i0, nbb, np, V, Y, tv, vbs, ybs); };
+          if (nc <= 2) go(std::integral_constant<int, 2>{});
+          else if (nc <= 4) go(std::integral_constant<int, 4>{});
+          else if (nc <= 6) go(std::integral_constant<int, 6>{});
+          else if (nc <= 8) go(std::integral_constant<int, 8>{});
+          else if (nc <= 12) go(std::integral_constant<int, 12>{});
+          else if (nc <= 16) go(std::integral_constant<int, 16>{});
+          else if (nc <= 24) go(std::integral_constant<int, 24>{});
+          else go(std::integral_constant<int, 40>{});
+          if (wy) {
+            for (int64_t c0 = 0; c0 < nbt; c0 += kMaxGridYZ) {
+              const int64_t nbc = std::min<int64_t>(kMaxGridYZ, nbt - c0);
+              MV<T> Wc{Wtr.p + c0 * Wtr.bs, Wtr.rs, Wtr.cs, Wtr.bs};
+              k_wy_apply<T, kWyRows, R::NW * R::RPW>
+                  <<<dim3((unsigned)cdiv(mr, kWyRows), (unsigned)nbc), 128, wy_smem(nb, np, sizeof(T)), st>>>(
+                      Wc, mr, nbb, np, V + c0 * vbs, Y + c0 * ybs, vbs, ybs);
+            }
+            continue;  // (the next batch part)
+          }
+        } else if (cl) {
           const size_t smem = size_t(nbb) * ((np + kClusterSize - 1) / kClusterSize) * sizeof(T);
           k_tria_panel_cl<T, kClusterSize><<<(unsigned)(nbt * kClusterSize), 256, smem, st>>>(Wb, i0, nbb, np, V, TV,
                                                                                             vbs, 0);
@@ -161,16 +242,15 @@ struct Ctx {
           const size_t smem = size_t(nbb) * np * sizeof(T);
           k_tria_panel<T><<<(unsigned)nbt, 512, smem, st>>>(Wb, i0, nbb, np, V, TV, vbs, 0);
         }
-        const int mt = m - i0 - nbb;
-        if (mt > 0) {
-          MV<T> Wtr = sub(Wb, i0 + nbb, i0);
+        if (mr > 0) {
           MV<T> Vt{V, 1, np, vbs};  // V^T (np x nbb)
           MV<T> Yv{Y, nbb, 1, ybs};
           MV<T> TVv{TV, np, 1, vbs};
-          gemm(nbt, mt, nbb, np, T(1), Wtr, Vt, T(0), Yv);
-          gemm(nbt, mt, np, nbb, T(-1), Yv, TVv, T(1), Wtr);
+          gemm(nbt, mr, nbb, np, T(1), Wtr, Vt, T(0), Yv);
+          gemm(nbt, mr, np, nbb, T(-1), Yv, TVv, T(1), Wtr);
         }
       }
+      i0 += nbb;
     }
   }
 
@@ -292,23 +372,28 @@ int run(int which, int64_t n, int D, int d, const void* x0m, const void* x0L, co
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(k_tria_panel_cl<T, kClusterSize>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)kPanelSmem);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(k_wy_apply<T, kWyRows, RegPanel<T>::NW * RegPanel<T>::RPW>,
+                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPanelSmem);
     if (e != cudaSuccess) return cuda_status(e);
     attr_set = true;
   }
   const char* e = getenv("POF_DENSE_TF32");
   const char* ec = getenv("POF_DENSE_CLUSTER");
-  Ctx<T> cx{st, L.V, L.TV, L.Y, L.vbs, L.ybs, L.maxbatch, !(e && e[0] == '0'), D, 0, !(ec && ec[0] == '0')};
-  // one transition matrix: is it block-diagonal (Q1 = D / d, the IWP prior)?
-  if (fts == 0 && d >= 1 && D % d == 0 && D / d < D) {
-    const int q1 = D / d;
-    cudaError_t ce = cudaMemsetAsync(L.flag, 0, sizeof(unsigned int), st);
+  Ctx<T> cx{st, L.V, L.TV, L.Y, L.vbs, L.ybs, L.maxbatch, !(e && e[0] == '0'), D, 0, false, !(ec && ec[0] == '0')};
+  // one transition model: is F block-diagonal (Q1 = D / d, the IWP prior), QL
+  // lower triangular?
+  if (fts == 0) {
+    const int q1 = d >= 1 && D % d == 0 ? D / d : D;
+    cudaError_t ce = cudaMemsetAsync(L.flag, 0, 2 * sizeof(unsigned int), st);
     if (ce != cudaSuccess) return cuda_status(ce);
-    k_offblock_count<T><<<64, 256, 0, st>>>(D, q1, static_cast<const T*>(F), L.flag);
-    unsigned int h = 1;
-    ce = cudaMemcpyAsync(&h, L.flag, sizeof(h), cudaMemcpyDeviceToHost, st);
+    k_structure_count<T><<<64, 256, 0, st>>>(D, q1, static_cast<const T*>(F), static_cast<const T*>(QL), L.flag);
+    unsigned int h[2] = {1, 1};
+    ce = cudaMemcpyAsync(h, L.flag, sizeof(h), cudaMemcpyDeviceToHost, st);
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(st);
     if (ce != cudaSuccess) return cuda_status(ce);
-    if (h == 0) cx.fq1 = q1;
+    if (h[0] == 0 && q1 < D) cx.fq1 = q1;
+    cx.qlow = h[1] == 0;
   }
   run_schedule<T>(cx, L, which, static_cast<const T*>(x0m), static_cast<const T*>(x0L), static_cast<const T*>(F),
                   static_cast<const T*>(QL), fts, static_cast<const T*>(H), static_cast<const T*>(c),

@@ -12,6 +12,7 @@
 #include <stdint.h>
 
 #include "pof_dense_views.h"
+#include "pof_linalg.cuh"
 
 namespace pof {
 namespace dense {
@@ -20,7 +21,8 @@ namespace dense {
 // C = alpha * A B + beta * C, A (M x K), B (K x N), C (M x N) views; beta == 0
 // does not read C.  One CTA per BM x BN tile of one batch entry; the K loop
 // stages BK-deep tiles in shared memory with the loads ordered along
-// whichever index is contiguous in memory; each thread accumulates TM x TN
+// whichever index is contiguous in memory, the next tile on its way in
+// registers while the current one is used; each thread accumulates TM x TN
 // outputs strided across the tile.
 // ---------------------------------------------------------------------------
 template <typename T, int BM, int BN, int BK, int TM, int TN>
@@ -45,32 +47,56 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN))
     for (int j = 0; j < TN; ++j) acc[i][j] = T(0);
   const bool a_kc = A.cs == 1;
   const bool b_nc = B.cs == 1;
-  for (int k0 = 0; k0 < K; k0 += BK) {
-    for (int l = t; l < BM * BK; l += NT) {
+  constexpr int LA = (BM * BK + NT - 1) / NT, LB = (BK * BN + NT - 1) / NT;
+  T ra[LA], rb[LB];
+  auto a_at = [&](int l, int& mm, int& kk) {
+    if (a_kc)
+      kk = l % BK, mm = l / BK;
+    else
+      mm = l % BM, kk = l / BM;
+  };
+  auto b_at = [&](int l, int& nn, int& kk) {
+    if (b_nc)
+      nn = l % BN, kk = l / BN;
+    else
+      kk = l % BK, nn = l / BK;
+  };
+  auto load = [&](int k0) {
+#pragma unroll
+    for (int u = 0; u < LA; ++u) {
+      const int l = t + u * NT;
       int mm, kk;
-      if (a_kc) {
-        kk = l % BK;
-        mm = l / BK;
-      } else {
-        mm = l % BM;
-        kk = l / BM;
-      }
+      a_at(l, mm, kk);
       const int gm = m0 + mm, gk = k0 + kk;
-      As[kk][mm] = (gm < M && gk < K) ? Ab[gm * A.rs + gk * A.cs] : T(0);
+      ra[u] = (l < BM * BK && gm < M && gk < K) ? Ab[gm * A.rs + gk * A.cs] : T(0);
     }
-    for (int l = t; l < BK * BN; l += NT) {
+#pragma unroll
+    for (int u = 0; u < LB; ++u) {
+      const int l = t + u * NT;
       int nn, kk;
-      if (b_nc) {
-        nn = l % BN;
-        kk = l / BN;
-      } else {
-        kk = l % BK;
-        nn = l / BK;
-      }
+      b_at(l, nn, kk);
       const int gn = n0 + nn, gk = k0 + kk;
-      Bs[kk][nn] = (gn < N && gk < K) ? Bb[gk * B.rs + gn * B.cs] : T(0);
+      rb[u] = (l < BK * BN && gn < N && gk < K) ? Bb[gk * B.rs + gn * B.cs] : T(0);
+    }
+  };
+  load(0);
+  for (int k0 = 0; k0 < K; k0 += BK) {
+#pragma unroll
+    for (int u = 0; u < LA; ++u) {
+      const int l = t + u * NT;
+      int mm, kk;
+      a_at(l, mm, kk);
+      if (l < BM * BK) As[kk][mm] = ra[u];
+    }
+#pragma unroll
+    for (int u = 0; u < LB; ++u) {
+      const int l = t + u * NT;
+      int nn, kk;
+      b_at(l, nn, kk);
+      if (l < BK * BN) Bs[kk][nn] = rb[u];
     }
     __syncthreads();
+    if (k0 + BK < K) load(k0 + BK);
 #pragma unroll
     for (int kk = 0; kk < BK; ++kk) {
       T a[TM], bv[TN];
@@ -95,6 +121,46 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN))
       if (gn >= N) continue;
       T* c = Cb + gm * C.rs + gn * C.cs;
       *c = beta == T(0) ? alpha * acc[i][j] : fma(alpha, acc[i][j], beta * *c);
+    }
+  }
+}
+
+// y = alpha A x + beta y (one column): a warp per row when A's rows are
+// contiguous, else a thread per row (the lanes then read along a column).  The
+// skinny GEMM tile computed 16 columns for it: 80 us per product at M = K =
+// 128 in double.
+template <typename T>
+__global__ void __launch_bounds__(128) k_gemv(int M, int K, T alpha, MV<T> A, MV<T> x, T beta, MV<T> y, int64_t b0) {
+  const int64_t b = b0 + blockIdx.y;
+  const T* __restrict__ Ab = A.p + b * A.bs;
+  const T* __restrict__ xb = x.p + b * x.bs;
+  T* yb = y.p + b * y.bs;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (A.cs == 1) {
+    const int i = blockIdx.x * 4 + warp;
+    if (i >= M) return;
+    T s = T(0);
+    for (int k = lane; k < K; k += 32) s = fma(Ab[i * A.rs + k], xb[k * x.rs], s);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) {
+      T* o = yb + i * y.rs;
+      *o = beta == T(0) ? alpha * s : fma(alpha, s, beta * *o);
+    }
+  } else {
+    // 32 rows per CTA, the K range in four parts
+    __shared__ T part[4][32];
+    const int i = blockIdx.x * 32 + lane;
+    const int kq = (K + 3) / 4, k1 = min(K, (warp + 1) * kq);
+    T s = T(0);
+    if (i < M)
+      for (int k = warp * kq; k < k1; ++k) s = fma(Ab[i * A.rs + k * A.cs], xb[k * x.rs], s);
+    part[warp][lane] = s;
+    __syncthreads();
+    if (warp == 0 && i < M) {
+      s = (part[0][lane] + part[1][lane]) + (part[2][lane] + part[3][lane]);
+      T* o = yb + i * y.rs;
+      *o = beta == T(0) ? alpha * s : fma(alpha, s, beta * *o);
     }
   }
 }
@@ -313,18 +379,8 @@ __global__ void __launch_bounds__(512)
   __syncthreads();
   for (int j = 0; j < nbb; ++j) {
     const T* pr = P + j * np;
-    const T alpha = pr[j], s = nrm[j];
     T bj, tj, scale;
-    if (s == T(0)) {
-      tj = T(0);
-      bj = alpha;
-      scale = T(0);
-    } else {
-      const T h = hypot(alpha, sqrt(s));
-      bj = alpha >= T(0) ? -h : h;
-      tj = (bj - alpha) / bj;
-      scale = T(1) / (alpha - bj);
-    }
+    householder(pr[j], nrm[j], bj, tj, scale);
     if (t == 0) {
       tau[j] = tj;
       beta[j] = bj;
@@ -458,18 +514,8 @@ __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(256)
     cluster.sync();
     T tot = T(0);
     for (int r = 0; r < CS; ++r) tot += *cluster.map_shared_rank(&sq[pb], r);
-    const T alpha = *cluster.map_shared_rank(&al[pb], own);
     T bj, tj, scale;
-    if (tot == T(0)) {
-      tj = T(0);
-      bj = alpha;
-      scale = T(0);
-    } else {
-      const T h = hypot(alpha, sqrt(tot));
-      bj = alpha >= T(0) ? -h : h;
-      tj = (bj - alpha) / bj;
-      scale = T(1) / (alpha - bj);
-    }
+    householder(*cluster.map_shared_rank(&al[pb], own), tot, bj, tj, scale);
     for (int c = t; c < wl; c += bd)
       if (c0 + c > j) pr[c] *= scale;
     if (t == 0) {
@@ -559,6 +605,292 @@ __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(256)
 }
 
 // ---------------------------------------------------------------------------
+// The panel with its rows in registers: one CTA of NW warps per matrix, row r
+// of the panel in warp r mod NW (RPW rows each, nb = NW RPW), column c in lane
+// c mod 32 (NC columns per lane).  Per reflector the owner of row j forms its
+// squared norm and scalars and puts the row into shared memory (double
+// buffered: one barrier per reflector); every warp then takes the dot products
+// of its RPW rows with it -- the rows below are updated, the finished rows
+// above yield the Gram entries v_r . v_j of the compact WY factor, which cost
+// no pass of their own.  The RPW sums are reduced together (a value is halved
+// with every exchange: 6 additions for 4 rows instead of 20).
+//
+// k_tria_panel keeps the panel in shared memory, which it read and wrote four
+// times per reflector, and every thread of it formed hypot and two IEEE
+// divisions (about 100 FP64 instructions in double): 415 us per panel of 32
+// rows x 256 columns in double, 137 us at 768 columns in float.
+//
+// double: reflectors unnormalized (v = (u, x), coefficient kap); float:
+// v = (1, scal x), coefficient tau (Reflector).  Writes V (nbb x np), T (nb x
+// nb, upper triangular, H_0 .. H_{nbb-1} = I - V^T T V) and, when TV is given,
+// T V.
+// ---------------------------------------------------------------------------
+template <typename T>
+struct PanelCoef;  // what a reflector's row update and its V row need
+template <>
+struct PanelCoef<double> {
+  double beta, u, kap;
+  __device__ __forceinline__ void set(double alpha, double xn2) {
+    if (is_zero(xn2)) {
+      beta = alpha, u = 0.0, kap = 0.0;
+    } else {
+      const Reflector<double> h(alpha, xn2);
+      beta = h.beta, u = h.u, kap = h.kap;
+    }
+  }
+  __device__ __forceinline__ double row(double a, double dot, double& ws) const {
+    ws = kap * fma(u, a, dot);
+    return fma(-ws, u, a);
+  }
+  __device__ __forceinline__ double vdiag() const { return u; }
+  __device__ __forceinline__ double vscale() const { return 1.0; }
+  __device__ __forceinline__ double tau() const { return kap; }
+};
+template <>
+struct PanelCoef<float> {
+  float beta, t, scal;
+  __device__ __forceinline__ void set(float alpha, float xn2) { householder(alpha, xn2, beta, t, scal); }
+  __device__ __forceinline__ float row(float a, float dot, float& ws) const {
+    const float w = t * fmaf(scal, dot, a);
+    ws = w * scal;
+    return a - w;
+  }
+  __device__ __forceinline__ float vdiag() const { return 1.f; }
+  __device__ __forceinline__ float vscale() const { return scal; }
+  __device__ __forceinline__ float tau() const { return t; }
+};
+
+// sums of R values over the warp (R a power of two up to 32): lane l returns
+// the sum of value l / (32 / R)
+template <typename T, int R>
+__device__ __forceinline__ T warp_sums(const T (&v)[R]) {
+  const int lane = threadIdx.x & 31;
+  T a[R];
+#pragma unroll
+  for (int i = 0; i < R; ++i) a[i] = v[i];
+  int o = 16;
+#pragma unroll
+  for (int n = R; n > 1; n >>= 1, o >>= 1) {
+    const bool hi = (lane & o) != 0;
+#pragma unroll
+    for (int i = 0; i < n / 2; ++i) {
+      const T keep = hi ? a[i + n / 2] : a[i], give = hi ? a[i] : a[i + n / 2];
+      a[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+    }
+  }
+#pragma unroll
+  for (; o > 0; o >>= 1) a[0] += __shfl_xor_sync(0xffffffffu, a[0], o);
+  return a[0];
+}
+
+// CTAs per SM that the registers of a panel's rows leave room for
+template <typename T, int NC>
+constexpr int panel_ctas() {
+  return sizeof(T) == 8 ? (NC <= 6 ? 4 : (NC <= 12 ? 2 : 1)) : (NC <= 16 ? 2 : 1);
+}
+
+template <typename T, int NW, int RPW, int NC>
+__global__ void __launch_bounds__(NW * 32, (panel_ctas<T, NC>()))
+    k_lq_panel(MV<T> W, int i0, int nbb, int np, T* __restrict__ V, T* __restrict__ TT, T* __restrict__ TV,
+               int64_t vbs, int64_t tbs) {
+  constexpr int NB = NW * RPW;
+  __shared__ T pr[2][NC * 32];
+  __shared__ PanelCoef<T> co[NB];
+  __shared__ T G[NB][NB + 1], Tm[NB][NB + 1];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t b = blockIdx.x;
+  T* Wb = W.p + b * W.bs + (int64_t)i0 * W.rs + (int64_t)i0 * W.cs;
+  T q[RPW][NC];
+#pragma unroll
+  for (int s = 0; s < RPW; ++s) {
+    const int r = warp + NW * s;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      const int col = lane + 32 * c;
+      q[s][c] = (r < nbb && col < np) ? Wb[r * W.rs + col * W.cs] : T(0);
+    }
+  }
+  for (int j = 0; j < nbb; ++j) {
+    T* x_ = pr[j & 1];
+    if (warp == j % NW) {
+      const int js = j / NW;
+      T x[NC], s2 = T(0);
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        x[c] = q[0][c];
+#pragma unroll
+        for (int s = 1; s < RPW; ++s)
+          if (s == js) x[c] = q[s][c];
+      }
+      const T alpha = __shfl_sync(0xffffffffu, x[0], j);
+      if (lane <= j) x[0] = T(0);
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        s2 = fma(x[c], x[c], s2);
+        x_[lane + 32 * c] = x[c];
+      }
+      s2 = warp_sum(s2);
+      PanelCoef<T> h;
+      h.set(alpha, s2);
+      if (lane == 0) co[j] = h;
+    }
+    __syncthreads();
+    const PanelCoef<T> h = co[j];
+    T x[NC], d[RPW];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) x[c] = x_[lane + 32 * c];
+#pragma unroll
+    for (int s = 0; s < RPW; ++s) {
+      d[s] = T(0);
+#pragma unroll
+      for (int c = 0; c < NC; ++c) d[s] = fma(q[s][c], x[c], d[s]);
+    }
+    const T sum = warp_sums<T, RPW>(d);
+#pragma unroll
+    for (int s = 0; s < RPW; ++s) {
+      const int r = warp + NW * s;
+      const T dot = __shfl_sync(0xffffffffu, sum, s * (32 / RPW));
+      const T a = __shfl_sync(0xffffffffu, q[s][0], j);
+      if (r > j && r < nbb) {
+        T ws;
+        const T an = h.row(a, dot, ws);
+#pragma unroll
+        for (int c = 0; c < NC; ++c) q[s][c] = fma(-ws, x[c], q[s][c]);
+        if (lane == j) q[s][0] = an;
+      } else if (r < j) {  // finished row: v_r . v_j
+        if (lane == 0) G[r][j] = co[r].vscale() * fma(h.vscale(), dot, a * h.vdiag());
+      }
+    }
+  }
+  __syncthreads();
+  // panel rows of W and V
+  T* Vb = V + b * vbs;
+#pragma unroll
+  for (int s = 0; s < RPW; ++s) {
+    const int r = warp + NW * s;
+    if (r < nbb) {
+      const PanelCoef<T> h = co[r];
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        const int col = lane + 32 * c;
+        if (col < np) {
+          const T v = q[s][c];
+          Wb[r * W.rs + col * W.cs] = col < r ? v : (col == r ? h.beta : T(0));
+          Vb[(int64_t)r * np + col] = col < r ? T(0) : (col == r ? h.vdiag() : h.vscale() * v);
+        }
+      }
+    }
+  }
+  // T (upper triangular, forward column recurrence of dlarft), one row per lane
+  if (warp == 0 && lane < NB) {
+#pragma unroll 1
+    for (int j = 0; j < NB; ++j) {
+      T v = T(0);
+      if (j < nbb) {
+        T acc = T(0);
+#pragma unroll 8
+        for (int k = 0; k < j; ++k) acc = fma(Tm[lane][k], G[k][j], acc);
+        v = lane < j ? -co[j].tau() * acc : (lane == j ? co[j].tau() : T(0));
+      }
+      Tm[lane][j] = v;
+    }
+  }
+  __syncthreads();
+  T* Tb = TT + b * tbs;
+  for (int l = threadIdx.x; l < NB * NB; l += NW * 32) Tb[l] = Tm[l / NB][l % NB];
+  if (TV) {
+    T* TVb = TV + b * vbs;
+    for (int c = threadIdx.x; c < np; c += NW * 32) {
+      T v[NB];
+#pragma unroll
+      for (int k = 0; k < NB; ++k) v[k] = k < nbb ? Vb[(int64_t)k * np + c] : T(0);
+#pragma unroll 1
+      for (int i = 0; i < nbb; ++i) {
+        T acc = T(0);
+#pragma unroll
+        for (int k = 0; k < NB; ++k) acc = fma(Tm[i][k], v[k], acc);  // T is zero left of its diagonal
+        TVb[(int64_t)i * np + c] = acc;
+      }
+    }
+  }
+}
+
+// Rows below a panel: W <- W - ((W V^T) T) V, RB rows per CTA, in one launch
+// with the rows and V in shared memory (two GEMM launches with the product
+// W V^T going through memory before).  double: bound by the FP64 pipe, so small
+// row blocks that reach many SMs cost nothing.
+template <typename T, int RB, int NB>
+__global__ void __launch_bounds__(128)
+    k_wy_apply(MV<T> W, int rows, int nbb, int np, const T* __restrict__ V, const T* __restrict__ TT, int64_t vbs,
+               int64_t tbs) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int ld = np | 1;
+  T* Ws = reinterpret_cast<T*>(smem_raw);  // RB x ld
+  T* Vs = Ws + RB * ld;                    // NB x ld, zero from row nbb on
+  __shared__ T Ys[RB][NB + 1], Y2[NB][RB], Ts[NB][NB + 1];
+  const int t = threadIdx.x;
+  const int64_t b = blockIdx.y;
+  const int r0 = blockIdx.x * RB;
+  T* Wb = W.p + b * W.bs + (int64_t)r0 * W.rs;
+  const T* Vb = V + b * vbs;
+  const int nr = min(RB, rows - r0);
+  for (int l = t; l < RB * np; l += 128) {
+    const int r = l / np, c = l - r * np;
+    Ws[r * ld + c] = r < nr ? Wb[r * W.rs + c * W.cs] : T(0);
+  }
+  for (int l = t; l < NB * np; l += 128) {
+    const int r = l / np, c = l - r * np;
+    Vs[r * ld + c] = r < nbb ? Vb[l] : T(0);
+  }
+  for (int l = t; l < NB * NB; l += 128) Ts[l / NB][l % NB] = TT[b * tbs + l];
+  __syncthreads();
+  {  // Y = W V^T: thread t has row t mod RB and the columns t / RB + CS u
+    constexpr int CS = 128 / RB, U = NB / CS;
+    const int r = t % RB, j0 = t / RB;
+    T acc[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) acc[u] = T(0);
+#pragma unroll 4
+    for (int c = 0; c < np; ++c) {
+      const T w = Ws[r * ld + c];
+#pragma unroll
+      for (int u = 0; u < U; ++u) acc[u] = fma(w, Vs[(j0 + CS * u) * ld + c], acc[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) Ys[r][j0 + CS * u] = acc[u];
+  }
+  __syncthreads();
+  for (int l = t; l < RB * NB; l += 128) {
+    const int r = l % RB, j = l / RB;
+    T s = T(0);
+#pragma unroll
+    for (int k = 0; k < NB; ++k)
+      if (k <= j) s = fma(Ys[r][k], Ts[k][j], s);
+    Y2[j][r] = s;
+  }
+  __syncthreads();
+  for (int c = t; c < np; c += 128) {  // W -= (Y T) V, a column of the row block per thread
+    T acc[RB];
+#pragma unroll
+    for (int r = 0; r < RB; ++r) acc[r] = Ws[r * ld + c];
+    const int je = min(nbb, c + 1);  // V_j starts at column j
+#pragma unroll 2
+    for (int j = 0; j < je; ++j) {
+      const T v = Vs[j * ld + c];
+#pragma unroll
+      for (int r = 0; r < RB; ++r) acc[r] = fma(-Y2[j][r], v, acc[r]);
+    }
+#pragma unroll
+    for (int r = 0; r < RB; ++r) Ws[r * ld + c] = acc[r];
+  }
+  __syncthreads();
+  for (int l = t; l < nr * np; l += 128) {
+    const int r = l / np, c = l - r * np;
+    Wb[r * W.rs + c * W.cs] = Ws[r * ld + c];
+  }
+}
+
+// ---------------------------------------------------------------------------
 // Triangular solves.  op(L) X = B in place in B (M x K), L an M x M view that
 // is lower triangular (`upper` == false) or upper triangular (a transposed
 // lower view).  Few columns: k_trsv, one CTA per (column, batch entry),
@@ -599,13 +931,16 @@ constexpr int kTrsmBlock = 32;
 
 template <typename T>
 __global__ void k_trsm_diag(int nbr, MV<T> L, bool upper, MV<T> B, int K, int64_t b0) {
+  // (the diagonal inverted once per CTA: a division per column and row was
+  // most of this kernel's FP64 work)
   __shared__ T Ls[kTrsmBlock][kTrsmBlock + 1];
   const int t = threadIdx.x;
   const int64_t b = b0 + blockIdx.y;
   const T* Lb = L.p + b * L.bs;
   for (int l = t; l < nbr * nbr; l += blockDim.x) {
     const int i = l / nbr, j = l - i * nbr;
-    Ls[i][j] = Lb[i * L.rs + j * L.cs];
+    const T v = Lb[i * L.rs + j * L.cs];
+    Ls[i][j] = i == j ? rcp(v) : v;
   }
   __syncthreads();
   const int col = blockIdx.x * blockDim.x + t;
@@ -621,7 +956,7 @@ __global__ void k_trsm_diag(int nbr, MV<T> L, bool upper, MV<T> B, int K, int64_
         T v = x[i];
 #pragma unroll
         for (int j = 0; j < i; ++j) v -= Ls[i][j] * x[j];
-        x[i] = v / Ls[i][i];
+        x[i] = v * Ls[i][i];
       }
     }
   } else {
@@ -632,7 +967,7 @@ __global__ void k_trsm_diag(int nbr, MV<T> L, bool upper, MV<T> B, int K, int64_
 #pragma unroll
         for (int j = i + 1; j < kTrsmBlock; ++j)
           if (j < nbr) v -= Ls[i][j] * x[j];
-        x[i] = v / Ls[i][i];
+        x[i] = v * Ls[i][i];
       }
     }
   }
@@ -689,16 +1024,19 @@ __global__ void k_blockdiag_mm(int D, int Q1, int K, MV<T> F, MV<T> X, T alpha, 
 }
 
 // out[0] = number of non-zero entries of F (D x D) outside its diagonal
-// Q1 x Q1 blocks (out[0] must be zero on entry).
+// Q1 x Q1 blocks, out[1] = of QL above its diagonal (both zero on entry).
 template <typename T>
-__global__ void k_offblock_count(int D, int Q1, const T* __restrict__ F, unsigned int* __restrict__ out) {
-  unsigned int cnt = 0;
+__global__ void k_structure_count(int D, int Q1, const T* __restrict__ F, const T* __restrict__ QL,
+                                  unsigned int* __restrict__ out) {
+  unsigned int cf = 0, cq = 0;
   for (int64_t l = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; l < (int64_t)D * D;
        l += (int64_t)gridDim.x * blockDim.x) {
     const int i = (int)(l / D), j = (int)(l - (int64_t)i * D);
-    if (i / Q1 != j / Q1 && F[l] != T(0)) ++cnt;
+    if (i / Q1 != j / Q1 && F[l] != T(0)) ++cf;
+    if (j > i && QL[l] != T(0)) ++cq;
   }
-  if (cnt) atomicAdd(out, cnt);
+  if (cf) atomicAdd(out, cf);
+  if (cq) atomicAdd(out + 1, cq);
 }
 
 // Per-step filter terms from P11 (d x d lower), w = P11^{-1}(-r) and

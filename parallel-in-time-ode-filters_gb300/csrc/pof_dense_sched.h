@@ -10,6 +10,15 @@
 //   tria(batch, m, n, W)                           W (m x n, n >= m) -> L in
 //                                                  its first m columns, zeros
 //                                                  elsewhere (L L^T = W W^T)
+//   tria_rows(batch, mt, m, n, W, low), ql_low     optional: the factorization
+//                                                  of W's first mt rows only,
+//                                                  applied to the rows below,
+//                                                  with W = [X | S], S lower
+//                                                  triangular from column low
+//                                                  on (0: no such structure);
+//                                                  whether QL is lower
+//                                                  triangular.  Without them
+//                                                  tria factors all rows.
 //   trsm(batch, M, K, L, upper, B)                 op(L) X = B in place
 //   step_terms(batch, d, P11, w, wq, nll, ssq, stride), sqnorm(batch, len, x, out),
 //   scalars(nll, ssq, fobj, sobj, n, C0, d, out, which)
@@ -180,13 +189,51 @@ Layout<T> layout(char* base, int which, int64_t n, int D, int d, int chunks,
   const int nmax = std::max(2 * D, D + d), mmax = std::max(2 * D, D + d);
   L.maxbatch = std::max<int64_t>(P, S);
   L.vbs = (int64_t)kMaxPanel * nmax;
-  L.ybs = (int64_t)mmax * kMaxPanel;
+  L.ybs = (int64_t)std::max(mmax, kMaxPanel) * kMaxPanel;  // W V^T of the rows below, or a panel's T
   L.V = a.take<T>(L.maxbatch * L.vbs);
   L.TV = a.take<T>(L.maxbatch * L.vbs);
   L.Y = a.take<T>(L.maxbatch * L.ybs);
   L.flag = reinterpret_cast<unsigned int*>(a.take<double>(1));
   L.total = a.off + 256;  // alignment slack of aligned_ws
   return L;
+}
+
+// tria_rows of a context that has it, else tria of all m rows (nf >= m columns,
+// those beyond n zero).
+template <typename X, typename T>
+auto lead_tria(X& cx, int64_t batch, int mt, int m, int n, int nf, MV<T> W, int low, int)
+    -> decltype(cx.tria_rows(batch, mt, m, n, W, low), void()) {
+  (void)nf;
+  cx.tria_rows(batch, mt, m, n, W, low);
+}
+template <typename X, typename T>
+void lead_tria(X& cx, int64_t batch, int, int m, int, int nf, MV<T> W, int, long) {
+  cx.tria(batch, m, nf, W);
+}
+// [X | S], S lower triangular from column low on: all m rows
+template <typename X, typename T>
+void tria_low(X& cx, int64_t batch, int m, int n, MV<T> W, int low) {
+  lead_tria(cx, batch, m, m, n, n, W, low, 0);
+}
+// low of [F L | QL]: D when the context knows QL to be lower triangular
+template <typename X>
+auto ql_low(const X& cx, int D, int) -> decltype((void)cx.qlow, int()) {
+  return cx.qlow ? D : 0;
+}
+template <typename X>
+int ql_low(const X&, int, long) {
+  return 0;
+}
+// Phi = [[F L, QL], [L, 0]] (2 D x 2 D): the first D rows' factorization, then
+// the bottom right block's own (a smaller matrix than factoring all rows).
+template <typename X, typename T>
+auto phi_tria(X& cx, int64_t batch, int D, MV<T> Phi, int) -> decltype((void)cx.qlow, void()) {
+  cx.tria_rows(batch, D, 2 * D, 2 * D, Phi, cx.qlow ? D : 0);
+  cx.tria(batch, D, D, sub(Phi, D, D));
+}
+template <typename X, typename T>
+void phi_tria(X& cx, int64_t batch, int D, MV<T> Phi, long) {
+  cx.tria(batch, 2 * D, 2 * D, Phi);
 }
 
 template <typename T>
@@ -288,7 +335,9 @@ struct OpScratch {
   }
 };
 
-// Xi = tria([[U1^T Z2, I], [Z2, 0]]) and m = Xi11^{-1} U1^T (filter.py:117-142)
+// Xi = tria([[U1^T Z2, I], [Z2, 0]]) and m = Xi11^{-1} U1^T (filter.py:117-142);
+// Xi22, the bottom right block, enters only Z = tria([A1^T Xi22, Z1]), which
+// takes any square root: it is left as the first D rows' reflectors make it
 template <typename T, typename X>
 void op_xi(X& cx, int D, int64_t G, MV<T> U1, MV<T> Z2, const OpScratch<T>& o) {
   const T one(1), zero(0);
@@ -296,7 +345,7 @@ void op_xi(X& cx, int D, int64_t G, MV<T> U1, MV<T> Z2, const OpScratch<T>& o) {
   cx.fill(G, D, D, zero, one, sub(o.Xi, 0, D));
   cx.copy(G, D, D, Z2, sub(o.Xi, D, 0));
   cx.fill(G, D, D, zero, zero, sub(o.Xi, D, D));
-  cx.tria(G, 2 * D, 2 * D, o.Xi);
+  lead_tria(cx, G, D, 2 * D, 2 * D, 2 * D, o.Xi, D, 0);
   cx.copy(G, D, D, tr(U1), o.m);
   cx.trsm(G, D, D, o.Xi, false, o.m);
 }
@@ -335,7 +384,7 @@ void op_filter(X& cx, int D, int64_t G, const FElem<T>& e1, const FElem<T>& e2, 
   // U = tria([M^T | U2])
   cx.copy(G, D, D, tr(o.M), o.X5);
   cx.copy(G, D, D, e2.U, sub(o.X5, 0, D));
-  cx.tria(G, D, 2 * D, o.X5);
+  tria_low(cx, G, D, 2 * D, o.X5, D);
   cx.copy(G, D, D, o.X5, out.U);
   // eta = A1^T (I - e^T U1^T)(eta2 - Z2 Z2^T b1) + eta1,  e = Xi11^{-T} Xi21^T
   cx.copy(G, D, D, tr(Xi21), o.e);
@@ -351,7 +400,7 @@ void op_filter(X& cx, int D, int64_t G, const FElem<T>& e1, const FElem<T>& e2, 
   // Z = tria([A1^T Xi22 | Z1])
   cx.gemm(G, D, D, D, one, tr(A1), Xi22, zero, o.X6);
   cx.copy(G, D, D, e1.Z, sub(o.X6, 0, D));
-  cx.tria(G, D, 2 * D, o.X6);
+  tria_low(cx, G, D, 2 * D, o.X6, D);
   cx.copy(G, D, D, o.X6, out.Z);
 }
 
@@ -366,7 +415,7 @@ void op_propagate(X& cx, int D, int64_t G, const State<T>& s, const FElem<T>& e2
   op_b(cx, D, G, s.m, s.L, A2, b2, e2.eta, out.m, o);
   cx.gemm(G, D, D, D, one, A2, tr(o.m), zero, o.X5);
   cx.copy(G, D, D, e2.U, sub(o.X5, 0, D));
-  cx.tria(G, D, 2 * D, o.X5);
+  tria_low(cx, G, D, 2 * D, o.X5, D);
   cx.copy(G, D, D, o.X5, out.L);
 }
 
@@ -442,7 +491,7 @@ void smoother_tree(X& cx, const Layout<T>& L, const SElem<T>& lev0, const State<
     cx.gemm(G2, D, D, D, one, early.E, late.E, zero, out.E);
     cx.gemm(G2, D, D, D, one, early.E, late.Dm, zero, o.X5);
     cx.copy(G2, D, D, early.Dm, sub(o.X5, 0, D));
-    cx.tria(G2, D, 2 * D, o.X5);
+    tria_low(cx, G2, D, 2 * D, o.X5, D);
     cx.copy(G2, D, D, o.X5, out.Dm);
     if (n[l] % 2) {
       const SElem<T> a = lev[l].at(n[l] - 1), b = lev[l + 1].at(G2);
@@ -465,7 +514,7 @@ void smoother_tree(X& cx, const Layout<T>& L, const SElem<T>& lev0, const State<
     cx.gemm(G2, D, 1, D, one, late.E, en[l + 1].m, one, even.m);
     cx.gemm(G2, D, D, D, one, late.E, en[l + 1].L, zero, o.X5);
     cx.copy(G2, D, D, late.Dm, sub(o.X5, 0, D));
-    cx.tria(G2, D, 2 * D, o.X5);
+    tria_low(cx, G2, D, 2 * D, o.X5, D);
     cx.copy(G2, D, D, o.X5, even.L);
     if (n[l] % 2) {  // a last element alone in its pair ends where its parent ends
       const State<T> a = en[l + 1].at(G2), b = en[l].at(n[l] - 1);
@@ -503,12 +552,13 @@ void run_filter(X& cx, const Layout<T>& L, const Model<T>& md, const T* x0m, con
       cx.fill(Pa, d, d, zero, zero, sub(X2v, 0, D));
     cx.copy(Pa, D, D, X1v, sub(X2v, d, 0));
     cx.fill(Pa, D, d, zero, zero, sub(X2v, d, D));
-    cx.tria(Pa, d + D, D + d, X2v);
+    // without noise the last d columns are zero
+    lead_tria(cx, Pa, d + D, d + D, md.R ? D + d : D, D + d, X2v, 0, 0);
   };
   auto predict = [&](int Pa, int s, MV<T> Lprev) {
     cx.fmul(Pa, D, Fv(s), Lprev, one, zero, X1v);
     cx.copy(Pa, D, D, QLv(s), sub(X1v, 0, D));
-    cx.tria(Pa, D, 2 * D, X1v);
+    tria_low(cx, Pa, D, 2 * D, X1v, ql_low(cx, D, 0));
   };
 
   // phase 1: conditional fold of every chunk
@@ -531,9 +581,10 @@ void run_filter(X& cx, const Layout<T>& L, const Model<T>& md, const T* x0m, con
     // reads the totals of chunks 0..P-2 only, which are active every step)
     cur = 1 - cur;
     cx.gemm(Pa, D, 1, d, T(-1), tr(Grv), sub(Grv, 0, D), one, etav);
-    cx.copy(Pa, D, D, Zv, X3v);
-    cx.copy(Pa, D, d, tr(Grv), sub(X3v, 0, D));
-    cx.tria(Pa, D, D + d, X3v);
+    // [W^T | Z], Z lower triangular: the tails are d + 1 columns long
+    cx.copy(Pa, D, d, tr(Grv), X3v);
+    cx.copy(Pa, D, D, Zv, sub(X3v, 0, d));
+    tria_low(cx, Pa, D, D + d, X3v, d);
     cx.copy(Pa, D, D, X3v, Zv);
     cx.copy(Pa, D, D, U, Lcv);
   }
@@ -591,7 +642,7 @@ void run_smoother(X& cx, const Layout<T>& L, const T* F, const T* QL, int64_t ft
     cx.copy(Sb, D, D, QLk, sub(Phiv, 0, D));
     cx.copy(Sb, D, D, Lk, sub(Phiv, D, 0));
     cx.fill(Sb, D, D, zero, zero, sub(Phiv, D, D));
-    cx.tria(Sb, 2 * D, 2 * D, Phiv);
+    phi_tria(cx, Sb, D, Phiv, 0);
     cx.trsm(Sb, D, D, tr(Phiv), true, tr(sub(Phiv, D, 0)));  // P21 block := E = P21 P11^{-1}
     cx.copy(Sb, D, D, sub(Phiv, D, 0), Ek);
     cx.copy(Sb, D, D, sub(Phiv, D, D), Dk);
@@ -618,7 +669,7 @@ void run_smoother(X& cx, const Layout<T>& L, const T* F, const T* QL, int64_t ft
     cx.gemm(Pa, D, 1, D, one, tEv[0], gv(off), one, tgv);
     cx.gemm(Pa, D, D, D, one, tEv[0], Dv(off), zero, Xsv);
     cx.copy(Pa, D, D, tDv, sub(Xsv, 0, D));
-    cx.tria(Pa, D, 2 * D, Xsv);
+    tria_low(cx, Pa, D, 2 * D, Xsv, D);
     cx.copy(Pa, D, D, Xsv, tDv);
     cx.copy(Pa, D, D, tEv[1], tEv[0]);
   }
@@ -633,7 +684,7 @@ void run_smoother(X& cx, const Layout<T>& L, const T* F, const T* QL, int64_t ft
     cx.gemm(Pa, D, 1, D, one, Ev(off), emv, one, tmv);
     cx.gemm(Pa, D, D, D, one, Ev(off), eLv, zero, Xsv);
     cx.copy(Pa, D, D, Dv(off), sub(Xsv, 0, D));
-    cx.tria(Pa, D, 2 * D, Xsv);
+    tria_low(cx, Pa, D, 2 * D, Xsv, D);
     cx.copy(Pa, D, 1, tmv, MV<T>{om + (int64_t)off * D, 1, 1, (int64_t)C0 * D});
     cx.copy(Pa, D, D, Xsv, rowmajor(oL + off * DD, D, C0 * DD));
     cx.copy(Pa, D, 1, tmv, emv);
