@@ -206,6 +206,63 @@ struct Reflector<float> {
   }
 };
 
+// Accumulator of an inner product, v + sum a b.  double: fused multiply-adds.
+// float: compensated (Ogita, Rump and Oishi, "Accurate sum and dot product",
+// SISC 2005, Dot2), one rounding for the whole sum: the states carry integrals
+// over the grid, along which the sums' rounding errors add up.  FP32
+// instructions are not what bounds these kernels: on a float32 pass of 2000
+// steps at D = 6 all team sums compensated cost 0.420 -> 0.460 ms and take the
+// means' error against 64 bits from 2.0e-6 to 1.6e-6 (16 inputs), of 2900
+// steps from 4.0e-6 to 2.8e-6.
+template <typename T>
+struct Acc;
+template <>
+struct Acc<double> {
+  double h;
+  Acc() = default;
+  __device__ __forceinline__ explicit Acc(double v) : h(v) {}
+  __device__ __forceinline__ void mul_add(double a, double b) { h = fma(a, b, h); }
+  __device__ __forceinline__ void join(unsigned mask, int o, int width) {
+    h += __shfl_xor_sync(mask, h, o, width);
+  }
+  __device__ __forceinline__ double plus(double v) const { return v + h; }   // v + the sum
+  __device__ __forceinline__ double from(double v) const { return v - h; }   // v - the sum
+  __device__ __forceinline__ double value() const { return h; }
+};
+template <>
+struct Acc<float> {
+  float h, l;
+  Acc() = default;
+  __device__ __forceinline__ explicit Acc(float v) : h(v), l(0.f) {}
+  __device__ __forceinline__ void add(float p) {  // h + p exactly as h + error
+    const float s = __fadd_rn(h, p), t = __fsub_rn(s, h);
+    l = __fadd_rn(l, __fadd_rn(__fsub_rn(h, __fsub_rn(s, t)), __fsub_rn(p, t)));
+    h = s;
+  }
+  __device__ __forceinline__ void mul_add(float a, float b) {
+    const float p = __fmul_rn(a, b);
+    l = __fadd_rn(l, __fmaf_rn(a, b, -p));
+    add(p);
+  }
+  __device__ __forceinline__ void join(unsigned mask, int o, int width) {
+    const float h2 = __shfl_xor_sync(mask, h, o, width), l2 = __shfl_xor_sync(mask, l, o, width);
+    add(h2);
+    l = __fadd_rn(l, l2);
+  }
+  __device__ __forceinline__ float plus(float v) const {
+    Acc<float> a = *this;
+    a.add(v);
+    return a.value();
+  }
+  __device__ __forceinline__ float from(float v) const {
+    Acc<float> a(v);
+    a.add(-h);
+    a.l = __fsub_rn(a.l, l);
+    return a.value();
+  }
+  __device__ __forceinline__ float value() const { return __fadd_rn(h, l); }
+};
+
 // C(MxN) = A(MxK) * B(KxN)
 template <typename T, int M, int K, int N, int LDA, int LDB, int LDC>
 __device__ __forceinline__ void mm(const T* __restrict__ A, const T* __restrict__ B, T* __restrict__ C) {

@@ -54,14 +54,14 @@ template <typename T, int TS, int M, int K, int N, int LDA, int LDB, int LDC, bo
 __device__ __forceinline__ void t_mm(const Team<TS>& tm, const T* A, const T* B, T* C) {
   for (int idx = tm.r; idx < M * N; idx += TS) {
     const int i = idx / N, j = idx % N;
-    T s = T(0);
+    Acc<T> s(T(0));
 #pragma unroll
     for (int k = 0; k < K; ++k) {
       const T a = TA ? A[k * LDA + i] : A[i * LDA + k];
       const T b = TB ? B[j * LDB + k] : B[k * LDB + j];
-      s = fma(a, b, s);
+      s.mul_add(a, b);
     }
-    C[i * LDC + j] = s;
+    C[i * LDC + j] = s.value();
   }
 }
 
@@ -69,10 +69,10 @@ __device__ __forceinline__ void t_mm(const Team<TS>& tm, const T* A, const T* B,
 template <typename T, int TS, int M, int K, int LDA, bool TA = false>
 __device__ __forceinline__ void t_mv(const Team<TS>& tm, const T* A, const T* x, T* y) {
   for (int i = tm.r; i < M; i += TS) {
-    T s = T(0);
+    Acc<T> s(T(0));
 #pragma unroll
-    for (int k = 0; k < K; ++k) s = fma(TA ? A[k * LDA + i] : A[i * LDA + k], x[k], s);
-    y[i] = s;
+    for (int k = 0; k < K; ++k) s.mul_add(TA ? A[k * LDA + i] : A[i * LDA + k], x[k]);
+    y[i] = s.value();
   }
 }
 
@@ -160,12 +160,12 @@ __device__ __forceinline__ void t_lq(const Team<TS>& tm, T* X, T* Y, const Tail&
     const T alpha = xj[j];
     const int ne = M - j + MB;  // entries of this reflector; pass p has one if p RS < ne
     T* row[NP];
-    T dot[NP];
+    Acc<T> dot[NP];
 #pragma unroll
     for (int p = 0; p < NP; ++p) {
       const int e = slot + p * RS;
       row[p] = e >= ne ? X + j * LD : (e < M - j ? X + (j + e) * LD : Y + (e - (M - j)) * LDY);
-      dot[p] = T(0);
+      dot[p] = Acc<T>(T(0));
     }
     if constexpr (Tail::count > 0 && Tail::count % G == 0) {
 #pragma unroll
@@ -173,7 +173,7 @@ __device__ __forceinline__ void t_lq(const Team<TS>& tm, T* X, T* Y, const Tail&
         const T x = xj[kb + ph + t];
 #pragma unroll
         for (int p = 0; p < NP; ++p)
-          if (p == 0 || p * RS < ne) dot[p] = fma(row[p][kb + ph + t], x, dot[p]);
+          if (p == 0 || p * RS < ne) dot[p].mul_add(row[p][kb + ph + t], x);
       }
     } else {
 #pragma unroll 2
@@ -181,14 +181,14 @@ __device__ __forceinline__ void t_lq(const Team<TS>& tm, T* X, T* Y, const Tail&
         const T x = xj[k];
 #pragma unroll
         for (int p = 0; p < NP; ++p)
-          if (p == 0 || p * RS < ne) dot[p] = fma(row[p][k], x, dot[p]);
+          if (p == 0 || p * RS < ne) dot[p].mul_add(row[p][k], x);
       }
     }
 #pragma unroll
     for (int o = RS; o < TS; o <<= 1)
 #pragma unroll
-      for (int p = 0; p < NP; ++p) dot[p] += __shfl_xor_sync(tm.mask, dot[p], o, TS);
-    const T xn2 = __shfl_sync(tm.mask, dot[0], src);
+      for (int p = 0; p < NP; ++p) dot[p].join(tm.mask, o, TS);
+    const T xn2 = __shfl_sync(tm.mask, dot[0].value(), src);
     pj = -1;
     if (is_zero(xn2)) continue;
     const Reflector<T> h(alpha, xn2);
@@ -200,7 +200,7 @@ __device__ __forceinline__ void t_lq(const Team<TS>& tm, T* X, T* Y, const Tail&
       if (e == 0 || e >= ne) continue;
       T* xi = row[p];
       T ws;
-      const T a = h.row(xi[j], dot[p], ws);
+      const T a = h.row(xi[j], dot[p].value(), ws);
       if (ph == 0) xi[j] = a;
       if constexpr (Tail::count > 0 && Tail::count % G == 0) {
 #pragma unroll
@@ -216,25 +216,26 @@ __device__ __forceinline__ void t_lq(const Team<TS>& tm, T* X, T* Y, const Tail&
   tm.sync();
 }
 
-// The value (op(A) x)(i) for row i = lane's row slot (zero for slots beyond
-// M), A given by its row and column strides; G = TS / slots lanes share a
-// row's terms, every lane of a slot gets the sum.
+// The sum (op(A) x)(i) for row i = lane's row slot, A given by its row and
+// column strides; G = TS / slots lanes share a row's terms, every lane of a
+// slot gets the sum (slots beyond M: row 0's).
 template <typename T, int TS, int M, int K>
-__device__ __forceinline__ T t_dotrow(const Team<TS>& tm, const T* A, int rs, int cs, const T* x) {
+__device__ __forceinline__ Acc<T> t_dotrow(const Team<TS>& tm, const T* A, int rs, int cs, const T* x) {
   constexpr int RS = Pow2Ceil<M>::v < TS ? Pow2Ceil<M>::v : TS;
   constexpr int G = TS / RS;
   static_assert(M <= RS, "one row per lane");
   const int i = tm.r % RS < M ? tm.r % RS : 0;
-  T s = T(0);
+  Acc<T> s(T(0));
 #pragma unroll
   for (int k0 = 0; k0 < K; k0 += G) {
     const int k = k0 + tm.r / RS;
-    if (K % G == 0 || k < K) s = fma(A[i * rs + k * cs], x[k], s);
+    if (K % G == 0 || k < K) s.mul_add(A[i * rs + k * cs], x[k]);
   }
 #pragma unroll
-  for (int o = RS; o < TS; o <<= 1) s += __shfl_xor_sync(tm.mask, s, o, TS);
+  for (int o = RS; o < TS; o <<= 1) s.join(tm.mask, o, TS);
   return s;
 }
+
 // C(M x N) = A(M x N) B with B (N x N) lower triangular: column group t of
 // the outputs starts its sum at the group's first column (terms above B's
 // diagonal are exact zeros), one row per lane slot.
@@ -250,10 +251,10 @@ __device__ __forceinline__ void t_mm_lowB(const Team<TS>& tm, const T* A, const 
     for (int t = 0; t < N; t += CG) {
       const int j = t + tm.r / RS;
       if (N % CG != 0 && j >= N) continue;
-      T s = T(0);
+      Acc<T> s(T(0));
 #pragma unroll
-      for (int k = t; k < N; ++k) s = fma(A[i * LDA + k], B[k * LDB + j], s);
-      C[i * LDC + j] = s;
+      for (int k = t; k < N; ++k) s.mul_add(A[i * LDA + k], B[k * LDB + j]);
+      C[i * LDC + j] = s.value();
     }
   }
 }
@@ -279,20 +280,20 @@ __device__ __forceinline__ void t_trsm_l(const Team<TS>& tm, const T* L, T* B) {
     for (int j = tm.r; j < NR; j += TS) {
 #pragma unroll
       for (int i = 0; i < M; ++i) {
-        T s = B[i * LDB + j];
+        Acc<T> s(B[i * LDB + j]);
 #pragma unroll
-        for (int k = 0; k < i; ++k) s = fma(-L[i * LDL + k], B[k * LDB + j], s);
-        B[i * LDB + j] = s * rdi[i];
+        for (int k = 0; k < i; ++k) s.mul_add(-L[i * LDL + k], B[k * LDB + j]);
+        B[i * LDB + j] = s.value() * rdi[i];
       }
     }
   } else {
     for (int j = tm.r; j < NR; j += TS) {
 #pragma unroll
       for (int i = 0; i < M; ++i) {
-        T s = B[i * LDB + j];
+        Acc<T> s(B[i * LDB + j]);
 #pragma unroll
-        for (int k = 0; k < i; ++k) s = fma(-L[i * LDL + k], B[k * LDB + j], s);
-        B[i * LDB + j] = s * rcp(L[i * LDL + i]);
+        for (int k = 0; k < i; ++k) s.mul_add(-L[i * LDL + k], B[k * LDB + j]);
+        B[i * LDB + j] = s.value() * rcp(L[i * LDL + i]);
       }
     }
   }
@@ -310,20 +311,20 @@ __device__ __forceinline__ void t_trsm_lt(const Team<TS>& tm, const T* L, T* B) 
     for (int j = tm.r; j < NR; j += TS) {
 #pragma unroll
       for (int i = M - 1; i >= 0; --i) {
-        T s = B[i * LDB + j];
+        Acc<T> s(B[i * LDB + j]);
 #pragma unroll
-        for (int k = i + 1; k < M; ++k) s = fma(-L[k * LDL + i], B[k * LDB + j], s);
-        B[i * LDB + j] = s * rdi[i];
+        for (int k = i + 1; k < M; ++k) s.mul_add(-L[k * LDL + i], B[k * LDB + j]);
+        B[i * LDB + j] = s.value() * rdi[i];
       }
     }
   } else {
     for (int j = tm.r; j < NR; j += TS) {
 #pragma unroll
       for (int i = M - 1; i >= 0; --i) {
-        T s = B[i * LDB + j];
+        Acc<T> s(B[i * LDB + j]);
 #pragma unroll
-        for (int k = i + 1; k < M; ++k) s = fma(-L[k * LDL + i], B[k * LDB + j], s);
-        B[i * LDB + j] = s * rcp(L[i * LDL + i]);
+        for (int k = i + 1; k < M; ++k) s.mul_add(-L[k * LDL + i], B[k * LDB + j]);
+        B[i * LDB + j] = s.value() * rcp(L[i * LDL + i]);
       }
     }
   }
@@ -408,35 +409,35 @@ __device__ __forceinline__ void t_filt_combine(const Team<TS>& tm, FiltTeamWs<T,
   T* const va = hi ? w.v3 : w.v1;
   T* const vb = hi ? w.v4 : w.v2;
   const T* const S = hi ? w.Z2 : w.U1;
-  T x = t_dotrow<T, TS / 2, D, D>(h, S, 1, L1, hi ? w.b1 : w.e2);
-  if (put) va[h.r] = x;
+  Acc<T> x = t_dotrow<T, TS / 2, D, D>(h, S, 1, L1, hi ? w.b1 : w.e2);
+  if (put) va[h.r] = x.value();
   tm.sync();
   x = t_dotrow<T, TS / 2, D, D>(h, S, L1, 1, va);
-  if (put) vb[h.r] = hi ? w.e2[h.r] - x : w.b1[h.r] + x;  // read again after t_filt_xi's barriers
+  if (put) vb[h.r] = hi ? x.from(w.e2[h.r]) : x.plus(w.b1[h.r]);  // read again after t_filt_xi's barriers
   t_filt_xi<T, TS, D>(tm, w);
   // b: t3 = Xi21^T t2, t2 -= Mu^T t3; eta: s3 = Mu s2, s2 -= Xi21 s3
   // (one instruction stream: the halves differ in pointers and strides)
   x = t_dotrow<T, TS / 2, D, D>(h, hi ? w.Mu : w.Xb, hi ? L1 : 1, hi ? 1 : L2, vb);
-  if (put) va[h.r] = x;
+  if (put) va[h.r] = x.value();
   tm.sync();
   x = t_dotrow<T, TS / 2, D, D>(h, hi ? w.Xb : w.Mu, hi ? L2 : 1, hi ? 1 : L1, va);
-  if (put) vb[h.r] -= x;
+  if (put) vb[h.r] = x.from(vb[h.r]);
   tm.sync();
   // b = A2 t2 + b2; eta = A1^T s2 + eta1
   x = t_dotrow<T, TS / 2, D, D>(h, hi ? w.A1 : w.A2, hi ? 1 : L1, hi ? L1 : 1, vb);
   if (put) {
     if (hi)
-      w.e1[h.r] += x;
+      w.e1[h.r] = x.plus(w.e1[h.r]);
     else
-      w.b1[h.r] = w.b2[h.r] + x;
+      w.b1[h.r] = x.plus(w.b2[h.r]);
   }
   // W = A2 - M^T Xi21^T
   for (int idx = tm.r; idx < D * D; idx += TS) {
     const int i = idx / D, j = idx % D;
-    T s = w.A2[i * L1 + j];
+    Acc<T> s(w.A2[i * L1 + j]);
 #pragma unroll
-    for (int k = 0; k < D; ++k) s = fma(-w.M[k * L1 + i], w.Xb[j * L2 + k], s);
-    w.W[i * L1 + j] = s;
+    for (int k = 0; k < D; ++k) s.mul_add(-w.M[k * L1 + i], w.Xb[j * L2 + k]);
+    w.W[i * L1 + j] = s.value();
   }
   // Z = tria([Z1 | A1^T Xi22]) (the rows of Xt reused), U = tria([U2 | M^T])
   t_mm<T, TS, D, D, D, L1, L2, L2, true, false>(tm, w.A1, w.Xb + D, w.Xt + D);
@@ -464,22 +465,22 @@ __device__ __forceinline__ void t_filt_apply(const Team<TS>& tm, FiltTeamWs<T, D
   using W = FiltTeamWs<T, D>;
   constexpr int L1 = W::LD1, L2 = W::LD2;
   const bool put = tm.r < D;
-  T x = t_dotrow<T, TS, D, D>(tm, w.U1, 1, L1, w.e2);
-  if (put) w.v1[tm.r] = x;
+  Acc<T> x = t_dotrow<T, TS, D, D>(tm, w.U1, 1, L1, w.e2);
+  if (put) w.v1[tm.r] = x.value();
   tm.sync();
   x = t_dotrow<T, TS, D, D>(tm, w.U1, L1, 1, w.v1);
-  if (put) w.v2[tm.r] = w.b1[tm.r] + x;
+  if (put) w.v2[tm.r] = x.plus(w.b1[tm.r]);
   t_filt_xi<T, TS, D>(tm, w);
   x = t_dotrow<T, TS, D, D>(tm, w.Xb, 1, L2, w.v2);
-  if (put) w.v3[tm.r] = x;
+  if (put) w.v3[tm.r] = x.value();
   t_copy<T, TS, D, D, L1, L2, true>(tm, w.M, w.UX + D);
   t_copy<T, TS, D, D, L1, L2>(tm, w.U2, w.UX);
   tm.sync();
   x = t_dotrow<T, TS, D, D>(tm, w.Mu, 1, L1, w.v3);
-  if (put) w.v1[tm.r] = w.v2[tm.r] - x;
+  if (put) w.v1[tm.r] = x.from(w.v2[tm.r]);
   tm.sync();
   x = t_dotrow<T, TS, D, D>(tm, w.A2, L1, 1, w.v1);
-  if (put) w.b1[tm.r] = w.b2[tm.r] + x;
+  if (put) w.b1[tm.r] = x.plus(w.b2[tm.r]);
   t_lq<T, TS, D, 0, L2, L2>(tm, w.UX, w.UX, TailFixed<D, 2 * D>{});
   t_copy<T, TS, D, D, L2, L1>(tm, w.UX, w.U1);
   tm.sync();
@@ -502,12 +503,12 @@ template <typename T, int TS, int D>
 __device__ __forceinline__ void t_smooth_combine(const Team<TS>& tm, SmoTeamWs<T, D>& w) {
   using W = SmoTeamWs<T, D>;
   constexpr int L1 = W::LD1, L2 = W::LD2;
-  const T x = t_dotrow<T, TS, D, D>(tm, w.E2, L1, 1, w.g1);
+  const Acc<T> x = t_dotrow<T, TS, D, D>(tm, w.E2, L1, 1, w.g1);
   t_mm_lowB<T, TS, D, D, L1, L1, L2>(tm, w.E2, w.D1, w.X + D);
   t_copy<T, TS, D, D, L1, L2>(tm, w.D2m, w.X);
   t_mm<T, TS, D, D, D, L1, L1, L1>(tm, w.E2, w.E1, w.En);
   t_lq<T, TS, D, 0, L2, L2>(tm, w.X, w.X, TailFixed<D, 2 * D>{});
-  if (tm.r < D) w.g2[tm.r] += x;
+  if (tm.r < D) w.g2[tm.r] = x.plus(w.g2[tm.r]);
   t_copy<T, TS, D, D, L1, L1>(tm, w.En, w.E2);
   t_copy<T, TS, D, D, L2, L1>(tm, w.X, w.D2m);
   tm.sync();
@@ -519,11 +520,11 @@ template <typename T, int TS, int D>
 __device__ __forceinline__ void t_smooth_apply(const Team<TS>& tm, SmoTeamWs<T, D>& w) {
   using W = SmoTeamWs<T, D>;
   constexpr int L1 = W::LD1, L2 = W::LD2;
-  const T x = t_dotrow<T, TS, D, D>(tm, w.E2, L1, 1, w.g1);
+  const Acc<T> x = t_dotrow<T, TS, D, D>(tm, w.E2, L1, 1, w.g1);
   t_mm<T, TS, D, D, D, L1, L1, L2>(tm, w.E2, w.D1, w.X + D);
   t_copy<T, TS, D, D, L1, L2>(tm, w.D2m, w.X);
   t_lq<T, TS, D, 0, L2, L2>(tm, w.X, w.X, TailFixed<D, 2 * D>{});
-  if (tm.r < D) w.g1[tm.r] = x + w.g2[tm.r];
+  if (tm.r < D) w.g1[tm.r] = x.plus(w.g2[tm.r]);
   t_copy<T, TS, D, D, L2, L1>(tm, w.X, w.D1);
   tm.sync();
 }
@@ -563,10 +564,10 @@ __device__ __forceinline__ void t_mm_cols(const Team<TS>& tm, const T* A, const 
 #pragma unroll
     for (int k = 0; k < N; ++k) a[k] = A[i * LDA + k];
     for (int j = tm.r / RS; j < nc; j += CG) {
-      T s = T(0);
+      Acc<T> s(T(0));
 #pragma unroll
-      for (int k = 0; k < N; ++k) s = fma(a[k], B[k * LDB + j], s);
-      C[i * LDC + j] = s;
+      for (int k = 0; k < N; ++k) s.mul_add(a[k], B[k * LDB + j]);
+      C[i * LDC + j] = s.value();
     }
   }
 }
@@ -591,7 +592,7 @@ __device__ __forceinline__ void t_smooth_combine_raw(const Team<TS>& tm, SmoTeam
   using W = SmoTeamWs<T, D>;
   constexpr int L1 = W::LD1, L2 = W::LD2;
   const int n1 = t_ncols<T, TS, D, D, L1>(tm, w.D1);
-  const T x = t_dotrow<T, TS, D, D>(tm, w.E2, L1, 1, w.g1);
+  const Acc<T> x = t_dotrow<T, TS, D, D>(tm, w.E2, L1, 1, w.g1);
   t_mm<T, TS, D, D, D, L1, L1, L1>(tm, w.E2, w.E1, w.En);
   if (first) {  // [E2 D1 | D2], both dense
     const int n2 = t_ncols<T, TS, D, D, L1>(tm, w.D2m);
@@ -606,7 +607,7 @@ __device__ __forceinline__ void t_smooth_combine_raw(const Team<TS>& tm, SmoTeam
     t_copy<T, TS, D, D, L1, L2>(tm, w.D2m, w.X);
     t_lq<T, TS, D, 0, L2, L2>(tm, w.X, w.X, TailRange{D, D + n1});
   }
-  if (tm.r < D) w.g2[tm.r] += x;
+  if (tm.r < D) w.g2[tm.r] = x.plus(w.g2[tm.r]);
   t_copy<T, TS, D, D, L1, L1>(tm, w.En, w.E2);
   for (int idx = tm.r; idx < D * D; idx += TS) {
     const int i = idx / D, k = idx % D;
@@ -622,14 +623,14 @@ __device__ __forceinline__ void t_smooth_apply_raw(const Team<TS>& tm, SmoTeamWs
   using W = SmoTeamWs<T, D>;
   constexpr int L1 = W::LD1, L2 = W::LD2;
   const int nk = t_ncols<T, TS, D, D, L1>(tm, w.D2m);
-  const T x = t_dotrow<T, TS, D, D>(tm, w.E2, L1, 1, w.g1);
+  const Acc<T> x = t_dotrow<T, TS, D, D>(tm, w.E2, L1, 1, w.g1);
   if (lower)
     t_mm_lowB<T, TS, D, D, L1, L1, L2>(tm, w.E2, w.D1, w.X);
   else
     t_mm<T, TS, D, D, D, L1, L1, L2>(tm, w.E2, w.D1, w.X);
   t_copy<T, TS, D, D, L1, L2>(tm, w.D2m, w.X + D);
   t_lq<T, TS, D, 0, L2, L2>(tm, w.X, w.X, TailUpper{D + nk});
-  if (tm.r < D) w.g1[tm.r] = x + w.g2[tm.r];
+  if (tm.r < D) w.g1[tm.r] = x.plus(w.g2[tm.r]);
   for (int idx = tm.r; idx < D * D; idx += TS) {
     const int i = idx / D, k = idx % D;
     w.D1[i * L1 + k] = k <= i ? w.X[i * L2 + k] : T(0);
@@ -746,9 +747,9 @@ __device__ __forceinline__ void t_predict(const Team<TS>& tm, WS& w, const T* F,
     const int i = idx / D, j = idx % D;
     if (j >= nl) continue;
     const int k0 = ss.wf ? i : 0, k1 = ss.wf ? (i / ss.wf + 1) * ss.wf : D;
-    T s = T(0);
-    for (int k = k0; k < k1; ++k) s = fma(F[i * L1 + k], w.L[k * L1 + j], s);
-    w.X[i * L2 + D + j] = s;
+    Acc<T> s(T(0));
+    for (int k = k0; k < k1; ++k) s.mul_add(F[i * L1 + k], w.L[k * L1 + j]);
+    w.X[i * L2 + D + j] = s.value();
   }
   T* Y = w.X;
   if constexpr (SMOOTH) {
@@ -779,9 +780,9 @@ __device__ __forceinline__ void t_psi(const Team<TS>& tm, WS& w, StepObs ob) {
   constexpr int L1 = W::LD1, L2 = W::LD2, LP = W::LDP, DP = W::DP;
   for (int idx = tm.r; idx < DY * D; idx += TS) {
     const int i = idx / D, j = idx % D;
-    T s = T(0);
-    for (int k = 0; k < ob.h1; ++k) s = fma(w.H[i * L1 + k], w.X[k * L2 + j], s);
-    w.P[i * LP + j] = s;
+    Acc<T> s(T(0));
+    for (int k = 0; k < ob.h1; ++k) s.mul_add(w.H[i * L1 + k], w.X[k * L2 + j]);
+    w.P[i * LP + j] = s.value();
   }
   if (!ob.rzero)
     for (int idx = tm.r; idx < DY * DY; idx += TS) w.P[(idx / DY) * LP + D + idx % DY] = w.R[idx];
@@ -815,8 +816,9 @@ __device__ __forceinline__ void t_innovation(const Team<TS>& tm, WS& w, const T*
   constexpr int L1 = W::LD1, LP = W::LDP;
   const int src = (threadIdx.x & 31) / TS * TS;
   const int i = tm.r % DY;
-  T s = w.c[i];
-  for (int k = 0; k < h1; ++k) s = fma(w.H[i * L1 + k], x[k], s);
+  Acc<T> sa(w.c[i]);
+  for (int k = 0; k < h1; ++k) sa.mul_add(w.H[i * L1 + k], x[k]);
+  const T s = sa.value();
   const T rd = rcp(w.P[i * LP + i]);
 #pragma unroll
   for (int a = 0; a < DY; ++a) {
@@ -843,9 +845,9 @@ __device__ __forceinline__ void t_predict_gain(const Team<TS>& tm, WS& w, const 
   static_assert(D <= TS && DY <= TS, "one row of the state per lane");
   for (int i = tm.r; i < D; i += TS) {
     const int k0 = ss.wf ? i : 0, k1 = ss.wf ? (i / ss.wf + 1) * ss.wf : D;
-    T s = T(0);
-    for (int k = k0; k < k1; ++k) s = fma(F[i * L1 + k], w.m[k], s);
-    w.mp[i] = s;
+    Acc<T> s(T(0));
+    for (int k = k0; k < k1; ++k) s.mul_add(F[i * L1 + k], w.m[k]);
+    w.mp[i] = s.value();
   }
   t_predict<T, TS, D, DY, SMOOTH>(tm, w, F, QL, ss, nl, lower);  // Phi11 = X[:, :D], Phi21 = Y[:, :D]
   if constexpr (SMOOTH) {
@@ -856,16 +858,16 @@ __device__ __forceinline__ void t_predict_gain(const Team<TS>& tm, WS& w, const 
     T x[D];
 #pragma unroll
     for (int i = D - 1; i >= 0; --i) {
-      T s = w.Y[j * L2 + i];
+      Acc<T> s(w.Y[j * L2 + i]);
 #pragma unroll
-      for (int k = i + 1; k < D; ++k) s = fma(-w.X[k * L2 + i], x[k], s);
-      x[i] = s * __shfl_sync(tm.mask, rd, src + i);
+      for (int k = i + 1; k < D; ++k) s.mul_add(-w.X[k * L2 + i], x[k]);
+      x[i] = s.value() * __shfl_sync(tm.mask, rd, src + i);
     }
-    T gj = w.m[j];
+    Acc<T> gj(w.m[j]);
 #pragma unroll
-    for (int i = 0; i < D; ++i) gj = fma(-x[i], w.mp[i], gj);
+    for (int i = 0; i < D; ++i) gj.mul_add(-x[i], w.mp[i]);
     if (tm.r < D) {
-      w.g[j] = gj;
+      w.g[j] = gj.value();
 #pragma unroll
       for (int i = 0; i < D; ++i) w.E[j * L1 + i] = x[i];
     }
@@ -899,10 +901,10 @@ __device__ __forceinline__ int t_kf_step(const Team<TS>& tm, WS& w, const T* F, 
   yy += (double)y2;
   if (tm.r < DY) lp.mul(w.P[tm.r * LP + tm.r]);
   for (int i = tm.r; i < D; i += TS) {
-    T acc = w.mp[i];
+    Acc<T> acc(w.mp[i]);
 #pragma unroll
-    for (int k = 0; k < DY; ++k) acc = fma(w.P[(DY + i) * LP + k], wv[k], acc);
-    w.m[i] = acc;
+    for (int k = 0; k < DY; ++k) acc.mul_add(w.P[(DY + i) * LP + k], wv[k]);
+    w.m[i] = acc.value();
   }
   t_psi22<T, TS, D, DY>(tm, w, ob);
   tm.sync();
@@ -940,25 +942,25 @@ __device__ __forceinline__ int t_cond_fold_step(const Team<TS>& tm, StepFoldWs<T
   if (Q1 > 0 && ss.wf) {
 #pragma unroll
     for (int i = 0; i < D; ++i) {
-      T s = T(0);
+      Acc<T> s(T(0));
 #pragma unroll
-      for (int k = i; k < (i / (Q1 > 0 ? Q1 : 1) + 1) * Q1; ++k) s = fma(F[i * L1 + k], fr.a[k], s);
-      fa[i] = s;
+      for (int k = i; k < (i / (Q1 > 0 ? Q1 : 1) + 1) * Q1; ++k) s.mul_add(F[i * L1 + k], fr.a[k]);
+      fa[i] = s.value();
     }
   } else {
 #pragma unroll
     for (int i = 0; i < D; ++i) {
-      T s = T(0);
+      Acc<T> s(T(0));
 #pragma unroll
-      for (int k = 0; k < D; ++k) s = fma(F[i * L1 + k], fr.a[k], s);
-      fa[i] = s;
+      for (int k = 0; k < D; ++k) s.mul_add(F[i * L1 + k], fr.a[k]);
+      fa[i] = s.value();
     }
   }
   for (int i = tm.r; i < D; i += TS) {
     const int k0 = ss.wf ? i : 0, k1 = ss.wf ? (i / ss.wf + 1) * ss.wf : D;
-    T s = T(0);
-    for (int k = k0; k < k1; ++k) s = fma(F[i * L1 + k], w.m[k], s);
-    w.mp[i] = s;
+    Acc<T> s(T(0));
+    for (int k = k0; k < k1; ++k) s.mul_add(F[i * L1 + k], w.m[k]);
+    w.mp[i] = s.value();
   }
   tm.sync();
   // w = Psi11^{-1} (H Fb + c) = -wv, W = Psi11^{-1} H FA (lane's column)
@@ -966,13 +968,13 @@ __device__ __forceinline__ int t_cond_fold_step(const Team<TS>& tm, StepFoldWs<T
   t_innovation<T, TS, D, DY>(tm, w, w.mp, ob.h1, r, rdv, wv);
 #pragma unroll
   for (int i = 0; i < DY; ++i) {
-    T s = T(0);
+    Acc<T> s(T(0));
 #pragma unroll
     for (int k = 0; k < D; ++k)
-      if (k < ob.h1) s = fma(w.H[i * L1 + k], fa[k], s);
+      if (k < ob.h1) s.mul_add(w.H[i * L1 + k], fa[k]);
 #pragma unroll
-    for (int k = 0; k < i; ++k) s = fma(-w.P[i * LP + k], wc[k], s);
-    wc[i] = s * rdv[i];
+    for (int k = 0; k < i; ++k) s.mul_add(-w.P[i * LP + k], wc[k]);
+    wc[i] = s.value() * rdv[i];
   }
   // A = FA - Psi21 W; b = Fb - Psi21 w; eta -= W^T w; [Z | W^T]
 #pragma unroll
@@ -989,10 +991,10 @@ __device__ __forceinline__ int t_cond_fold_step(const Team<TS>& tm, StepFoldWs<T
     for (int k = 0; k < DY; ++k) w.ZX[tm.r * LZ + D + k] = wc[k];
   }
   for (int i = tm.r; i < D; i += TS) {
-    T acc = w.mp[i];
+    Acc<T> acc(w.mp[i]);
 #pragma unroll
-    for (int k = 0; k < DY; ++k) acc = fma(w.P[(DY + i) * LP + k], wv[k], acc);
-    w.m[i] = acc;
+    for (int k = 0; k < DY; ++k) acc.mul_add(w.P[(DY + i) * LP + k], wv[k]);
+    w.m[i] = acc.value();
   }
   t_psi22<T, TS, D, DY>(tm, w, ob);
   t_lq<T, TS, D, 0, LZ, LZ>(tm, w.ZX, w.ZX, TailFixed<D, D + DY>{});
