@@ -72,7 +72,7 @@ struct Layout {
   // batched operator application over at most G = ceil(P / 2) pairs
   T *TAb, *TU, *Teta, *TZ, *Sb, *SU;
   T *TgS, *TES, *TDS, *Em, *EL;
-  T *OXi, *OM, *OT, *Om, *Oe, *OX5, *OX6, *Ov;
+  T *OXi, *OM, *OT, *Om, *OX5, *OX6, *Ov;
   int G;
   double *nll, *ssq, *fobj, *sobj;
   // smoother
@@ -181,7 +181,6 @@ Layout<T> layout(char* base, int which, int64_t n, int D, int d, int chunks,
   L.OM = a.take<T>(G * DD);
   L.OT = a.take<T>(G * DD);
   L.Om = a.take<T>(G * DD);
-  L.Oe = a.take<T>(G * DD);
   L.OX5 = a.take<T>(G * 2 * DD);
   L.OX6 = a.take<T>(G * 2 * DD);
   L.Ov = a.take<T>(G * 8 * D);
@@ -319,7 +318,7 @@ struct SElem {  // smoother elements (g, E, D)
 
 template <typename T>
 struct OpScratch {
-  MV<T> Xi, M, Tm, m, e, X5, X6;
+  MV<T> Xi, M, Tm, m, X5, X6;
   MV<T> v[8];
   explicit OpScratch(const Layout<T>& L) {
     const int D = L.D;
@@ -328,7 +327,6 @@ struct OpScratch {
     M = rowmajor(L.OM, D, DD);
     Tm = rowmajor(L.OT, D, DD);
     m = rowmajor(L.Om, D, DD);
-    e = rowmajor(L.Oe, D, DD);
     X5 = rowmajor(L.OX5, 2 * D, 2 * DD);
     X6 = rowmajor(L.OX6, 2 * D, 2 * DD);
     for (int i = 0; i < 8; ++i) v[i] = MV<T>{L.Ov + (int64_t)i * L.G * D, 1, 1, D};
@@ -350,18 +348,20 @@ void op_xi(X& cx, int D, int64_t G, MV<T> U1, MV<T> Z2, const OpScratch<T>& o) {
   cx.trsm(G, D, D, o.Xi, false, o.m);
 }
 
-// b = A2 (I - m^T Xi21^T)(b1 + U1 U1^T eta2) + b2, written to out
+// s2 = eta2 - Z2 Z2^T b1 in v[1], s3 = m s2 in v[2], and
+// b = A2 (I - m^T Xi21^T)(b1 + U1 U1^T eta2) + b2 = A2 (b1 + m^T s3) + b2,
+// written to out (m = Xi11^{-1} U1^T; the second form has no terms that cancel
+// where the information is large)
 template <typename T, typename X>
-void op_b(X& cx, int D, int64_t G, MV<T> b1, MV<T> U1, MV<T> A2, MV<T> b2, MV<T> eta2, MV<T> out,
+void op_b(X& cx, int D, int64_t G, MV<T> b1, MV<T> Z2, MV<T> A2, MV<T> b2, MV<T> eta2, MV<T> out,
           const OpScratch<T>& o) {
   const T one(1), zero(0);
-  const MV<T> Xi21 = sub(o.Xi, D, 0);
-  cx.gemm(G, D, 1, D, one, tr(U1), eta2, zero, o.v[0]);
-  cx.copy(G, D, 1, b1, o.v[1]);
-  cx.gemm(G, D, 1, D, one, U1, o.v[0], one, o.v[1]);
-  cx.gemm(G, D, 1, D, one, tr(Xi21), o.v[1], zero, o.v[2]);
-  cx.copy(G, D, 1, o.v[1], o.v[3]);
-  cx.gemm(G, D, 1, D, T(-1), tr(o.m), o.v[2], one, o.v[3]);
+  cx.gemm(G, D, 1, D, one, tr(Z2), b1, zero, o.v[0]);
+  cx.copy(G, D, 1, eta2, o.v[1]);
+  cx.gemm(G, D, 1, D, T(-1), Z2, o.v[0], one, o.v[1]);
+  cx.gemm(G, D, 1, D, one, o.m, o.v[1], zero, o.v[2]);
+  cx.copy(G, D, 1, b1, o.v[3]);
+  cx.gemm(G, D, 1, D, one, tr(o.m), o.v[2], one, o.v[3]);
   cx.copy(G, D, 1, b2, out);
   cx.gemm(G, D, 1, D, one, A2, o.v[3], one, out);
 }
@@ -380,21 +380,16 @@ void op_filter(X& cx, int D, int64_t G, const FElem<T>& e1, const FElem<T>& e2, 
   cx.gemm(G, D, D, D, one, tr(Xi21), A1, zero, o.Tm);
   cx.gemm(G, D, D, D, one, A2, A1, zero, out.Ab);
   cx.gemm(G, D, D, D, T(-1), tr(o.M), o.Tm, one, out.Ab);
-  op_b(cx, D, G, b1, e1.U, A2, b2, e2.eta, sub(out.Ab, 0, D), o);
+  op_b(cx, D, G, b1, e2.Z, A2, b2, e2.eta, sub(out.Ab, 0, D), o);
   // U = tria([M^T | U2])
   cx.copy(G, D, D, tr(o.M), o.X5);
   cx.copy(G, D, D, e2.U, sub(o.X5, 0, D));
   tria_low(cx, G, D, 2 * D, o.X5, D);
   cx.copy(G, D, D, o.X5, out.U);
-  // eta = A1^T (I - e^T U1^T)(eta2 - Z2 Z2^T b1) + eta1,  e = Xi11^{-T} Xi21^T
-  cx.copy(G, D, D, tr(Xi21), o.e);
-  cx.trsm(G, D, D, tr(Xi11), true, o.e);
-  cx.gemm(G, D, 1, D, one, tr(e2.Z), b1, zero, o.v[4]);
-  cx.copy(G, D, 1, e2.eta, o.v[5]);
-  cx.gemm(G, D, 1, D, T(-1), e2.Z, o.v[4], one, o.v[5]);
-  cx.gemm(G, D, 1, D, one, tr(e1.U), o.v[5], zero, o.v[6]);
-  cx.copy(G, D, 1, o.v[5], o.v[7]);
-  cx.gemm(G, D, 1, D, T(-1), tr(o.e), o.v[6], one, o.v[7]);
+  // eta = A1^T (I - e^T U1^T)(eta2 - Z2 Z2^T b1) + eta1 with e = Xi11^{-T} Xi21^T,
+  // e^T U1^T = Xi21 m
+  cx.copy(G, D, 1, o.v[1], o.v[7]);
+  cx.gemm(G, D, 1, D, T(-1), Xi21, o.v[2], one, o.v[7]);
   cx.copy(G, D, 1, e1.eta, out.eta);
   cx.gemm(G, D, 1, D, one, tr(A1), o.v[7], one, out.eta);
   // Z = tria([A1^T Xi22 | Z1])
@@ -412,7 +407,7 @@ void op_propagate(X& cx, int D, int64_t G, const State<T>& s, const FElem<T>& e2
   const T one(1), zero(0);
   const MV<T> A2 = e2.Ab, b2 = sub(e2.Ab, 0, D);
   op_xi(cx, D, G, s.L, e2.Z, o);
-  op_b(cx, D, G, s.m, s.L, A2, b2, e2.eta, out.m, o);
+  op_b(cx, D, G, s.m, e2.Z, A2, b2, e2.eta, out.m, o);
   cx.gemm(G, D, D, D, one, A2, tr(o.m), zero, o.X5);
   cx.copy(G, D, D, e2.U, sub(o.X5, 0, D));
   tria_low(cx, G, D, 2 * D, o.X5, D);
