@@ -29,7 +29,7 @@ BatchShape batch_shape(int dtype, int D, int d, int C0, int Cg, int64_t total_st
   sh.team = env_int("POF_BATCH_TEAM_WIDE") ? ops->tsw : ops->tsn;
   sh.team_up = ops->tsw;
   if (C0 <= 0) C0 = env_int("POF_BATCH_C0");
-  sh.C0 = C0 > 0 ? C0 : batch_pick_c0(total_steps, sh.team);
+  sh.C0 = C0 > 0 ? C0 : batch_pick_c0(total_steps, sh.team, sh.esz);
   if (Cg <= 1) Cg = env_int("POF_BATCH_CG");
   sh.Cg = Cg > 1 ? Cg : 2;
   return sh;
@@ -335,7 +335,7 @@ int pof_ieks_solve_batch(int32_t dtype, int64_t B, const int64_t* n_steps, int32
 size_t pof_batch_mixed_workspace_bytes(int64_t B, const int64_t* n_steps, int32_t D, int32_t d, int32_t C0,
                                        int32_t Cg) {
   BatchCtx c64, c32;
-  if (c64.init(POF_F64, B, n_steps, D, d, C0, Cg) || c32.init(POF_F32, B, n_steps, D, d, C0, Cg)) return 0;
+  if (c32.init(POF_F32, B, n_steps, D, d, C0, Cg) || c64.init(POF_F64, B, n_steps, D, d, c32.sh.C0, Cg)) return 0;
   return c64.bytes() + c32.bytes() + mixed_extras(c32).total + 256;
 }
 
@@ -346,8 +346,9 @@ int pof_ieks_solve_batch_mixed(int64_t B, const int64_t* n_steps, int32_t D, int
                                int32_t Cg, double* info, double* info_f32, void* workspace, size_t workspace_bytes,
                                void* stream) {
   BatchCtx c64, c32;
-  int rc = c64.init(POF_F64, B, n_steps, D, d, C0, Cg);
-  if (!rc) rc = c32.init(POF_F32, B, n_steps, D, d, C0, Cg);
+  // both phases in the float32 one's chunks: the float64 phase has few problems left
+  int rc = c32.init(POF_F32, B, n_steps, D, d, C0, Cg);
+  if (!rc) rc = c64.init(POF_F64, B, n_steps, D, d, c32.sh.C0, Cg);
   if (rc) return rc;
   rc = check_fields(B, d, fields, h);
   if (rc) return rc;

@@ -107,16 +107,23 @@ inline BatchPersist batch_persist(int64_t B, int64_t G, int D, int DY, int esz) 
   return p;
 }
 
-// Chunk length rule when the caller gives none: about 8 x 8192 level-0
-// chunks over the whole batch for 8-lane teams (several waves of the ~3600
-// teams a GB300 holds at once, so the tail of the last wave is short),
-// chunks as long as that allows, since the levels above level 0 cost more
-// per step.  Measured on 512 FitzHugh-Nagumo problems (1.14 M steps): C0 =
-// 32 (36 k chunks) 14.1 s, 64 (18 k) 14.9 s, 128 (9 k) 18.1 s.
-inline int batch_pick_c0(int64_t total_steps, int lanes) {
-  const int64_t target = 8 * (65536 / (lanes > 0 ? lanes : 1));
+// Chunk length rule when the caller gives none, in two parts.  From 4 to 8
+// steps once chunks of 4 would be more than 49152 lanes (float32: 262144,
+// its combines cost less against a step's latency): a step of level 0 costs
+// less than its share of the levels above, and there are lanes enough without
+// the shorter chunks.  From 8 on only while more than 8 x 65536 lanes are left
+// (several waves of the ~3600 8-lane teams a GB300 holds at once), since a
+// batch loses problems as they converge and its last ones wait for their
+// longest chunk.  Van der Pol solves, ms with chunks of 4 / 8 / 16 / 32: 40
+// problems of 10 k steps in all (q = 2) 11.5 / 13.2 / 18.4 / 29.3, 45 of 31 k
+// (q = 3) 25.6 / 23.6 / 27.8, 64 of 47 k 30.8 / 27.4 / 30.9 / 45.0, 192 of
+// 227 k 110 / 98.9 / 97.8 / 97.7; with the float32 phase 64 of 47 k 26.7 /
+// 28.7 / 37.5, 192 of 227 k 73.9 / 70.5 / 75.0 / 89.7.
+inline int batch_pick_c0(int64_t total_steps, int lanes, int esz = 8) {
+  const int64_t l = lanes > 0 ? lanes : 1;
   int c = 4;
-  while (c < 256 && total_steps / c > target) c *= 2;
+  if (total_steps / c > (esz == 4 ? 262144 : 49152) / l) c = 8;
+  while (c < 256 && total_steps / c > 8 * (65536 / l)) c *= 2;
   return c;
 }
 
