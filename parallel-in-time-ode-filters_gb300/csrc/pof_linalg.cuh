@@ -206,6 +206,23 @@ struct Reflector<float> {
   }
 };
 
+// A kernel launched while the one before it still runs (launch_next in
+// pof_driver.cuh): grid_begin waits for that kernel's end and its writes, then
+// lets the next launch come in.  Every thread passes it before it touches
+// memory, and the pointers go through it, so that no load of a read-only
+// parameter can be moved ahead of the wait.  In an ordinary launch both
+// instructions do nothing that could be seen.
+template <typename P>
+__device__ __forceinline__ void grid_begin_ptr(P& p) {
+  asm volatile("" : "+l"(p)::"memory");
+}
+template <typename... P>
+__device__ __forceinline__ void grid_begin(P&... p) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  (grid_begin_ptr(p), ...);
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // Accumulator of an inner product, v + sum a b.  double: fused multiply-adds.
 // float: compensated (Ogita, Rump and Oishi, "Accurate sum and dot product",
 // SISC 2005, Dot2), one rounding for the whole sum: the states carry integrals

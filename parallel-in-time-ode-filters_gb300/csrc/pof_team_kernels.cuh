@@ -177,6 +177,7 @@ __device__ __forceinline__ void t_store_smo(const Team<TS>& tm, T* base, int64_t
 // Filter up-sweep at level l >= 1: fold C consecutive elements per team.
 template <typename T, int D, int TS>
 __global__ void k_filt_reduce_team(const T* __restrict__ in, int64_t nin, int C, T* __restrict__ out, int64_t nout) {
+  grid_begin(in, out);
   using WS = FiltTeamWs<T, D>;
   POF_TEAM_PROLOGUE(WS)
   if (t >= nout) return;
@@ -214,6 +215,7 @@ __device__ __forceinline__ void t_filt_advance(const Team<TS>& tm, FiltTeamWs<T,
 template <typename T, int D, int TS>
 __global__ void k_filt_down_team(const T* __restrict__ elems, int64_t n, int C, const T* __restrict__ states_up,
                                  int64_t nup, T* __restrict__ states) {
+  grid_begin(elems, states_up, states);
   using WS = FiltTeamWs<T, D>;
   POF_TEAM_PROLOGUE(WS)
   if (t >= nup) return;
@@ -245,6 +247,7 @@ __global__ void k_filt_down_team(const T* __restrict__ elems, int64_t n, int C, 
 template <typename T, int D, int TS>
 __global__ void k_filt_top_team(const T* __restrict__ elems, int64_t n, const T* __restrict__ x0m,
                                 const T* __restrict__ x0L, T* __restrict__ states) {
+  grid_begin(elems, x0m, x0L, states);
   using WS = FiltTeamWs<T, D>;
   POF_TEAM_PROLOGUE(WS)
   if (t != 0) return;
@@ -260,6 +263,7 @@ __global__ void k_filt_top_team(const T* __restrict__ elems, int64_t n, const T*
 // Smoother up-sweep at level l >= 1.
 template <typename T, int D, int TS>
 __global__ void k_smo_reduce_team(const T* __restrict__ in, int64_t nin, int C, T* __restrict__ out, int64_t nout) {
+  grid_begin(in, out);
   using WS = SmoTeamWs<T, D>;
   POF_TEAM_PROLOGUE(WS)
   if (t >= nout) return;
@@ -281,6 +285,7 @@ __global__ void k_smo_reduce_team(const T* __restrict__ in, int64_t nin, int C, 
 template <typename T, int D, int TS>
 __global__ void k_smo_down_team(const T* __restrict__ elems, int64_t n, int C, const T* __restrict__ ends_up,
                                 int64_t nup, T* __restrict__ ends) {
+  grid_begin(elems, ends_up, ends);
   using WS = SmoTeamWs<T, D>;
   POF_TEAM_PROLOGUE(WS)
   if (t >= nup) return;
@@ -305,6 +310,7 @@ __global__ void k_smo_down_team(const T* __restrict__ elems, int64_t n, int C, c
 template <typename T, int D, int TS>
 __global__ void k_smo_top_team(const T* __restrict__ elems, int64_t n, const T* __restrict__ mT,
                                const T* __restrict__ LT, T* __restrict__ ends) {
+  grid_begin(elems, mT, LT, ends);
   using WS = SmoTeamWs<T, D>;
   POF_TEAM_PROLOGUE(WS)
   if (t != 0) return;
