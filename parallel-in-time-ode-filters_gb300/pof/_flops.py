@@ -3,14 +3,15 @@
 Counts follow the loops of the kernels: an FMA is 2 flops; add, multiply,
 divide, square root and log are 1.  They are the algorithmic work of each
 kernel -- the operations it performs, the structural zeros it skips not
-counted (a few products over a triangular factor that the team kernels run
-dense are counted at their triangular size, mm_lowerB, so the figure errs
-low) -- and the numerator of its achieved-FLOP/s figure.  The thread-per-
-chunk level 0 (D < 6, csrc/pof_ops.cuh) runs the dense loops; the team
-kernels (level 0 from D = 6 on, every level >= 1, csrc/pof_team.cuh) skip the
-zeros of the lower-triangular right blocks of the triangularizations, the
-zero columns of the noiseless update and the zero blocks of the IWP
-transition matrix (structured=True).  ``reference_step_flops`` is the work
+counted -- and the numerator of its achieved-FLOP/s figure.  structured=True
+(level 0 from D = 6 on, csrc/pof_team.cuh) is the IWP prior with exact
+observations of the EK1 model, as a solve has it: block-diagonal F, block
+staircase in the predicted factor's triangularization, D - d columns in the
+factor of an updated state, observation rows that end at the last derivative
+of order one.  The thread-per-chunk level 0 (D < 6, csrc/pof_ops.cuh) is
+counted as the general model's dense loops: it skips the same zeros, so the
+figures for it err high.
+``reference_step_flops`` is the work
 per step and IEKS iteration of the reference's own formulation (per-step
 elements, ~2 combines per element in the associative scan, sigma^2/NLL pass).
 """
@@ -31,6 +32,17 @@ def tria(M, NC, MB=0, wlow=0, ncut=None):
         f += 2 * t + 2 + 1 + 3 + t  # |x|^2, nrm (fma + sqrt), beta/tau/scal, scale tail
         rows = (M - j - 1) + MB
         f += rows * (4 * t + 2)
+    return f
+
+
+def lq(M, tail, MB=0):
+    """t_lq of csrc/pof_team.cuh: reflector j of M combines the pivot with
+    tail(j) columns, over the rows below it and MB more."""
+    f = 0
+    for j in range(M):
+        t = tail(j)
+        if t > 0:
+            f += 2 * t + 8 + (M - j - 1 + MB) * (4 * t + 3)  # |x|^2, scalars, rows
     return f
 
 
@@ -61,18 +73,32 @@ def trsm(M, NR):
     return NR * M * (M - 1) + M * NR + M
 
 
+def _predict(D, d, smooth):
+    """tria([QL | F L]) with L's D - d columns; with the smoother's rows [0 | L]."""
+    Q, nl = D // d, D - d if d < D else D
+    return mm_f(D, nl, d) + lq(D, lambda j: min((j // Q + 1) * Q, nl), D if smooth else 0)
+
+
+def _psi(D, d):
+    """tria([[H Lp], [Lp]]): H's columns end at the last derivative of order 1."""
+    h = (d - 1) * (D // d) + 2
+    return 2 * d * h * D + lq(min(h, D + d), lambda j: h - j - 1, D + d - min(h, D + d))
+
+
 def kf_step(D, d, smooth, structured=None):
     st = D >= 6 if structured is None else structured
-    w = D if st else 0
-    f = mm_f(D, D, d) if st else mm_lowerB(D, D)
-    if smooth:
-        f += tria(D, 2 * D, MB=D, wlow=w) + tria(D, D)
-        f += trsm(D, D) + mv(D, D) + D
+    if st:
+        f = _predict(D, d, smooth) + _psi(D, d) + mm_f(D, 1, d)
+        if smooth:
+            f += trsm(D, D) + mv(D, D) + D
     else:
-        f += tria(D, 2 * D, wlow=w)
-    f += mm_f(D, 1, d) if st else mv(D, D)  # predicted mean
-    f += mm_lowerB(d, D)  # H Lp (Lp lower)
-    f += tria(D + d, D + d, ncut=D if st else None)
+        f = mm_lowerB(D, D) + mv(D, D)
+        if smooth:
+            f += tria(D, 2 * D, MB=D) + tria(D, D)
+            f += trsm(D, D) + mv(D, D) + D
+        else:
+            f += tria(D, 2 * D)
+        f += mm_lowerB(d, D) + tria(D + d, D + d)  # H Lp (Lp lower), Psi
     f += mv(d, D) + d  # r
     f += 2 * trsv(d)
     f += d * (2 + 2 + 1)  # ssq, y^2, log
@@ -83,37 +109,35 @@ def kf_step(D, d, smooth, structured=None):
 
 def cond_fold_step(D, d, structured=None):
     st = D >= 6 if structured is None else structured
-    f = (mm_f(D, D, d) + tria(D, 2 * D, wlow=D)) if st else (mm_lowerB(D, D) + tria(D, 2 * D))
-    f += mm_lowerB(d, D) + tria(D + d, D + d, ncut=D if st else None)
-    f += (mm_f(D, D, d) + mm_f(D, 1, d)) if st else (mm(D, D, D) + mv(D, D))  # F A, F b
+    if st:
+        f = _predict(D, d, False) + _psi(D, d) + mm_f(D, D, d) + mm_f(D, 1, d)
+        f += lq(D, lambda j: d)  # [Z | W^T]
+    else:
+        f = mm_lowerB(D, D) + tria(D, 2 * D) + mm_lowerB(d, D) + tria(D + d, D + d)
+        f += mm(D, D, D) + mv(D, D)  # F A, F b
+        f += tria(D, D + d)
     f += mm(d, D, D) + mv(d, D) + d  # H FA, H Fb + c
     f += trsm(d, D) + trsv(d)
     f += D * D * 2 * d + D * 2 * d + D * 2 * d  # A, b, eta
-    f += tria(D, D + d)
     return f
 
 
 def filt_combine(D):
-    f = mm(D, D, D)  # U1^T Z2
-    f += tria(D, 2 * D, MB=D, wlow=D) + tria(D, D)
-    f += mm(D, D, D) + trsm(D, D)  # M
-    f += trsm(D, D)  # Mu
-    f += mm(D, D, D)  # MX
-    f += mm(D, D, D) + D * D  # A
-    f += 2 * mv(D, D) + D + mv(D, D) + mv(D, D) + D + mv(D, D) + D  # b
-    f += trsm(D, D)  # e
-    f += 2 * mv(D, D) + D + mv(D, D) + mv(D, D) + D + mv(D, D) + D  # eta
-    f += tria(D, 2 * D, wlow=D)  # U
-    f += mm(D, D, D) + tria(D, 2 * D, wlow=D)  # Z
+    def tail(_):
+        return D
+    f = mm(D, D, D) + lq(D, tail, D)  # U1^T Z2, Xi
+    f += mm(D, D, D) + 2 * trsm(D, D)  # M, Mu
+    f += 2 * mm(D, D, D)  # A = (A2 - M^T Xi21^T) A1
+    f += 5 * (mv(D, D) + D) * 2  # b, eta
+    f += lq(D, tail)  # U
+    f += mm(D, D, D) + lq(D, tail)  # Z
     return f
 
 
 def filt_apply(D):
-    f = mm(D, D, D) + tria(D, 2 * D, MB=D, wlow=D)
-    f += mm(D, D, D) + trsm(D, D) + trsm(D, D)
-    f += 2 * mv(D, D) + D + mv(D, D) + mv(D, D) + D + mv(D, D) + D
-    f += tria(D, 2 * D, wlow=D)
-    return f
+    def tail(_):
+        return D
+    return 2 * mm(D, D, D) + lq(D, tail, D) + 2 * trsm(D, D) + 5 * (mv(D, D) + D) + lq(D, tail)
 
 
 def smooth_combine(D, structured=True):
@@ -227,11 +251,13 @@ def kernel_bytes(n, D, d, esz=8):
 
 
 # ---------------------------------------------------------------------------
-# the dense path (csrc/pof_dense_sched.h): flops as its launches run them,
+# the dense path (csrc/pof_dense_sched.h): flops of the schedule's operations,
 # GEMM M N K -> 2 M N K, tria of an m x n block -> 2 m^2 n - 2/3 m^3 (the
 # Householder LQ's arithmetic, without the compact-WY overhead), triangular
-# solve M x K -> M^2 K.  Per step and filter + smoother pass; the top levels
-# (P - 1 sequential combines each way) are added per chunk.
+# solve M x K -> M^2 K.  The launches skip the zeros of triangular operands,
+# which are counted here, so a rate from these counts errs high.  Per step and
+# filter + smoother pass; the top levels (P - 1 combines each way) are added
+# per chunk.
 # ---------------------------------------------------------------------------
 
 
