@@ -196,10 +196,8 @@ def plan_levels(n, D=4, C0=None, Cg=2, top=2):
     """The level sizes libpof uses (csrc/pof_plan.h make_plan)."""
     if C0 is None:
         lanes = l0_lanes(D)
-        C0 = 4 if lanes == 1 else 2
-        target = 16384 if lanes == 1 else max(1024, 65536 // lanes)
-        while C0 < 64 and n // C0 > target:
-            C0 *= 2
+        target = 19456 if lanes == 1 else 48640 // lanes
+        C0 = min(max(-(-n // target), 4 if lanes == 1 else 2), 64)
     cnt = [None, (n + C0 - 1) // C0]
     while cnt[-1] > top:
         cnt.append((cnt[-1] + Cg - 1) // Cg)
