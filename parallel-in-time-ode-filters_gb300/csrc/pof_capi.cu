@@ -65,11 +65,11 @@ int env_int(const char* name, int dflt = 0) {
 Plan plan_for(int dtype, int64_t n, int D, int DY, bool solver) {
   const int C0 = env_int("POF_C0"), Cg = env_int("POF_CG"), ks = env_int("POF_KS", 0);
   const bool narrow = env_int("POF_TEAM_WIDE_L0") != 0;
-  const Plan p = make_plan(n, D, DY, esz(dtype), solver, C0, Cg, narrow, ks);
-  // A pass that only longer chunks bring under the scratch of the
+  const Plan p = make_plan(n, D, DY, esz(dtype), solver, C0 > 0 ? C0 : even_c0(n, l0_lanes(D, !narrow)), Cg, narrow, ks);
+  // A pass that only pick_c0's chunks bring under the scratch of the
   // allocation-free entry point takes those.
   if (!solver && C0 <= 0 && p.total > POF_NOALLOC_SCRATCH_BYTES) {
-    const Plan q = make_plan(n, D, DY, esz(dtype), solver, long_c0(n, l0_lanes(D, !narrow)), Cg, narrow, ks);
+    const Plan q = make_plan(n, D, DY, esz(dtype), solver, 0, Cg, narrow, ks);
     if (q.total <= POF_NOALLOC_SCRATCH_BYTES) return q;
   }
   return p;

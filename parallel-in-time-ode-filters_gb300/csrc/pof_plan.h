@@ -52,33 +52,33 @@ inline int l0_lanes(int D, bool narrow) { return D >= 6 ? team_lanes(D, narrow) 
 // instruction); levels >= 1 are latency-bound (wide teams finish a combine
 // sooner).  Measured on GB300: D = 8, narrow level 0 is 2x faster than wide.
 
-// Chunk length of level 0: as many chunks as the chip runs at once in even
-// shares, so that no SM is left with one more than the others at the end.
-// A thread per chunk: one warp on each of the 4 sub-partitions of 152 SMs, 19456
-// chunks.  Teams: 5 blocks of 64 threads per SM (what shared memory lets the
-// down-sweep run), 6080 chunks of 8 lanes, 3040 of 16.  Short grids take short
-// chunks for the latency of a chunk's chain, but not below 4 and 2, from where
-// on the tree costs more.  Measured, ms, powers of two up to 16384 and 65536 /
-// lanes chunks before / this: logistic q = 3 solves of 150000 steps 17.9 / 15.2
-// (16, 8 steps), of 262143 20.9 / 20.1 (16, 14), of 90000 13.3 / 12.7 (8, 5);
-// FitzHugh-Nagumo q = 3 passes of 65535 steps 5.89 / 5.45 (8, 11), of 60000
-// 5.65 / 5.07 (8, 10), q = 2 of 30000 2.21 / 2.09 (4, 5); Van der Pol q = 3
-// solve of 16000 19.8 / 18.0 (2, 3); rigid body (D = 12) of 7000 30.1 / 26.6
-// (2, 3).
+// Chunk length of level 0 when make_plan is given none: the next power of two
+// with at most ~16k lanes of chunks (threads) or 65536 / lanes chunks (teams).
+// Longer chunks than even_c0's in places, and then less workspace.
 inline int pick_c0(int64_t n, int lanes) {
-  const int lo = lanes == 1 ? 4 : 2;
-  const int64_t target = lanes == 1 ? 19456 : 48640 / lanes;
-  const int64_t c = (n + target - 1) / target;
-  return (int)(c < lo ? lo : (c > 64 ? 64 : c));
-}
-
-// The next power of two up to 16384 (threads) or 65536 / lanes (teams) chunks:
-// longer chunks than pick_c0's in places, for less workspace.
-inline int long_c0(int64_t n, int lanes) {
   int c = lanes == 1 ? 4 : 2;
   const int64_t target = lanes == 1 ? 16384 : (65536 / lanes > 1024 ? 65536 / lanes : 1024);
   while (c < 64 && n / c > target) c *= 2;
   return c;
+}
+
+// Chunk length of the passes and solves: as many chunks as the chip runs at
+// once in even shares, so that no SM is left with one more than the others at
+// the end.  A thread per chunk: one warp on each of the 4 sub-partitions of 152
+// SMs, 19456 chunks.  Teams: 5 blocks of 64 threads per SM (what shared memory
+// lets the down-sweep run), 6080 chunks of 8 lanes, 3040 of 16.  Short grids take
+// short chunks for the latency of a chunk's chain, but not below 4 and 2, from
+// where on the tree costs more.  Measured, ms, pick_c0 / this (steps per chunk):
+// logistic q = 3 solves of 150000 steps 17.9 / 15.2 (16, 8), of 262143 20.9 /
+// 20.1 (16, 14), of 90000 13.3 / 12.7 (8, 5); FitzHugh-Nagumo q = 3 passes of
+// 65535 steps 5.89 / 5.45 (8, 11), of 60000 5.65 / 5.07 (8, 10), q = 2 of 30000
+// 2.21 / 2.09 (4, 5); Van der Pol q = 3 solve of 16000 19.8 / 18.0 (2, 3); rigid
+// body (D = 12) of 7000 30.1 / 26.6 (2, 3).
+inline int even_c0(int64_t n, int lanes) {
+  const int lo = lanes == 1 ? 4 : 2;
+  const int64_t target = lanes == 1 ? 19456 : 48640 / lanes;
+  const int64_t c = (n + target - 1) / target;
+  return (int)(c < lo ? lo : (c > 64 ? 64 : c));
 }
 
 inline size_t align_up(size_t x) { return (x + 255) & ~size_t(255); }

@@ -193,7 +193,7 @@ def l0_lanes(D):
 
 
 def plan_levels(n, D=4, C0=None, Cg=2, top=2):
-    """The level sizes libpof uses (csrc/pof_plan.h make_plan)."""
+    """The level sizes libpof uses (csrc/pof_plan.h even_c0, make_plan)."""
     if C0 is None:
         lanes = l0_lanes(D)
         target = 19456 if lanes == 1 else 48640 // lanes
