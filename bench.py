@@ -69,7 +69,7 @@ MAXITERS = 10_000  # the reference's default (pof/solver.py:12)
 # (dram__bytes_read.sum + dram__bytes_write.sum from one ncu capture of
 # k_filt_l0_down_team<double, 8, 2, 8> on this workload; not measured by the
 # bench run itself)
-NCU_TRAFFIC = {("fhn_q3_N65536", "filt_l0_down"): 16.334080e6 + 49.652480e6}
+NCU_TRAFFIC = {("fhn_q3_N65536", "filt_l0_down"): 15.318016e6 + 52.400128e6}
 
 
 def workload_config(workload):
