@@ -97,12 +97,13 @@ __device__ __forceinline__ void t_mv(const Team<TS>& tm, const T* A, const T* x,
 // row's own squared norm is therefore one more of the dot products (entry 0),
 // the scalars are computed by every lane instead of on one and broadcast (the
 // same instructions), the tail is not rescaled, and one team barrier per
-// reflector is left.  An exactly zero tail (LAPACK's tau = 0) skips the
-// reflector.
+// reflector is left where a row belongs to one lane.  An exactly zero tail
+// (LAPACK's tau = 0) skips the reflector.
 //
 // Entries (the reflector's row and the rows below) are spread over RS row
 // slots; a team with more lanes than entries gives each row G = TS / RS
-// lanes, which take every G-th tail column.
+// lanes, which take every G-th tail column.  All of them need the row's pivot
+// entry and the first writes it, so a second barrier separates the two.
 // ---------------------------------------------------------------------------
 template <int R>
 struct Pow2Ceil {
@@ -160,11 +161,13 @@ __device__ __forceinline__ void t_lq(const Team<TS>& tm, T* X, T* Y, const Tail&
     const T alpha = xj[j];
     const int ne = M - j + MB;  // entries of this reflector; pass p has one if p RS < ne
     T* row[NP];
+    T piv[NP];
     Acc<T> dot[NP];
 #pragma unroll
     for (int p = 0; p < NP; ++p) {
       const int e = slot + p * RS;
       row[p] = e >= ne ? X + j * LD : (e < M - j ? X + (j + e) * LD : Y + (e - (M - j)) * LDY);
+      piv[p] = row[p][j];
       dot[p] = Acc<T>(T(0));
     }
     if constexpr (Tail::count > 0 && Tail::count % G == 0) {
@@ -191,6 +194,8 @@ __device__ __forceinline__ void t_lq(const Team<TS>& tm, T* X, T* Y, const Tail&
     const T xn2 = __shfl_sync(tm.mask, dot[0].value(), src);
     pj = -1;
     if (is_zero(xn2)) continue;
+    // a row's G lanes have read its pivot entry before the first of them writes it
+    if constexpr (G > 1) tm.sync();
     const Reflector<T> h(alpha, xn2);
     pend = h.beta;
     pj = j;
@@ -200,7 +205,7 @@ __device__ __forceinline__ void t_lq(const Team<TS>& tm, T* X, T* Y, const Tail&
       if (e == 0 || e >= ne) continue;
       T* xi = row[p];
       T ws;
-      const T a = h.row(xi[j], dot[p].value(), ws);
+      const T a = h.row(piv[p], dot[p].value(), ws);
       if (ph == 0) xi[j] = a;
       if constexpr (Tail::count > 0 && Tail::count % G == 0) {
 #pragma unroll

@@ -1,0 +1,145 @@
+"""The team kernels (csrc/pof_team*.cuh, pof_seq.cuh) on the host, every thread
+of a block a fiber (tests/team_cpu.cpp), no GPU: results must not depend on the
+order in which the lanes run between two barriers, nor on what shared memory
+and scratch held before, and agree with the oracle."""
+
+import ctypes
+import os
+import re
+import shutil
+import subprocess
+
+import numpy as np
+import pytest
+
+from oracle import core, filtsmooth as ofs
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CSRC = os.path.join(ROOT, "parallel-in-time-ode-filters_gb300", "csrc")
+# PTX statements and shared-memory declarations of the headers, and their host forms
+SUBST = [
+    (r'asm\("rcp\.approx\.ftz\.f32 %0, %1;" : "=f"\(y\) : "f"\(x\)\);', "y = 1.0f / x;"),
+    (r'asm\("rsqrt\.approx\.ftz\.f32 %0, %1;" : "=f"\(y\) : "f"\(x\)\);', "y = 1.0f / sqrtf(x);"),
+    (r'asm volatile\("[^"]*"(?: : "\+l"\(p\))?\s*::: ?"memory"\);', ""),
+    (r'asm volatile\("" : "\+l"\(p\)::"memory"\);', ""),
+    (r"extern __shared__ __align__\(16\) unsigned char smem_raw_\[\];", "unsigned char* smem_raw_ = host_smem;"),
+    (r"__shared__ ", "static "),
+]
+
+
+@pytest.fixture(scope="module")
+def lib(tmp_path_factory):
+    cxx = shutil.which("g++") or shutil.which("c++")
+    if cxx is None:
+        pytest.skip("no host C++ compiler")
+    d = tmp_path_factory.mktemp("team")
+    for name in os.listdir(CSRC):
+        if name.endswith((".cuh", ".h")):
+            with open(os.path.join(CSRC, name)) as f:
+                text = f.read()
+            for pat, rep in SUBST:
+                text = re.sub(pat, rep, text)
+            if name != "pof_dense.cuh":
+                assert "asm" not in re.sub(r"//.*", "", text), name
+            (d / name).write_text(text)
+    (d / "cuda_runtime.h").write_text("")
+    so = str(d / "team_cpu.so")
+    subprocess.run([cxx, "-std=c++17", "-O1", "-ffp-contract=off", "-w", "-shared", "-fPIC", "-I", str(d),
+                    os.path.join(ROOT, "tests", "team_cpu.cpp"), "-o", so], check=True, capture_output=True, text=True)
+    return ctypes.CDLL(so)
+
+
+def _p(a):
+    return None if a is None else a.ctypes.data_as(ctypes.c_void_p)
+
+
+def _model(D, d, n, prior, noise, per_step, seed, dtype):
+    rng = np.random.default_rng(seed)
+    q = D // d - 1
+    if prior:
+        F, QL = core.preconditioned_discretize(d, q)
+    else:
+        F = np.eye(D) + 0.1 * rng.standard_normal((D, D))
+        QL = 0.5 * np.eye(D) + 0.1 * rng.standard_normal((D, D))
+    H = rng.standard_normal((n, d, D))
+    if prior:  # observation rows of the solver: the first two columns of each block
+        keep = np.zeros(D, bool)
+        keep[:: q + 1] = keep[1 :: q + 1] = True
+        H[:, :, ~keep] = 0.0
+    R = {"none": None, "some": 0.2 * np.tril(rng.standard_normal((n, d, d)) + 2 * np.eye(d))
+         * (np.arange(n) % 3 == 1)[:, None, None]}[noise]
+    if per_step:
+        F, QL = np.tile(F, (n, 1, 1)), np.tile(QL, (n, 1, 1))
+    c = rng.standard_normal((n, d))
+    m0, L0 = rng.standard_normal(D), 0.3 * np.eye(D) + 0.1 * rng.standard_normal((D, D))
+    return [None if x is None else np.ascontiguousarray(x, dtype) for x in (F, QL, H, c, R, m0, L0)]
+
+
+def _pass(lib, dtype, order, poison, n, C0, D, d, model):
+    F, QL, H, c, R, m0, L0 = model
+    out = [np.zeros((n + 1, D), dtype), np.zeros((n + 1, D, D), dtype), np.zeros((n + 1, D), dtype),
+           np.zeros((n + 1, D, D), dtype), np.zeros(4)]
+    rc = lib.team_cpu_pass(int(dtype == np.float32), order, poison, ctypes.c_int64(n), C0, D, d, _p(F), _p(QL),
+                           ctypes.c_int64(D * D if F.ndim == 3 else 0), _p(H), _p(c), _p(R), _p(m0), _p(L0),
+                           *[_p(x) for x in out])
+    assert rc == 0 and not lib.team_cpu_deadlock()
+    return out
+
+
+def _sequential(lib, dtype, order, poison, n, D, d, model, field=0, params=None, p0=0.0, p1=0.0):
+    F, QL, H, c, R, m0, L0 = model
+    out = [np.zeros((n + 1, D), dtype), np.zeros((n + 1, D, D), dtype), np.zeros(3)]
+    rc = lib.team_cpu_sequential(int(dtype == np.float32), order, poison, ctypes.c_int64(n), D, d, _p(F), _p(QL),
+                                 ctypes.c_int64(D * D if F.ndim == 3 else 0), _p(H), _p(c), _p(R), field, _p(params),
+                                 ctypes.c_double(p0), ctypes.c_double(p1), _p(m0), _p(L0), *[_p(x) for x in out])
+    assert rc == 0 and not lib.team_cpu_deadlock()
+    return out
+
+
+ORDERS = [(0, 0xff), (1, 0xff), (2, 0xff), (3, 0x3f), (0, 0)]  # (order of the lanes, what memory held)
+
+
+def _same(a, b):
+    return all(x.tobytes() == y.tobytes() for x, y in zip(a, b))
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("D,d,n,C0,prior,noise,per_step", [
+    (6, 2, 19, 2, True, "none", False), (8, 2, 13, 3, True, "none", False), (8, 2, 9, 2, True, "some", True),
+    (9, 3, 11, 2, False, "some", False), (12, 3, 7, 1, True, "none", True)])
+def test_pass_does_not_depend_on_lane_order(lib, dtype, D, d, n, C0, prior, noise, per_step):
+    model = _model(D, d, n, prior, noise, per_step, D + n, dtype)
+    ref = _pass(lib, dtype, *ORDERS[0], n, C0, D, d, model)
+    for o in ORDERS[1:]:
+        assert _same(ref, _pass(lib, dtype, *o, n, C0, D, d, model)), o
+    if dtype == np.float64:
+        F, QL, H, c, R, m0, L0 = model
+        rep = lambda A: np.broadcast_to(A, (n, D, D))  # noqa: E731
+        (om, oL), nll, _, _ = ofs.sequential_linear_filtsmooth(
+            (m0, L0), (rep(F), rep(QL)), (H, c, np.zeros((n, d, d)) if R is None else R))
+        assert np.abs(ref[2] - om).max() <= 1e-8 * np.abs(om).max()
+        cov = lambda L: L @ np.swapaxes(L, -1, -2)  # noqa: E731
+        assert np.abs(cov(ref[3]) - cov(oL)).max() <= 1e-8 * np.abs(cov(oL)).max()
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("D,d,prior,noise,per_step", [
+    (2, 1, True, "none", False), (4, 1, True, "some", True), (8, 2, True, "none", False), (9, 3, False, "some", True),
+    (12, 3, True, "none", False)])
+def test_sequential_twin_does_not_depend_on_lane_order(lib, dtype, D, d, prior, noise, per_step):
+    n = 6
+    model = _model(D, d, n, prior, noise, per_step, D + 10 * d, dtype)
+    ref = _sequential(lib, dtype, *ORDERS[0], n, D, d, model)
+    for o in ORDERS[1:]:
+        assert _same(ref, _sequential(lib, dtype, *o, n, D, d, model)), o
+
+
+def test_sequential_ekf_does_not_depend_on_lane_order(lib):
+    D, d, n = 8, 2, 6  # Van der Pol, q = 3
+    F, QL, _, _, _, m0, L0 = _model(D, d, n, True, "none", False, 3, np.float64)
+    params = np.array([1.0])
+    args = (n, D, d, (F, QL, None, None, None, m0, L0), 3, params, 0.1, 0.3)
+    ref = _sequential(lib, np.float64, *ORDERS[0], *args)
+    assert all(np.isfinite(x).all() for x in ref)
+    for o in ORDERS[1:]:
+        assert _same(ref, _sequential(lib, np.float64, *o, *args)), o
