@@ -789,8 +789,9 @@ __device__ __forceinline__ void t_psi(const Team<TS>& tm, WS& w, StepObs ob) {
     for (int k = 0; k < ob.h1; ++k) s.mul_add(w.H[i * L1 + k], w.X[k * L2 + j]);
     w.P[i * LP + j] = s.value();
   }
-  if (!ob.rzero)
-    for (int idx = tm.r; idx < DY * DY; idx += TS) w.P[(idx / DY) * LP + D + idx % DY] = w.R[idx];
+  // (with more observations than states Psi11 reaches into these columns)
+  if (!ob.rzero || DY > D)
+    for (int idx = tm.r; idx < DY * DY; idx += TS) w.P[(idx / DY) * LP + D + idx % DY] = ob.rzero ? T(0) : w.R[idx];
   for (int idx = tm.r; idx < D * DP; idx += TS) {
     const int i = idx / DP, j = idx % DP;
     w.P[(DY + i) * LP + j] = (j <= i) ? w.X[i * L2 + j] : T(0);
