@@ -620,8 +620,9 @@ __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(256)
 // divisions (about 100 FP64 instructions in double): 415 us per panel of 32
 // rows x 256 columns in double, 137 us at 768 columns in float.
 //
-// double: reflectors unnormalized (v = (u, x), coefficient kap); float:
-// v = (1, scal x), coefficient tau (Reflector).  Writes V (nbb x np), T (nb x
+// double: reflectors unnormalized (v = (u, x), coefficient kap; a row beyond
+// 2^+-500 is scaled before it becomes one); float: v = (1, scal x), coefficient
+// tau (Reflector).  Writes V (nbb x np), T (nb x
 // nb, upper triangular, H_0 .. H_{nbb-1} = I - V^T T V) and, when TV is given,
 // T V.
 // ---------------------------------------------------------------------------
@@ -630,11 +631,13 @@ struct PanelCoef;  // what a reflector's row update and its V row need
 template <>
 struct PanelCoef<double> {
   double beta, u, kap;
-  __device__ __forceinline__ void set(double alpha, double xn2) {
+  template <typename F>
+  __device__ __forceinline__ void set(double alpha, double xn2, F&& scale) {
     if (is_zero(xn2)) {
       beta = alpha, u = 0.0, kap = 0.0;
     } else {
-      const Reflector<double> h(alpha, xn2);
+      Reflector<double> h;
+      h.set(alpha, xn2, scale);
       beta = h.beta, u = h.u, kap = h.kap;
     }
   }
@@ -649,7 +652,10 @@ struct PanelCoef<double> {
 template <>
 struct PanelCoef<float> {
   float beta, t, scal;
-  __device__ __forceinline__ void set(float alpha, float xn2) { householder(alpha, xn2, beta, t, scal); }
+  template <typename F>
+  __device__ __forceinline__ void set(float alpha, float xn2, F&&) {
+    householder(alpha, xn2, beta, t, scal);
+  }
   __device__ __forceinline__ float row(float a, float dot, float& ws) const {
     const float w = t * fmaf(scal, dot, a);
     ws = w * scal;
@@ -731,7 +737,15 @@ __global__ void __launch_bounds__(NW * 32, (panel_ctas<T, NC>()))
       }
       s2 = warp_sum(s2);
       PanelCoef<T> h;
-      h.set(alpha, s2);
+      h.set(alpha, s2, [&](T sc) {  // (the same on every lane)
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+          x_[lane + 32 * c] = x[c] * sc;
+#pragma unroll
+          for (int s = 0; s < RPW; ++s)
+            if (s == js && (c > 0 || lane > j)) q[s][c] *= sc;
+        }
+      });
       if (lane == 0) co[j] = h;
     }
     __syncthreads();

@@ -145,12 +145,20 @@ __device__ __forceinline__ bool is_zero(float x) { return (__float_as_uint(x) <<
 // The same reflector with the tail x left as it is, so the squared norm can be
 // formed together with the dot products of the rows below and no pass scales
 // x: a row (a, y) with dot = y . x becomes (a - w, y - ws x), where
-//   double: H = I + kap v v^T, v = (u, x), u = alpha - beta, kap = 1 / (u beta):
-//     ws = -kap (u a + dot), w = u ws; ||(alpha, x)|| = h and
-//     1 / (u beta) = -1 / (a2 + |alpha| h) from single-precision seeds and one
+//   double: H = I - kap v v^T, v = (u, x), u = alpha - beta, kap = -1 / (u beta):
+//     ws = kap (u a + dot), w = u ws; ||(alpha, x)|| = h and
+//     kap = 1 / (a2 + |alpha| h) from single-precision seeds and one
 //     third-order correction each (as rsqrt_nr and rcp_nr), 11 FP64
 //     instructions of scalars and 2 per row; measured alone on a warp
-//     1399 cycles with 64-bit integer seeds one after the other;
+//     1399 cycles with 64-bit integer seeds one after the other.
+//     Beyond 2^+-1000 the squared norm's reciprocal leaves double's range although
+//     the reflector, which is that of s (alpha, x) but for beta, does not: there
+//     s = 2^-k brings the norm near 1, and `scale(s)` puts s x in place of x and
+//     of the dot products that were formed with it.  (As accurate as
+//     householder: what the square loses to underflow is lost to both.)  The
+//     rows that stay near 1 pay nothing for it; x left as it is, with a second u
+//     for the pivot's own update, cost the sequential smoother 3 %, a test of its
+//     own before the chain 6 %.
 //   float: w = tau (a + scal dot), ws = w scal (kap would leave float's range
 //     for tails below 1e-19).
 // For xn2 != 0 only.
@@ -160,7 +168,8 @@ struct Reflector;
 template <>
 struct Reflector<double> {
   double beta, u, kap;
-  __device__ __forceinline__ Reflector(double alpha, double xn2) {
+  template <typename F>
+  __device__ __forceinline__ void set(double alpha, double xn2, F&& scale) {
     const double a2 = fma(alpha, alpha, xn2);
     const int hi = __double2hiint(a2), ahi = __double2hiint(alpha) & 0x7fffffff;
     double h;
@@ -178,11 +187,21 @@ struct Reflector<double> {
       const double r = fma(-g, y, 1.0);
       h = fma(g, r * fma(r, 0.375, 0.5), g);
       const double s = fma(-fma(fabs(alpha), h, a2), z, 1.0);
-      kap = fma(z, fma(s, s, s), z);  // -1 / (u beta)
+      kap = fma(z, fma(s, s, s), z);
+      finish(alpha, h);
     } else {
-      h = sqrt(a2);
-      kap = 1.0 / fma(fabs(alpha), h, a2);
+      const int e = (hi >> 20) & 0x7ff;
+      const int k = e == 0 ? -524 : (e - 1023) >> 1;
+      const double s = __hiloint2double((1023 - k) << 20, 0), back = __hiloint2double((1023 + k) << 20, 0);
+      const double b2 = a2 * s * s;
+      h = sqrt(b2);
+      kap = 1.0 / fma(fabs(alpha * s), h, b2);
+      finish(alpha * s, h);
+      beta *= back;
+      scale(s);
     }
+  }
+  __device__ __forceinline__ void finish(double alpha, double h) {
     // sign(0) = +, so alpha = -0 reflects like +0
     const bool neg = __double2hiint(alpha) < 0 && !is_zero(alpha);
     beta = neg ? h : __hiloint2double(__double2hiint(h) ^ 0x80000000, __double2loint(h));
@@ -198,7 +217,10 @@ struct Reflector<double> {
 template <>
 struct Reflector<float> {
   float beta, tau, scal;
-  __device__ __forceinline__ Reflector(float alpha, float xn2) { householder(alpha, xn2, beta, tau, scal); }
+  template <typename F>
+  __device__ __forceinline__ void set(float alpha, float xn2, F&&) {
+    householder(alpha, xn2, beta, tau, scal);
+  }
   __device__ __forceinline__ float row(float a, float dot, float& ws) const {
     const float w = tau * fmaf(scal, dot, a);
     ws = w * scal;
@@ -242,6 +264,7 @@ struct Acc<double> {
   __device__ __forceinline__ void join(unsigned mask, int o, int width) {
     h += __shfl_xor_sync(mask, h, o, width);
   }
+  __device__ __forceinline__ void scale(double s) { h *= s; }
   __device__ __forceinline__ double plus(double v) const { return v + h; }   // v + the sum
   __device__ __forceinline__ double from(double v) const { return v - h; }   // v - the sum
   __device__ __forceinline__ double value() const { return h; }
@@ -266,6 +289,7 @@ struct Acc<float> {
     add(h2);
     l = __fadd_rn(l, l2);
   }
+  __device__ __forceinline__ void scale(float s) { h *= s, l *= s; }
   __device__ __forceinline__ float plus(float v) const {
     Acc<float> a = *this;
     a.add(v);
@@ -338,7 +362,11 @@ __device__ __forceinline__ void lq_rows(T* X) {
 #pragma unroll
     for (int k = j + 1; k < NC; ++k) xn2 = fma(xj[k], xj[k], xn2);
     if (!is_zero(xn2)) {
-      const Reflector<T> h(xj[j], xn2);
+      Reflector<T> h;
+      h.set(xj[j], xn2, [&](T s) {
+#pragma unroll
+        for (int k = j + 1; k < NC; ++k) xj[k] *= s;
+      });
       xj[j] = h.beta;
 #pragma unroll
       for (int i = j + 1; i < MX; ++i) {
@@ -358,7 +386,7 @@ __device__ __forceinline__ void lq_rows(T* X) {
 // [P | W], P lower triangular M x M, W with NW columns, over MB rows [Yp | Yw]:
 // P becomes L with L L^T = P P^T + W W^T, the rows below are multiplied by the
 // same orthogonal matrix.  Q > 0: row j of W ends with column (j / Q + 1) Q - 1
-// (W = F S, F block-diagonal, S lower triangular).  W is left as it is.
+// (W = F S, F block-diagonal, S lower triangular).  W must not be read after.
 template <typename T, int M, int NW, int MB, int Q, int LDP, int LDW, int LDYP, int LDYW>
 __device__ __forceinline__ void lq_pivot(T* P, T* W, T* Yp, T* Yw) {
 #pragma unroll
@@ -370,7 +398,12 @@ __device__ __forceinline__ void lq_pivot(T* P, T* W, T* Yp, T* Yw) {
     for (int k = 0; k < NW; ++k)
       if (k < nw) xn2 = fma(wj[k], wj[k], xn2);
     if (!is_zero(xn2)) {
-      const Reflector<T> h(P[j * LDP + j], xn2);
+      Reflector<T> h;
+      h.set(P[j * LDP + j], xn2, [&](T s) {
+#pragma unroll
+        for (int k = 0; k < NW; ++k)
+          if (k < nw) wj[k] *= s;
+      });
       P[j * LDP + j] = h.beta;
 #pragma unroll
       for (int i = j + 1; i < M + MB; ++i) {

@@ -82,8 +82,8 @@ __device__ __forceinline__ void t_mv(const Team<TS>& tm, const T* A, const T* x,
 // more rows Y in the same columns below: reflector j combines pivot column j
 // with row j's tail, so that afterwards the pivot block is L (lower
 // triangular, L L^T = P P^T + W W^T) and the rows Y have been multiplied by
-// the same orthogonal matrix.  The tails of the M rows are left as they are
-// (zero in exact arithmetic) and must not be read.
+// the same orthogonal matrix.  The tails of the M rows (zero in exact
+// arithmetic) are not cleared and must not be read.
 //
 // This is every triangularization of the filter and smoother: tria([X, L])
 // with a lower-triangular L is [P | W] = [L | X] (TailFixed), a general
@@ -157,7 +157,7 @@ __device__ __forceinline__ void t_lq(const Team<TS>& tm, T* X, T* Y, const Tail&
     if (kb >= ke) continue;
     tm.sync();
     if (pj >= 0 && tm.r == 0) X[pj * LD + pj] = pend;
-    const T* xj = X + j * LD;
+    T* xj = X + j * LD;
     const T alpha = xj[j];
     const int ne = M - j + MB;  // entries of this reflector; pass p has one if p RS < ne
     T* row[NP];
@@ -196,7 +196,14 @@ __device__ __forceinline__ void t_lq(const Team<TS>& tm, T* X, T* Y, const Tail&
     if (is_zero(xn2)) continue;
     // a row's G lanes have read its pivot entry before the first of them writes it
     if constexpr (G > 1) tm.sync();
-    const Reflector<T> h(alpha, xn2);
+    Reflector<T> h;
+    h.set(alpha, xn2, [&](T s) {  // (every lane has the same xn2)
+#pragma unroll
+      for (int p = 0; p < NP; ++p) dot[p].scale(s);
+      tm.sync();
+      for (int k = kb + tm.r; k < ke; k += TS) xj[k] *= s;
+      tm.sync();
+    });
     pend = h.beta;
     pj = j;
 #pragma unroll

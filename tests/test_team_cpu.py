@@ -152,3 +152,42 @@ def test_sequential_ekf_does_not_depend_on_lane_order(lib):
     assert all(np.isfinite(x).all() for x in ref)
     for o in ORDERS[1:]:
         assert _same(ref, _sequential(lib, np.float64, *o, *args)), o
+
+
+# rows of [P | W; Yp | Yw] scaled by powers of two: the factors scale with them
+SCALES = {np.float64: [0, -300, -495, -505, -512, -518, -530, 490, 505, 509], np.float32: [0, -40, -55, 50, 60]}
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("which", [0, 1, 2, 3])
+@pytest.mark.parametrize("rows", ["all", "first", "pivot zero"])
+def test_factorizations_of_rows_far_from_one(lib, dtype, which, rows):
+    """lq_rows, lq_pivot and t_lq (8 and 32 lanes) of a matrix with rows times
+    2^k equal the factors of the matrix itself with rows times 2^k.  Bound: 64
+    roundings of the entries' sums, and what the squared norm and the dot
+    products lose to underflow (units of the smallest number, 16 of them) where
+    they are small."""
+    M, MB, NW = 4, 3, 4
+    rng = np.random.default_rng(5)
+    X = rng.standard_normal((M + MB, M + NW))
+    X[:, :M] = np.tril(X[:, :M])
+    X[M:, :M] = 0.0 if which else X[M:, :M]
+    if rows == "pivot zero":  # the factors of an updated state
+        X[:M, :M][np.diag_indices(M)] = 0.0
+    X = X.astype(dtype)
+    tiny = {np.float64: -1074, np.float32: -149}[dtype]
+    for k in SCALES[dtype]:
+        s = np.ones((M + MB, 1), dtype)
+        s[: 1 if rows == "first" else M + MB] = np.ldexp(dtype(1), k)
+        out = []
+        for A in (X, X * s):
+            A = A.copy()
+            assert lib.team_cpu_factor(int(dtype == np.float32), which, 0, _p(A)) == 0
+            out.append(np.concatenate([np.tril(A[:M, :M]), A[M:, :M]]))  # L and the pivot columns below
+            if which:  # the rows below, all columns
+                out[-1] = np.concatenate([out[-1], A[M:, M:].reshape(-1, M)])
+        ref = out[0].astype(np.longdouble)
+        sc = np.concatenate([s, s[M:]]) if which else s
+        assert np.isfinite(out[1]).all(), k
+        err = np.abs(out[1].astype(np.longdouble) / sc - ref).max() / np.abs(ref).max()
+        assert err <= 64 * np.finfo(dtype).eps + 16 * 2.0 ** (tiny - 2 * k), (k, err)
