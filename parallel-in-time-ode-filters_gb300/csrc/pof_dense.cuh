@@ -344,6 +344,23 @@ __device__ inline T warp_sum(T v) {
   return v;
 }
 
+// householder() where alpha^2 may leave the type's range and the norm does not
+// (in float for |alpha| above 1.8e19; below 1e-19 it loses digits).
+template <typename T>
+__device__ __forceinline__ void panel_householder(T alpha, T xn2, T& beta, T& tau, T& scal) {
+  const T a2 = fma(alpha, alpha, xn2);
+  const T lo = sizeof(T) == 4 ? T(1.1754944e-38f) : T(2.2250738585072014e-308);
+  const T hi = sizeof(T) == 4 ? T(3.4028235e38f) : T(1.7976931348623157e308);
+  if ((a2 < lo || a2 > hi) && xn2 != T(0)) {
+    const T h = hypot(alpha, sqrt(xn2));
+    beta = alpha >= T(0) ? -h : h;
+    tau = (beta - alpha) / beta;
+    scal = T(1) / (alpha - beta);
+  } else {
+    householder(alpha, xn2, beta, tau, scal);
+  }
+}
+
 // One CTA per batch entry.  Dynamic shared memory: nbb * np elements.
 // V and TV are nbb x np, row-major, vbs elements apart per batch entry.
 // Row r of the panel belongs to warp r mod (warps): that warp applies every
@@ -380,7 +397,7 @@ __global__ void __launch_bounds__(512)
   for (int j = 0; j < nbb; ++j) {
     const T* pr = P + j * np;
     T bj, tj, scale;
-    householder(pr[j], nrm[j], bj, tj, scale);
+    panel_householder(pr[j], nrm[j], bj, tj, scale);
     if (t == 0) {
       tau[j] = tj;
       beta[j] = bj;
@@ -515,7 +532,7 @@ __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(256)
     T tot = T(0);
     for (int r = 0; r < CS; ++r) tot += *cluster.map_shared_rank(&sq[pb], r);
     T bj, tj, scale;
-    householder(*cluster.map_shared_rank(&al[pb], own), tot, bj, tj, scale);
+    panel_householder(*cluster.map_shared_rank(&al[pb], own), tot, bj, tj, scale);
     for (int c = t; c < wl; c += bd)
       if (c0 + c > j) pr[c] *= scale;
     if (t == 0) {
@@ -654,7 +671,7 @@ struct PanelCoef<float> {
   float beta, t, scal;
   template <typename F>
   __device__ __forceinline__ void set(float alpha, float xn2, F&&) {
-    householder(alpha, xn2, beta, t, scal);
+    panel_householder(alpha, xn2, beta, t, scal);
   }
   __device__ __forceinline__ float row(float a, float dot, float& ws) const {
     const float w = t * fmaf(scal, dot, a);

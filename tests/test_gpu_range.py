@@ -71,3 +71,28 @@ def test_passes_far_from_one(D, d, n, noise, dtype):
 @pytest.mark.parametrize("D,d,n,noise", [(40, 4, 9, True), (150, 10, 5, False)])
 def test_dense_passes_far_from_one(D, d, n, noise, dtype):
     _check(pfs.linear_filtsmooth, (D, d, n, dtype, noise), KS[dtype], dtype)
+
+
+@pytest.mark.parametrize("D,cluster", [(40, "1"), (1300, "0"), (1300, "1")])
+def test_dense_float32_pivots_whose_square_overflows(D, cluster, monkeypatch):
+    """The filter from an initial factor of 1e20 I with Q_L of order one: alpha^2 is
+    beyond float32, the norm is not.  D = 1300: beyond the register panels (2600
+    columns), one CTA or a cluster per matrix.  Bound: the float64 filter to 1e-3
+    of each array's largest entry."""
+    monkeypatch.setenv("POF_DENSE_CLUSTER", cluster)
+    n = 2
+    H = np.zeros((n, 1, D))
+    H[:, 0, 0] = 1.0
+    m0 = np.linspace(-1.0, 1.0, D)
+
+    def run(dtype):
+        out = pfs.linear_noiseless_filtering(MVNSqrt(T(m0, dtype), T(1e20 * np.eye(D), dtype)),
+                                             TransitionModel(T(np.eye(D), dtype), T(0.25 * np.eye(D), dtype)),
+                                             AffineModel(T(H, dtype), T(np.full((n, 1), -2.0), dtype), None))[0]
+        return out.mean.double(), out.chol.double() @ out.chol.double().mT
+
+    m, C = run(torch.float32)
+    m64, C64 = run(torch.float64)
+    assert torch.isfinite(m).all() and torch.isfinite(C).all()
+    assert float((m - m64).abs().max()) <= 1e-3 * float(m64.abs().max())
+    assert float((C - C64).abs().max()) <= 1e-3 * float(C64.max())
