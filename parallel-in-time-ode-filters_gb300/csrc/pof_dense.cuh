@@ -963,15 +963,16 @@ constexpr int kTrsmBlock = 32;
 template <typename T>
 __global__ void k_trsm_diag(int nbr, MV<T> L, bool upper, MV<T> B, int K, int64_t b0) {
   // (the diagonal inverted once per CTA: a division per column and row was
-  // most of this kernel's FP64 work)
-  __shared__ T Ls[kTrsmBlock][kTrsmBlock + 1];
+  // most of this kernel's FP64 work, a quotient is 3 instructions)
+  __shared__ T Ls[kTrsmBlock][kTrsmBlock + 1], rd[kTrsmBlock];
   const int t = threadIdx.x;
   const int64_t b = b0 + blockIdx.y;
   const T* Lb = L.p + b * L.bs;
   for (int l = t; l < nbr * nbr; l += blockDim.x) {
     const int i = l / nbr, j = l - i * nbr;
     const T v = Lb[i * L.rs + j * L.cs];
-    Ls[i][j] = i == j ? rcp(v) : v;
+    Ls[i][j] = v;
+    if (i == j) rd[i] = quotient_rcp(v);
   }
   __syncthreads();
   const int col = blockIdx.x * blockDim.x + t;
@@ -987,7 +988,7 @@ __global__ void k_trsm_diag(int nbr, MV<T> L, bool upper, MV<T> B, int K, int64_
         T v = x[i];
 #pragma unroll
         for (int j = 0; j < i; ++j) v -= Ls[i][j] * x[j];
-        x[i] = v * Ls[i][i];
+        x[i] = quotient(v, Ls[i][i], rd[i]);
       }
     }
   } else {
@@ -998,7 +999,7 @@ __global__ void k_trsm_diag(int nbr, MV<T> L, bool upper, MV<T> B, int K, int64_
 #pragma unroll
         for (int j = i + 1; j < kTrsmBlock; ++j)
           if (j < nbr) v -= Ls[i][j] * x[j];
-        x[i] = v * Ls[i][i];
+        x[i] = quotient(v, Ls[i][i], rd[i]);
       }
     }
   }

@@ -111,6 +111,26 @@ __device__ __forceinline__ T rcp(T a) {
     return T(1) / a;
 }
 
+// v / l with r = quotient_rcp(l): the product v r and one correction with its
+// exact residual, rounded as the division is (Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
+// Dev. 1990).  Divisors whose reciprocal the type may not hold have r = 0 and
+// are divided by.
+__device__ __forceinline__ double quotient_rcp(double l) {
+  return exp_in_range(__double2hiint(l)) ? rcp(l) : 0.0;
+}
+__device__ __forceinline__ float quotient_rcp(float l) {
+  return (unsigned)(((__float_as_int(l) >> 23) & 0xff) - 27) <= 200u ? rcp(l) : 0.f;
+}
+__device__ __forceinline__ bool is_finite(double x) { return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000; }
+__device__ __forceinline__ bool is_finite(float x) { return (__float_as_int(x) & 0x7f800000) != 0x7f800000; }
+template <typename T>
+__device__ __forceinline__ T quotient(T v, T l, T r) {
+  if (r == T(0)) return v / l;
+  const T q = v * r;
+  return is_finite(q) ? fma(fma(-q, l, v), r, q) : q;
+}
+
 // Scalars of the Householder reflector that maps (alpha, x), ||x||^2 = xn2,
 // onto (beta, 0), with LAPACK dlarfg's conventions: beta = -sign(alpha)
 // ||(alpha, x)|| (sign(0) = +1), tau = (beta - alpha) / beta, the tail

@@ -58,7 +58,7 @@ static inline float __fmaf_rn(float a, float b, float c) { return fmaf(a, b, c);
 // fibers
 // ---------------------------------------------------------------------------
 namespace emu {
-constexpr int kMax = 64;
+constexpr int kMax = 128;
 constexpr size_t kStack = 256 * 1024;
 enum Wait { RUN, WARP, BLOCK, DONE };
 struct Fiber {
@@ -193,6 +193,8 @@ static inline unsigned __reduce_add_sync(unsigned mask, unsigned v) { return war
 static inline int __any_sync(unsigned mask, int v) { return warp_fold(mask, v != 0, 2) != 0; }
 
 #include "pof_seq.cuh"  // and with it every team kernel
+#include "pof_dense_views.h"
+#include "trsm_diag.h"  // k_trsm_diag of pof_dense.cuh
 
 using namespace pof;
 
@@ -358,6 +360,22 @@ int team_cpu_sequential(int f32, int order, int poison, int64_t n, int D, int d,
   X(2, 1) X(4, 1) X(3, 4)
 #undef X
   return 1;
+}
+
+// B (nbr x K, row-major) <- L^{-1} B (upper: L upper triangular)
+void team_cpu_trsm_diag(int f32, int nbr, int upper, int K, void* L, void* B) {
+  auto go = [&](auto t) {
+    using T = decltype(t);
+    const dense::MV<T> Lv{(T*)L, nbr, 1, 0}, Bv{(T*)B, K, 1, 0};
+    blockDim.x = 128;
+    for (int b = 0; b < (K + 127) / 128; ++b) {
+      blockIdx.x = b, blockIdx.y = 0;
+      auto f = [&] { dense::k_trsm_diag<T>(nbr, Lv, upper != 0, Bv, K, 0); };
+      emu::run_block(128, 0, [](void* p) { (*static_cast<decltype(f)*>(p))(); }, &f);
+    }
+    blockIdx.x = 0;
+  };
+  f32 ? go(1.f) : go(1.0);
 }
 
 // M = 4 rows with 3 rows below and a tail of 4 columns, teams of 8 and 32 lanes

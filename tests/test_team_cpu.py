@@ -43,6 +43,10 @@ def lib(tmp_path_factory):
                 assert "asm" not in re.sub(r"//.*", "", text), name
             (d / name).write_text(text)
     (d / "cuda_runtime.h").write_text("")
+    dense = (d / "pof_dense.cuh").read_text()
+    kern = re.search(r"constexpr int kTrsmBlock = \d+;", dense).group(0) + "\n" + \
+        re.search(r"template <typename T>\n__global__ void k_trsm_diag\(.*?\n}\n", dense, re.S).group(0)
+    (d / "trsm_diag.h").write_text("namespace pof {\nnamespace dense {\n%s}\n}\n" % kern)
     so = str(d / "team_cpu.so")
     subprocess.run([cxx, "-std=c++17", "-O1", "-ffp-contract=off", "-w", "-shared", "-fPIC", "-I", str(d),
                     os.path.join(ROOT, "tests", "team_cpu.cpp"), "-o", so], check=True, capture_output=True, text=True)
@@ -191,3 +195,29 @@ def test_factorizations_of_rows_far_from_one(lib, dtype, which, rows):
         assert np.isfinite(out[1]).all(), k
         err = np.abs(out[1].astype(np.longdouble) / sc - ref).max() / np.abs(ref).max()
         assert err <= 64 * np.finfo(dtype).eps + 16 * 2.0 ** (tiny - 2 * k), (k, err)
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("upper", [0, 1])
+def test_dense_diagonal_solves_round_like_divisions(lib, dtype, upper):
+    """k_trsm_diag with a diagonal matrix: the quotients, bit for bit, also of
+    zeros, infinities and entries at the ends of the range."""
+    rng = np.random.default_rng(1)
+    n, K = 32, 200
+    big = {np.float64: 1000, np.float32: 120}[dtype]
+    x = (rng.standard_normal((n, K)) * np.exp2(rng.integers(-5, 5, (n, K)))).astype(dtype)
+    diag = (rng.uniform(1, 2, n) * np.exp2(rng.integers(-8, 8, n))).astype(dtype)
+    diag[:6] = np.array([0.0, np.inf, -0.0, np.finfo(dtype).tiny / 4, 2.0**big, 2.0**-big], dtype)
+    x[6, :5] = [np.inf, -np.inf, 0.0, np.nan, np.finfo(dtype).max]
+    with np.errstate(all="ignore"):
+        ref = x / diag[:, None]
+
+    def solve(r0, r1):
+        b = np.ascontiguousarray(x[r0:r1])
+        lib.team_cpu_trsm_diag(int(dtype == np.float32), r1 - r0, upper, K,
+                               _p(np.ascontiguousarray(np.diag(diag[r0:r1]))), _p(b))
+        return b
+
+    for i in range(7):  # one by one: what is not finite would reach other rows as 0 * inf
+        assert np.array_equal(solve(i, i + 1), ref[i : i + 1], equal_nan=True), diag[i]
+    assert np.array_equal(solve(7, n), ref[7:])
