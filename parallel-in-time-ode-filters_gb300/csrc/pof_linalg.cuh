@@ -321,7 +321,12 @@ struct Acc<float> {
     a.l = __fsub_rn(a.l, l);
     return a.value();
   }
-  __device__ __forceinline__ float value() const { return __fadd_rn(h, l); }
+  // an overflowed or infinite sum has no error term (inf - inf): it is h, as in
+  // the plain sum
+  __device__ __forceinline__ float value() const {
+    const float v = __fadd_rn(h, l);
+    return v == v ? v : h;
+  }
 };
 
 // C(MxN) = A(MxK) * B(KxN)

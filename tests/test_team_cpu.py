@@ -221,3 +221,19 @@ def test_dense_diagonal_solves_round_like_divisions(lib, dtype, upper):
     for i in range(7):  # one by one: what is not finite would reach other rows as 0 * inf
         assert np.array_equal(solve(i, i + 1), ref[i : i + 1], equal_nan=True), diag[i]
     assert np.array_equal(solve(7, n), ref[7:])
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("D,d", [(4, 1), (8, 2)])
+def test_infinite_observation(lib, dtype, D, d):
+    """c infinite in the last step: sigma^2 and -log L are infinite, in float32
+    (compensated sums) as in float64, and the filtered mean is not a number only
+    where it is in float64."""
+    n = 5
+    model = _model(D, d, n, True, "some" if d == 1 else "none", False, D, dtype)
+    model[3][-1, 0] = np.inf
+    m, L, s = _sequential(lib, dtype, 0, 0, n, D, d, model)
+    m64 = _sequential(lib, np.float64, 0, 0, n, D, d, [None if x is None else x.astype(np.float64) for x in model])
+    if d == 1:
+        assert s[0] == -np.inf and s[2] == np.inf
+    assert np.array_equal(np.isnan(m), np.isnan(m64[0])) and np.array_equal(np.isnan(s), np.isnan(m64[2]))
