@@ -62,13 +62,15 @@ int env_int(const char* name, int dflt = 0) {
   return v ? atoi(v) : dflt;
 }
 
-Plan plan_for(int dtype, int64_t n, int D, int DY, bool solver) {
+// `scratch`: a pass of the filter and smoother entry points, whose workspace
+// query the allocation-free one shares.
+Plan plan_for(int dtype, int64_t n, int D, int DY, bool solver, bool scratch) {
   const int C0 = env_int("POF_C0"), Cg = env_int("POF_CG"), ks = env_int("POF_KS", 0);
   const bool narrow = env_int("POF_TEAM_WIDE_L0") != 0;
   const Plan p = make_plan(n, D, DY, esz(dtype), solver, C0 > 0 ? C0 : even_c0(n, l0_lanes(D, !narrow)), Cg, narrow, ks);
   // A pass that only pick_c0's chunks bring under the scratch of the
   // allocation-free entry point takes those.
-  if (!solver && C0 <= 0 && p.total > POF_NOALLOC_SCRATCH_BYTES) {
+  if (scratch && C0 <= 0 && p.total > POF_NOALLOC_SCRATCH_BYTES) {
     const Plan q = make_plan(n, D, DY, esz(dtype), solver, 0, Cg, narrow, ks);
     if (q.total <= POF_NOALLOC_SCRATCH_BYTES) return q;
   }
@@ -279,12 +281,12 @@ static bool dense_shape(int dtype, int D, int d) {
 size_t pof_filtsmooth_workspace_bytes(int32_t dtype, int64_t n_steps, int32_t D, int32_t d) {
   if (n_steps < 1 || D < 1) return 0;
   if (dense_shape(dtype, D, d)) return dense::workspace_bytes(dtype, 1, n_steps, D, d, 0);
-  return plan_for(dtype, n_steps, D, d, false).total;
+  return plan_for(dtype, n_steps, D, d, false, true).total;
 }
 
 size_t pof_ieks_workspace_bytes(int32_t dtype, int64_t n_steps, int32_t D, int32_t d) {
   if (n_steps < 1 || D < 1) return 0;
-  return plan_for(dtype, n_steps, D, d, true).total;
+  return plan_for(dtype, n_steps, D, d, true, false).total;
 }
 
 static int filtsmooth_impl(int which, int32_t dtype, int64_t n, int32_t D, int32_t d, const void* x0m,
@@ -300,7 +302,7 @@ static int filtsmooth_impl(int which, int32_t dtype, int64_t n, int32_t D, int32
   if (!x0m || !x0L || !F || !QL || !H || !c || !om || !oL || !ws) return POF_ERR_ARG;
   if (fts != 0 && fts != (int64_t)D * D) return POF_ERR_ARG;
   if (R && rs != 0 && rs != (int64_t)d * d) return POF_ERR_ARG;
-  Plan p = plan_for(dtype, n, D, d, false);
+  Plan p = plan_for(dtype, n, D, d, false, true);
   if (wsb < p.total) return POF_ERR_WORKSPACE;
   char* w = aligned_ws(ws);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -356,7 +358,7 @@ int pof_smoothing(int32_t dtype, int64_t n_steps, int32_t D, const void* F, cons
   if (n_steps < 1 || !F || !QL || !filt_mean || !filt_chol || !out_mean || !out_chol || !workspace)
     return POF_ERR_ARG;
   if (ft_stride != 0 && ft_stride != (int64_t)D * D) return POF_ERR_ARG;
-  Plan p = plan_for(dtype, n_steps, D, dy_used, false);
+  Plan p = plan_for(dtype, n_steps, D, dy_used, false, true);
   if (workspace_bytes < p.total) return POF_ERR_WORKSPACE;
   char* w = aligned_ws(workspace);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -671,8 +673,8 @@ struct MixedLayout {
 
 MixedLayout mixed_layout(int64_t n, int D, int d) {
   MixedLayout m;
-  m.p64 = plan_for(POF_F64, n, D, d, true);
-  m.p32 = plan_for(POF_F32, n, D, d, false);
+  m.p64 = plan_for(POF_F64, n, D, d, true, false);
+  m.p32 = plan_for(POF_F32, n, D, d, false, false);
   m.p32.fobj = false;
   size_t off = align_up(m.p64.total);
   m.off32 = off;
@@ -757,7 +759,7 @@ int pof_ieks_solve(int32_t dtype, int64_t n_steps, int32_t D, int32_t d, int32_t
   if (field <= 0 || field >= FIELD_COUNT || field_dim(field) != d) return POF_ERR_FIELD;
   if (!params || !x0_mean || !x0_chol || !F || !QL || !means || !chols || !workspace || maxiters < 0)
     return POF_ERR_ARG;
-  Plan p = plan_for(dtype, n_steps, D, d, true);
+  Plan p = plan_for(dtype, n_steps, D, d, true, false);
   if (workspace_bytes < p.total) return POF_ERR_WORKSPACE;
   double p0, p1;
   rc = nordsieck_p01(D, d, h, &p0, &p1);
