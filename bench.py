@@ -1087,9 +1087,9 @@ def run_gpu_batch(args, workload):
     torch.cuda.synchronize()
     prof = _lib.profile_read(reset=True)
     _lib.profile_enable(False)
-    per_step = {"filt_l0_down": _flops.kf_step(D, d, True) + _flops.objective_term(D),
+    per_step = {"filt_l0_down": _flops.kf_step(D, d, True),
                 "filt_l0_reduce": _flops.cond_fold_step(D, d),
-                "smo_l0_down": _flops.smooth_apply(D) + _flops.objective_term(D) + D * D}
+                "smo_l0_down": _flops.l0_smooth_apply(D, d) + _flops.objective_term(D, d) + D * D}
     kern = {k: v for k, v in prof.items() if v[1] > 0 and k in per_step}
     dom = max(kern, key=lambda k: kern[k][0])
     dom_ms = kern[dom][0]

@@ -4,13 +4,12 @@ Counts follow the loops of the kernels: an FMA is 2 flops; add, multiply,
 divide, square root and log are 1.  They are the algorithmic work of each
 kernel -- the operations it performs, the structural zeros it skips not
 counted -- and the numerator of its achieved-FLOP/s figure.  structured=True
-(level 0 from D = 6 on, csrc/pof_team.cuh) is the IWP prior with exact
-observations of the EK1 model, as a solve has it: block-diagonal F, block
+is the IWP prior with exact observations of the EK1 model, as every solve has
+it (level 0, csrc/pof_team.cuh and csrc/pof_ops.cuh): block-diagonal F, block
 staircase in the predicted factor's triangularization, D - d columns in the
 factor of an updated state, observation rows that end at the last derivative
-of order one.  The thread-per-chunk level 0 (D < 6, csrc/pof_ops.cuh) is
-counted as the general model's dense loops: it skips the same zeros, so the
-figures for it err high.
+of order one.  structured=False is a general model's dense loops below D = 6.
+``kernel_flops`` and what builds on it count the structured kernels.
 ``reference_step_flops`` is the work
 per step and IEKS iteration of the reference's own formulation (per-step
 elements, ~2 combines per element in the associative scan, sigma^2/NLL pass).
@@ -18,10 +17,10 @@ elements, ~2 combines per element in the associative scan, sigma^2/NLL pass).
 
 
 def tria(M, NC, MB=0, wlow=0, ncut=None):
-    """tria<M, NC> (+ MB extra rows for tria_top); wlow > 0: the right block
-    from column wlow is lower-triangular, reflector j stops at column
-    wlow + j; ncut: the columns from ncut on are zero (reflectors from
-    ncut - 1 on are skipped)."""
+    """Householder LQ of M rows of NC columns (lq_rows of csrc/pof_linalg.cuh)
+    over MB more rows; wlow > 0: the right block from column wlow is
+    lower-triangular, reflector j stops at column wlow + j; ncut: the columns
+    from ncut on are zero (reflectors from ncut - 1 on are skipped)."""
     f = 0
     mlim = M if ncut is None else min(M, ncut - 1)
     for j in range(mlim):
@@ -36,8 +35,9 @@ def tria(M, NC, MB=0, wlow=0, ncut=None):
 
 
 def lq(M, tail, MB=0):
-    """t_lq of csrc/pof_team.cuh: reflector j of M combines the pivot with
-    tail(j) columns, over the rows below it and MB more."""
+    """t_lq of csrc/pof_team.cuh, lq_pivot of csrc/pof_linalg.cuh: reflector j
+    of M combines the pivot with tail(j) columns, over the rows below it and
+    MB more."""
     f = 0
     for j in range(M):
         t = tail(j)
@@ -150,25 +150,40 @@ def smooth_apply(D, structured=True):
     return mv(D, D) + mm_lowerB(D, D) + tria(D, 2 * D, wlow=w) + D
 
 
-def objective_term(D):
-    return mv(D, D) + D + trsv(D) + 2 * D
+def l0_smooth_combine(D, d):
+    """Level-0 composite step: [D2 | E2 D1], the element's factor D1 with D - d
+    columns (t_smooth_combine_raw; smooth_combine of csrc/pof_ops.cuh)."""
+    nk = D - d if d < D else D
+    return mv(D, D) + mm(D, D, nk) + lq(D, lambda j: nk) + mm(D, D, D) + D
+
+
+def l0_smooth_apply(D, d):
+    """Level-0 application: [E L | D2], tails right of the diagonal."""
+    nk = D - d if d < D else D
+    return mv(D, D) + mm_lowerB(D, D) + lq(D, lambda j: D + nk - j - 1) + D
+
+
+def objective_term(D, d=None):
+    """d: F block-diagonal, its zeros skipped (the team kernels)."""
+    return (mv(D, D) if d is None else mm_f(D, 1, d)) + D + trsv(D) + 2 * D
 
 
 def kernel_flops(kind, n, D, d, C0, cnt):
     """Flops of one launch of a kernel kind over a problem with n steps and
     level sizes cnt = [None, cnt1, cnt2, ...] (all launches of that kind in
-    one filter + smoother pass, summed over levels)."""
+    one filter + smoother pass of a solve, summed over levels; a solve has no
+    filter objective)."""
     n1 = cnt[1]
     levels = len(cnt) - 1
     if kind == "filt_l0_reduce":
         first = min(C0, n)
-        return first * kf_step(D, d, False) + (n - first) * cond_fold_step(D, d)
+        return first * kf_step(D, d, False, True) + (n - first) * cond_fold_step(D, d, True)
     if kind == "filt_l0_down":
-        return n * (kf_step(D, d, True) + objective_term(D))
+        return n * kf_step(D, d, True, True)
     if kind == "smo_l0_reduce":
-        return (n - n1) * smooth_combine(D, D >= 6)
+        return (n - n1) * l0_smooth_combine(D, d)
     if kind == "smo_l0_down":
-        return n * (smooth_apply(D, D >= 6) + objective_term(D) + D * D)
+        return n * (l0_smooth_apply(D, d) + objective_term(D, d if D >= 6 else None) + D * D)
     if kind == "filt_reduce":
         return sum(cnt[l] - cnt[l + 1] for l in range(1, levels)) * filt_combine(D)
     if kind == "filt_down":
@@ -193,7 +208,8 @@ def l0_lanes(D):
 
 
 def plan_levels(n, D=4, C0=None, Cg=2, top=2):
-    """The level sizes libpof uses (csrc/pof_plan.h even_c0, make_plan)."""
+    """The level sizes of a solve (csrc/pof_plan.h even_c0, make_plan; a pass
+    whose workspace only longer chunks bring under 16 MiB takes those)."""
     if C0 is None:
         lanes = l0_lanes(D)
         target = 19456 if lanes == 1 else 48640 // lanes
