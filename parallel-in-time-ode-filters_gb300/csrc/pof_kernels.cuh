@@ -202,6 +202,7 @@ __global__ void __launch_bounds__(64) k_filt_l0_reduce(int64_t n, int C0, StepMo
     LogProd lp;
     bool thin = false, lower = false;
     for (int64_t s = 0; s < s1; ++s) {
+      if (!POF_IN(s, n)) break;
       StepView<T, D, DY> v(sm, s);
       kf_step_any<T, D, DY, false>(v, cm.exact(v), thin, lower, m, L, ssq, yy, lp, nullptr, nullptr, nullptr);
     }

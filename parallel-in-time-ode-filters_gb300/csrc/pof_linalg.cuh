@@ -356,18 +356,6 @@ __device__ __forceinline__ void mv(const T* __restrict__ A, const T* __restrict_
   }
 }
 
-// y(N) = A(MxN)^T x(M)
-template <typename T, int M, int N, int LDA>
-__device__ __forceinline__ void mtv(const T* __restrict__ A, const T* __restrict__ x, T* __restrict__ y) {
-#pragma unroll
-  for (int j = 0; j < N; ++j) {
-    T s = T(0);
-#pragma unroll
-    for (int i = 0; i < M; ++i) s = fma(A[i * LDA + j], x[i], s);
-    y[j] = s;
-  }
-}
-
 // The LQ factorisation by Householder reflectors of the first M of the MX
 // rows of X (NC columns): afterwards X[:M, :M] holds L in its lower triangle
 // (L L^T = the M rows' X X^T) and the rows below are multiplied by the same
@@ -456,34 +444,6 @@ __device__ __forceinline__ void trsv_l(const T* __restrict__ L, T* b) {
 #pragma unroll
     for (int k = 0; k < i; ++k) s = fma(-L[i * LDL + k], b[k], s);
     b[i] = s * rcp(L[i * LDL + i]);
-  }
-}
-
-// b <- L^{-T} b   (L lower-triangular M x M; back substitution with L^T)
-template <typename T, int M, int LDL>
-__device__ __forceinline__ void trsv_lt(const T* __restrict__ L, T* b) {
-#pragma unroll
-  for (int i = M - 1; i >= 0; --i) {
-    T s = b[i];
-#pragma unroll
-    for (int k = i + 1; k < M; ++k) s = fma(-L[k * LDL + i], b[k], s);
-    b[i] = s * rcp(L[i * LDL + i]);
-  }
-}
-
-// B(M x NR) <- L^{-1} B
-template <typename T, int M, int NR, int LDL, int LDB>
-__device__ __forceinline__ void trsm_l(const T* __restrict__ L, T* B) {
-#pragma unroll
-  for (int i = 0; i < M; ++i) {
-    const T inv = rcp(L[i * LDL + i]);
-#pragma unroll
-    for (int j = 0; j < NR; ++j) {
-      T s = B[i * LDB + j];
-#pragma unroll
-      for (int k = 0; k < i; ++k) s = fma(-L[i * LDL + k], B[k * LDB + j], s);
-      B[i * LDB + j] = s * inv;
-    }
   }
 }
 

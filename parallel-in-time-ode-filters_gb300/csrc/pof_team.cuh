@@ -65,17 +65,6 @@ __device__ __forceinline__ void t_mm(const Team<TS>& tm, const T* A, const T* B,
   }
 }
 
-// y(M) = op(A) x: lanes split the rows.
-template <typename T, int TS, int M, int K, int LDA, bool TA = false>
-__device__ __forceinline__ void t_mv(const Team<TS>& tm, const T* A, const T* x, T* y) {
-  for (int i = tm.r; i < M; i += TS) {
-    Acc<T> s(T(0));
-#pragma unroll
-    for (int k = 0; k < K; ++k) s.mul_add(TA ? A[k * LDA + i] : A[i * LDA + k], x[k]);
-    y[i] = s.value();
-  }
-}
-
 // ---------------------------------------------------------------------------
 // LQ with a triangular pivot block.  Rows [P | W] (M rows, pivot entry (j, j)
 // of row j in column j, tail columns [kb(j), ke(j)) given by `tail`) and MB
@@ -305,37 +294,6 @@ __device__ __forceinline__ void t_trsm_l(const Team<TS>& tm, const T* L, T* B) {
         Acc<T> s(B[i * LDB + j]);
 #pragma unroll
         for (int k = 0; k < i; ++k) s.mul_add(-L[i * LDL + k], B[k * LDB + j]);
-        B[i * LDB + j] = s.value() * rcp(L[i * LDL + i]);
-      }
-    }
-  }
-}
-
-// B(M x NR) <- L^{-T} B
-template <typename T, int TS, int M, int NR, int LDL, int LDB>
-__device__ __forceinline__ void t_trsm_lt(const Team<TS>& tm, const T* L, T* B) {
-  if constexpr (M <= TS) {
-    const int src = (threadIdx.x & 31) / TS * TS;
-    const T rd = t_recip_diag<T, TS, M, LDL>(tm, L);
-    T rdi[M];
-#pragma unroll
-    for (int i = 0; i < M; ++i) rdi[i] = __shfl_sync(tm.mask, rd, src + i);
-    for (int j = tm.r; j < NR; j += TS) {
-#pragma unroll
-      for (int i = M - 1; i >= 0; --i) {
-        Acc<T> s(B[i * LDB + j]);
-#pragma unroll
-        for (int k = i + 1; k < M; ++k) s.mul_add(-L[k * LDL + i], B[k * LDB + j]);
-        B[i * LDB + j] = s.value() * rdi[i];
-      }
-    }
-  } else {
-    for (int j = tm.r; j < NR; j += TS) {
-#pragma unroll
-      for (int i = M - 1; i >= 0; --i) {
-        Acc<T> s(B[i * LDB + j]);
-#pragma unroll
-        for (int k = i + 1; k < M; ++k) s.mul_add(-L[k * LDL + i], B[k * LDB + j]);
         B[i * LDB + j] = s.value() * rcp(L[i * LDL + i]);
       }
     }
