@@ -51,13 +51,14 @@ int panel_rows(int n, size_t es) {
   return nb;
 }
 
-// Panels of at least kClusterMinCols columns in batches of at most
-// kClusterMaxBatch matrices are factored by a cluster of kClusterSize CTAs
-// (k_tria_panel_cl), each holding a quarter of the columns: that puts idle
-// SMs to work in the tree levels above the chunks.  At the chunk loops'
-// batches (64-256) every SM already holds a panel, and the cluster's
-// barriers only add time (reaction-diffusion at D = 640: float32 4.64 s per
-// pass against 4.32 s, float64 10.3 s against 9.2 s for 512 steps).
+// Panels too wide for registers (RegPanel): in batches of at most
+// kClusterMaxBatch matrices, from kClusterMinCols columns on, a cluster of
+// kClusterSize CTAs factors one (k_tria_panel_cl), each holding a quarter of the
+// columns, which puts idle SMs to work in the tree levels above the chunks; else
+// one CTA (k_tria_panel).  Measured with the register panels switched off, ms,
+// cluster in small batches / one CTA always: float64 D = 512, 6 steps 250 / 311,
+// float32 D = 1280, 8 steps 323 / 352; but D = 128, 150 steps 105 / 101 and
+// float32 D = 384, 256 steps 204 / 183, sizes that take register panels.
 constexpr int kClusterSize = 4;
 constexpr int kClusterMinCols = 256;
 constexpr int64_t kClusterMaxBatch = 32;
@@ -67,7 +68,13 @@ constexpr int64_t kClusterMaxBatch = 32;
 // ---------------------------------------------------------------------------
 // Register panels (k_lq_panel): 16 rows in double (4 warps of 4 rows: a
 // panel's FP64 work grows with its rows squared and runs on one SM), 32 in
-// float (8 warps of 4), up to kRegCols columns.
+// float (8 warps of 4), up to `cols` columns.  Measured, passes in ms, 16 / 32
+// rows: float64 D = 128, 150 steps 61.0 / 71.9, D = 512, 6 steps 226 / 324;
+// float32 D = 384, 256 steps 159 / 137, D = 144, 128 steps 21.2 / 19.7.  Against
+// the shared-memory panels, also where the batch is small (a cluster for batches
+// of up to 4 / 16 / 32 matrices, register panels above): D = 128 74 / 85 / 90 and
+// 61.0 with register panels for all, float32 D = 384 160 / 178 / 187 and 137,
+// D = 1280, 8 steps 313 / 323 / 323 and 313.
 template <typename T>
 struct RegPanel;
 template <>
@@ -90,7 +97,10 @@ void launch_lq_panel(int64_t batch, cudaStream_t st, MV<T> W, int i0, int nbb, i
 // Row blocks of k_wy_apply: their rows and the panel's V fit 200 KB.  double
 // always takes it; float, whose two GEMMs run on the tensor cores, while the
 // row blocks are few (the tree levels above the chunks, where a launch costs
-// its latency).
+// its latency).  Measured, float32 passes in ms with up to 0 / 1 / 2 / 4 / 8 / 16
+// blocks per SM: D = 144, 128 steps 21.5 / 20.1 / 19.9 / 19.7 / 19.6 / 19.6;
+// D = 384, 256 steps 139 / 136 / 135 / 137 / 140 / 147; D = 640, 40 steps 157 /
+// 152 / 155 / 165 / 180 / 200.
 constexpr int kWyRows = 16;
 constexpr int64_t kWyMaxBlocksF32 = 4 * kSMs;
 inline size_t wy_smem(int nb, int np, size_t es) { return size_t(kWyRows + nb) * (np | 1) * es; }
@@ -119,6 +129,7 @@ struct Ctx {
         k_gemm<T, 128, 16, 16, 4, 2><<<dim3(cdiv(N, 16), cdiv(M, 128), nb), 256, 0, st>>>(M, N, K, alpha, A, B,
                                                                                              beta, C, b0);
       } else if (M <= 32 && (sizeof(T) == 4 || cdiv(N, 128) * nb >= 4 * kSMs)) {
+        // (double in this tile at any count: D = 128, 150 steps 64.3 ms for 61.1)
         k_gemm<T, 32, 128, 16, 2, 8><<<dim3(cdiv(N, 128), cdiv(M, 32), nb), 256, 0, st>>>(M, N, K, alpha, A, B,
                                                                                             beta, C, b0);
       } else if (tensor_f32()) {
@@ -126,7 +137,9 @@ struct Ctx {
       } else if (sizeof(T) == 8 && cdiv(N, 64) * cdiv(M, 64) * nb < 4 * kSMs) {
         // double is FP64-pipe bound whatever the tile (a 64 x 64 tile of K =
         // 128 holds an SM for 160 us): too few 64 x 64 tiles to fill the SMs
-        // evenly go as 32 x 32 ones
+        // evenly go as 32 x 32 ones.  D = 128, 150 steps with this from 0 / 1 /
+        // 2 / 4 / 8 / 16 tiles per SM down: 69.1 / 61.7 / 61.1 / 61.1 / 61.1 /
+        // 61.1 ms, D = 192, 40 steps 97.8 / 86.4 / 84.6 / 84.4 / 84.4 / 84.5
         k_gemm<T, 32, 32, 16, 4, 2><<<dim3(cdiv(N, 32), cdiv(M, 32), nb), 128, 0, st>>>(M, N, K, alpha, A, B, beta,
                                                                                           C, b0);
       } else {

@@ -39,9 +39,9 @@ struct Plan {
 };
 
 // Lanes that work on one level-0 chunk: 1 (thread per chunk, state in
-// registers) for small D, a team of 16 or 32 lanes (state in shared memory)
-// from D = 6 on, where per-thread state would spill.  Must match
-// Driver::kTeamL0 / TeamSize.
+// registers) for small D, a team (state in shared memory) from D = 6 on, where
+// per-thread state would spill: 8 lanes up to D = 8, 16 above, twice that in
+// wide teams.  Must match Driver::kTeamL0 / TeamSize.
 inline int team_lanes(int D, bool narrow) {
   const int wide = (2 * D <= 8) ? 8 : (2 * D <= 16 ? 16 : 32);
   return narrow ? (wide / 2 >= 4 ? wide / 2 : 4) : wide;
@@ -65,8 +65,9 @@ inline int pick_c0(int64_t n, int lanes) {
 // Chunk length of the passes and solves: as many chunks as the chip runs at
 // once in even shares, so that no SM is left with one more than the others at
 // the end.  A thread per chunk: one warp on each of the 4 sub-partitions of 152
-// SMs, 19456 chunks.  Teams: 5 blocks of 64 threads per SM (what shared memory
-// lets the down-sweep run), 6080 chunks of 8 lanes, 3040 of 16.  Short grids take
+// SMs, 19456 chunks.  Teams: 5 blocks of 64 threads per SM, 6080 chunks of 8
+// lanes, 3040 of 16 -- what shared memory lets the down-sweep run at D = 8 and 12;
+// at D = 6, 9 and 10, where 7 or 8 fit, the same line.  Short grids take
 // short chunks for the latency of a chunk's chain, but not below 4 and 2, from
 // where on the tree costs more.  Measured, ms, pick_c0 / this (steps per chunk):
 // logistic q = 3 solves of 150000 steps 17.9 / 15.2 (16, 8), of 262143 20.9 /
