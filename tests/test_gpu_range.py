@@ -60,8 +60,9 @@ KS = {torch.float64: (-300, -490, -505, 470, 500), torch.float32: (-40, -58, 50)
 @pytest.mark.parametrize("D,d,n,noise", [(2, 1, 40, False), (4, 1, 33, True), (6, 2, 25, False), (8, 2, 21, True),
                                          (12, 3, 9, False)])
 def test_passes_far_from_one(D, d, n, noise, dtype):
-    """(The parallel pass also carries the information's factor, in units of
-    2^-k, whose squares end 2^-k 10 earlier than the state's.)"""
+    """(The parallel pass also carries the information's factor, in units of 2^-k
+    and growing along the grid: its squares overflow a little before k = -512,
+    where the state's still hold.)"""
     _check(pfs.linear_filtsmooth, (D, d, n, dtype, noise), KS[dtype], dtype)
     ks = KS[dtype] + ((-512, -514, 505) if dtype == torch.float64 else ())
     _check(sfs.linear_filtsmooth, (D, d, n, dtype, noise), ks, dtype)
